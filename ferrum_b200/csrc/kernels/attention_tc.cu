@@ -313,33 +313,35 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     }
   } else if (warp <= NT) {
     // ------------------------------------------------------------ MMA issuer of one row tile
-    if (lane == 0) {
+    if (elect_one()) {
       const int t = warp - 1;
       const uint32_t idesc_qk = umma_idesc_16bit(128, BN, HALF);
       const uint32_t idesc_pv = umma_idesc_16bit(128, D, HALF) | (1u << 16);  // B (values) is MN-major
       const uint32_t q_addr = smem_base + Cfg::OFF_Q + t * Cfg::Q_TILE_BYTES;
       const uint32_t o_tmem = tmem_base + Cfg::O_COL + t * D;
+      const uint64_t q_desc = umma_desc_k_sw128(q_addr), k_desc0 = umma_desc_k_sw128(smem_base + Cfg::OFF_K);
+      const uint64_t v_desc0 = umma_desc_mn_sw128(smem_base + Cfg::OFF_V, Cfg::KV_HALF_BYTES, 1024);
       auto issue_qk = [&](int s, int buf) {
-        const uint32_t k_addr = smem_base + Cfg::OFF_K + s * Cfg::KV_STAGE_BYTES;
+        const uint64_t k_desc = k_desc0 + (uint64_t)(s * (Cfg::KV_STAGE_BYTES >> 4));
         const uint32_t s_tmem = tmem_base + Cfg::S_COL + (2 * t + buf) * BN;
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk) {
           const int h = kk >> 2, in = kk & 3;
-          umma_bf16(s_tmem, umma_desc_k_sw128(q_addr + h * 128 * 128) + (uint64_t)(in * 2),
-                    umma_desc_k_sw128(k_addr + h * Cfg::KV_HALF_BYTES) + (uint64_t)(in * 2), idesc_qk, kk > 0);
+          umma_bf16(s_tmem, q_desc + (uint64_t)((h * 128 * 128 >> 4) + in * 2),
+                    k_desc + (uint64_t)((h * Cfg::KV_HALF_BYTES >> 4) + in * 2), idesc_qk, kk > 0);
         }
       };
       auto issue_pv = [&](int s, int buf, bool accumulate) {
-        const uint32_t v_addr = smem_base + Cfg::OFF_V + s * Cfg::KV_STAGE_BYTES;
+        const uint64_t v_desc = v_desc0 + (uint64_t)(s * (Cfg::KV_STAGE_BYTES >> 4));
         const uint32_t p_tmem = tmem_base + Cfg::S_COL + (2 * t + buf) * BN;  // P lies over the scores it came from
 #pragma unroll
         for (int kk = 0; kk < BN / 16; ++kk)  // 16 keys on: 8 columns of P, 16 rows of V
-          umma_bf16_ts(o_tmem, p_tmem + kk * 8, umma_desc_mn_sw128(v_addr + kk * 16 * 128, Cfg::KV_HALF_BYTES, 1024), idesc_pv,
+          umma_bf16_ts(o_tmem, p_tmem + kk * 8, v_desc + (uint64_t)(kk * 16 * 128 >> 4), idesc_pv,
                        accumulate || kk > 0);
         if constexpr (WIDE) {
 #pragma unroll
           for (int kk = 0; kk < BN / 16; ++kk)  // the remainders, behind P
-            umma_bf16_ts(o_tmem, p_tmem + BN / 2 + kk * 8, umma_desc_mn_sw128(v_addr + kk * 16 * 128, Cfg::KV_HALF_BYTES, 1024), idesc_pv, true);
+            umma_bf16_ts(o_tmem, p_tmem + BN / 2 + kk * 8, v_desc + (uint64_t)(kk * 16 * 128 >> 4), idesc_pv, true);
         }
       };
       // the scores of stages 0 and 1 go ahead; in the loop the scores of stage j + 2 follow P V of stage j
@@ -756,27 +758,27 @@ attention_tc_pair_kernel(const __grid_constant__ CUtensorMap map_kv, const uint1
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (the leader's, for both CTAs)
-    if (lane == 0 && rank == 0) {
+    if (rank == 0 && elect_one()) {
       const uint32_t idesc_qk = umma_idesc_16bit(256, BN, HALF);
       const uint32_t idesc_pv = umma_idesc_16bit(256, D, HALF) | (1u << 16);  // B (values) is MN-major
       const uint32_t q_tmem = tmem_base + Cfg::Q_COL, o_tmem = tmem_base + Cfg::O_COL;
+      const uint64_t k_desc0 = umma_desc_k_sw128(smem_base + Cfg::OFF_K);
+      const uint64_t v_desc0 = umma_desc_mn_sw128(smem_base + Cfg::OFF_V, Cfg::V_STAGE_BYTES, 1024);
       auto issue_qk = [&](int s, int buf) {
-        const uint32_t k_addr = smem_base + Cfg::OFF_K + s * Cfg::K_STAGE_BYTES;
+        const uint64_t k_desc = k_desc0 + (uint64_t)(s * (Cfg::K_STAGE_BYTES >> 4));
         const uint32_t s_tmem = tmem_base + Cfg::S_COL + buf * BN;
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk) {  // 16 elements of the head on: 8 columns of Q, 32 bytes of a key row
           const int h = kk >> 2, in = kk & 3;
-          umma_16bit_pair_ts(s_tmem, q_tmem + kk * 8, umma_desc_k_sw128(k_addr + h * Cfg::K_HALF_BYTES) + (uint64_t)(in * 2),
-                             idesc_qk, kk > 0);
+          umma_16bit_pair_ts(s_tmem, q_tmem + kk * 8, k_desc + (uint64_t)((h * Cfg::K_HALF_BYTES >> 4) + in * 2), idesc_qk, kk > 0);
         }
       };
       auto issue_pv = [&](int s, int buf, bool accumulate) {
-        const uint32_t v_addr = smem_base + Cfg::OFF_V + s * Cfg::V_STAGE_BYTES;
+        const uint64_t v_desc = v_desc0 + (uint64_t)(s * (Cfg::V_STAGE_BYTES >> 4));
         const uint32_t p_tmem = tmem_base + Cfg::S_COL + buf * BN;  // P lies over the scores it came from
 #pragma unroll
         for (int kk = 0; kk < BN / 16; ++kk)  // 16 keys on: 8 columns of P, 16 rows of V
-          umma_16bit_pair_ts(o_tmem, p_tmem + kk * 8, umma_desc_mn_sw128(v_addr + kk * 16 * 128, Cfg::V_STAGE_BYTES, 1024),
-                             idesc_pv, accumulate || kk > 0);
+          umma_16bit_pair_ts(o_tmem, p_tmem + kk * 8, v_desc + (uint64_t)(kk * 16 * 128 >> 4), idesc_pv, accumulate || kk > 0);
       };
       bool ok = mbar_wait_cluster(q_ready, 0, abort_p);
       int code = 32;

@@ -207,11 +207,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0 && p.drop_loads) {
+    if (p.drop_loads) {
       // (test hook) nothing is requested, nothing will be in flight: the other roles' waits run out
       pdl_wait();
       pdl_launch();
-    } else if (lane == 0) {
+    } else if (elect_one()) {
       int s = 0;
       uint32_t phase = 0;
       long long tile = u_begin / nkb;
@@ -276,8 +276,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = umma_idesc_16bit(TILE_N, BT, p.half != 0);
+      const uint64_t desc0 = umma_desc_k_sw128(smem_base);
       int s = 0;
       uint32_t phase = 0;
       int seg = 0;
@@ -303,10 +304,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
             break;
           }
           tc_fence_after();
-          const uint32_t a = smem_base + s * Cfg::STAGE_BYTES;
-          const uint64_t a_desc = umma_desc_k_sw128(a);
-          const uint64_t a2_desc = umma_desc_k_sw128(a + A_BYTES);
-          const uint64_t b_desc = umma_desc_k_sw128(a + A_BYTES * (DUAL ? 2 : 1));
+          const uint64_t a_desc = desc0 + (uint64_t)(s * (Cfg::STAGE_BYTES >> 4));
+          const uint64_t a2_desc = a_desc + (A_BYTES >> 4);
+          const uint64_t b_desc = a_desc + (A_BYTES * (DUAL ? 2 : 1) >> 4);
 #pragma unroll
           for (int kk = 0; kk < TILE_K / UMMA_K; ++kk) {
             const bool acc = !first || kk > 0;
@@ -600,7 +600,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (both CTAs)
-    if (lane == 0) {
+    if (elect_one()) {
       int s = 0;
       uint32_t phase = 0;
       pdl_wait();
@@ -635,8 +635,9 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (leader only)
-    if (lane == 0 && rank == 0) {
+    if (rank == 0 && elect_one()) {
       const uint32_t idesc = umma_idesc_16bit(2 * TILE_N, PAIR_BT, p.half != 0);
+      const uint64_t desc0 = umma_desc_k_sw128(smem_base);
       int s = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -660,9 +661,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             break;
           }
           tc_fence_after();
-          const uint32_t a = smem_base + s * PAIR_STAGE_BYTES;
-          const uint64_t a_desc = umma_desc_k_sw128(a);
-          const uint64_t b_desc = umma_desc_k_sw128(a + A_BYTES);
+          const uint64_t a_desc = desc0 + (uint64_t)(s * (PAIR_STAGE_BYTES >> 4));
+          const uint64_t b_desc = a_desc + (A_BYTES >> 4);
 #pragma unroll
           for (int kk = 0; kk < TILE_K / UMMA_K; ++kk) {
             const uint64_t adv = (uint64_t)(kk * UMMA_K * 2 >> 4);
@@ -1561,7 +1561,7 @@ gemm_tc_grouped_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0 && !p.drop_loads) {     // (test hook: nothing is requested, the other roles' waits run out)
+    if (!p.drop_loads && elect_one()) {     // (test hook: nothing is requested, the other roles' waits run out)
       int s = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -1589,8 +1589,9 @@ gemm_tc_grouped_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = umma_idesc_16bit(TILE_N, BT, p.half != 0);
+      const uint64_t desc0 = umma_desc_k_sw128(smem_base);
       int s = 0;
       uint32_t phase = 0;
       int seg = 0;
@@ -1612,10 +1613,9 @@ gemm_tc_grouped_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
             break;
           }
           tc_fence_after();
-          const uint32_t a = smem_base + s * Cfg::STAGE_BYTES;
-          const uint64_t a_desc = umma_desc_k_sw128(a);
-          const uint64_t a2_desc = umma_desc_k_sw128(a + A_BYTES);
-          const uint64_t b_desc = umma_desc_k_sw128(a + A_BYTES * (DUAL ? 2 : 1));
+          const uint64_t a_desc = desc0 + (uint64_t)(s * (Cfg::STAGE_BYTES >> 4));
+          const uint64_t a2_desc = a_desc + (A_BYTES >> 4);
+          const uint64_t b_desc = a_desc + (A_BYTES * (DUAL ? 2 : 1) >> 4);
 #pragma unroll
           for (int kk = 0; kk < TILE_K / UMMA_K; ++kk) {
             const bool acc = kb > 0 || kk > 0;

@@ -11,6 +11,11 @@ namespace sm100 {
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
+// One lane of a whole warp, by the instruction that lets the compiler see that what follows runs in a single thread.
+// The tcgen05 and TMA instructions take their operands from registers that the warp shares: behind a plain
+// `lane == 0` the compiler makes them from a vector register for whichever lanes are active, and the matrix
+// unit waits for its issuer (measured on a B200, one CTA, 192 products of 128 x N x 16 in a row, clocks a product:
+// 162 whatever N is behind `lane == 0`, 129 at N = 256 and 65 at N = 128, the unit's own rate, behind this).
 __device__ __forceinline__ bool elect_one() {
   uint32_t pred;
   asm volatile(
@@ -119,6 +124,7 @@ __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::
 // bfloat16) with the 128-byte swizzle that a TMA load with SWIZZLE_128B writes: 8-row
 // groups of 1024 bytes follow each other (stride byte offset 1024).  The tile base must be
 // 1024-byte aligned; advancing by 16 elements along K adds 32 bytes to the start address.
+// (An issue loop makes one descriptor ahead and adds (bytes >> 4) to it: shared memory ends below the field's 18 bits.)
 __device__ __forceinline__ uint64_t umma_desc_k_sw128(uint32_t smem_addr) {
   uint64_t d = 0;
   d |= (uint64_t)((smem_addr & 0x3FFFF) >> 4);  // start address, bits [0,14)
