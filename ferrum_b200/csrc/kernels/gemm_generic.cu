@@ -1,7 +1,7 @@
 // out[t, n] = sum_k x[t, k] * w[n, k] on the CUDA cores, float32 accumulation with FFMA.
 //
-// This is the true 32-bit matrix product of the engine (the tensor cores have no float32
-// input type; TF32 is not 32-bit), and the 16-bit product for shapes the tcgen05 kernel
+// This is the 32-bit matrix product of the engine for a few tokens, small matrices and rows that TMA cannot address
+// (gemm_split.cu takes the others), and the 16-bit product for shapes the tcgen05 kernel
 // refuses (rows that are not 16-byte multiples).  The reference's product is a left-to-right
 // dot per output (crates/kernels/src/scalar.rs:221-241).  Two kernels:
 //

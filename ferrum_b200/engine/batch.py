@@ -355,6 +355,14 @@ class StepContext:
             self._splitk_counters = torch.zeros(2 * tiles, dtype=torch.int32, device=self.device)
         return self.scratch.get("gemm_partials", (floats,), torch.float32), self._splitk_counters
 
+    def gemm_split_scratch(self, M, N, K):
+        """(tokens' parts, partial sums) for the float32 product on the tensor cores."""
+        from ..ops import lib as ops
+        parts, partials = ops.gemm_split_workspace(M, N, K)
+        lane = "_side" if self.lane else ""
+        return (self.scratch.get("gemm_split_parts" + lane, (parts,), torch.float32),
+                self.scratch.get("gemm_split_partials" + lane, (partials,), torch.float32))
+
     def side_stream(self):
         """A second CUDA stream with a fork and a join event, made at first use: (stream, fork, join)."""
         if self._side is None:

@@ -25,6 +25,7 @@ _DEVICE_ERRORS = {
     10: "tensor-core product: the producer timed out", 11: "tensor-core product: the matrix unit timed out",
     12: "tensor-core product: the epilogue timed out", 13: "tensor-core product: the accumulator was not released in time",
     14: "tensor-core product: partial tiles did not arrive in time",
+    15: "tensor-core product: the weights were not ready in time",
     20: "tensor-core attention: the producer timed out", 22: "tensor-core attention: the queries did not arrive in time",
     23: "tensor-core attention: keys or values did not arrive in time", 24: "tensor-core attention: the weights were not ready in time",
     25: "tensor-core attention: the scores were not ready in time", 26: "tensor-core attention: the output was not ready in time",

@@ -26,7 +26,7 @@ TC_STORE_BF16, TC_STORE_F32, TC_RESIDUAL, TC_SWIGLU, TC_GEGLU, TC_SWISH_CLAMP, T
 
 _lib = None
 _lock = threading.Lock()
-ABI = 21
+ABI = 22
 
 
 def lib():
@@ -410,6 +410,48 @@ def gemm_generic(x, w, out, epilogue, M=None):
     _check(lib().ferrum_gemm_generic(_ptr(x), _ptr(w), _ptr(out), dtype_code(x.dtype), c_int(M), c_int(N), c_int(K),
                                      c_int(x.stride(0)), c_int(w.stride(0)), c_int(out.stride(0)), c_int(epilogue),
                                      _stream()), "gemm_generic")
+
+
+# Where the float32 product runs on the tensor cores: with more than 64 tokens, where the CUDA cores' kernel is the tiled one,
+# from 128 x 512 up (65 tokens: 512 x 512 43 us against 14, 1024 x 1024 82 against 15, 5120 x 3072 240 against 27; its error is
+# a third of the tiled kernel's at K = 512 and less beyond).  Up to 64 tokens the streaming kernel stays: it is slower from
+# some 16 tokens on (16384 x 3072, 16 tokens: 86 us against 41), but its sums are spread over 128 threads and its error is smaller
+# (K = 512: 0.8e-7 against 1.4e-7; equal at K = 8192).
+GEMM_SPLIT_MIN_TOKENS = 65
+
+
+def gemm_split_supported(x, w, M):
+    """Whether x[:M] @ w.T, both float32, runs on the tensor cores (see csrc/kernels/gemm_split.cu)."""
+    N, K = w.shape
+    return (x.dtype == torch.float32 and w.dtype == torch.float32 and M >= GEMM_SPLIT_MIN_TOKENS
+            and N >= 128 and K >= 512 and K % 8 == 0 and x.stride(0) % 4 == 0 and w.stride(0) % 4 == 0
+            and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
+
+
+@functools.lru_cache(maxsize=4096)
+def gemm_split_workspace(M, N, K):
+    """(floats for the tokens' parts, floats for partial sums) that a launch needs."""
+    floats = (c_longlong * 2)()
+    lib().ferrum_gemm_split_workspace(c_int(M), c_int(N), c_int(K), floats)
+    return int(floats[0]), int(floats[1])
+
+
+def gemm_split(x, w, out, err, parts, partials, M=None, add=False):
+    """out[t, n] (=, or += with `add`) sum_k x[t, k] w[n, k], all float32, as six bfloat16 products of the operands' three
+    parts.  parts and partials (float32) are scratch, see `gemm_split_workspace`."""
+    global launches
+    for t, name in ((x, "x"), (w, "w"), (out, "out")):
+        _need(t, torch.float32, name, 2)
+    _need(parts, torch.float32, "parts"); _need(partials, torch.float32, "partials")
+    M = x.shape[0] if M is None else M
+    N, K = w.shape
+    if x.shape[1] != K or out.shape[1] < N or out.shape[0] < M or x.shape[0] < M:
+        raise KernelError(f"gemm_split: shapes do not agree: x {tuple(x.shape)} w {tuple(w.shape)} out {tuple(out.shape)}")
+    _gemm_work(x, w, out, M, N, K)
+    _check(lib().ferrum_gemm_split(_ptr(x), _ptr(w), _ptr(out), c_int(M), c_int(N), c_int(K), c_int(x.stride(0)), c_int(w.stride(0)),
+                                   c_int(out.stride(0)), c_int(1 if add else 0), _ptr(parts), c_longlong(parts.numel()), _ptr(partials),
+                                   c_longlong(partials.numel()), _ptr(err), _stream()), "gemm_split")
+    launches += (1 + (partials.numel() > 0)) if M else 0      # (the tokens' parts and the sum of the ranges have kernels of their own)
 
 
 def thin_linear_supported(x, w, M):

@@ -48,6 +48,8 @@ def linear(x, w, out, mode, ctx, M=None):
         N, K = w.shape
         ws, cnt = ctx.gemm_scratch(M, N, K, False)
         ops.gemm_tc(x, w, out, _TC[mode], ctx.err, ws, cnt, M=M)
+    elif ops.gemm_split_supported(x, w, M):
+        ops.gemm_split(x, w, out, ctx.err, *ctx.gemm_split_scratch(M, *w.shape), M=M, add=mode == RESIDUAL)
     else:
         ops.gemm_generic(x, w, out, _GENERIC[mode], M=M)
 

@@ -1,0 +1,97 @@
+"""The float32 product on the tensor cores (csrc/kernels/gemm_split.cu) against float64 and against the CUDA cores' kernel."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from ferrum_b200.ops import lib
+    lib.require_cuda()
+    return lib
+
+
+def run(ops, x, w, M=None, add=None):
+    M = x.shape[0] if M is None else M
+    N, K = w.shape
+    parts, partials = ops.gemm_split_workspace(M, N, K)
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    out = add.clone() if add is not None else torch.full((M, N), float("nan"), device="cuda")
+    ops.gemm_split(x, w, out, err, torch.empty(parts, device="cuda"), torch.empty(partials, device="cuda"), M=M, add=add is not None)
+    assert err.item() == 0
+    return out
+
+
+# Edges: one token and the largest tile, a tile more; features and K that end inside a tile, a piece and 16 elements;
+# one range of K and several (their number follows from N and K), also where rows are no multiples of 16 bytes apart.
+@pytest.mark.parametrize("M,N,K", [(1, 128, 64), (9, 2048, 2048), (16, 130, 1024), (65, 200, 520), (112, 127, 1032), (113, 1001, 512),
+                                   (128, 129, 8), (129, 256, 4104), (300, 384, 3072), (257, 19000, 512), (2048, 128, 128)])
+def test_gemm_split(ops, M, N, K):
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    x = torch.randn(M, K, device="cuda", generator=g)
+    w = torch.randn(N, K, device="cuda", generator=g)
+    ref = x.double() @ w.double().T
+    # Of |x| |w|: 2^-23 for the products left out, 2^-22 for the matrix unit's cut-offs within a piece, half an ulp for
+    # every piece and range that is added.
+    bound = (x.double().abs() @ w.double().abs().T) * (2.0 ** -23 + 2.0 ** -22 + (K // 64 + 9) * 2.0 ** -24)
+    out = run(ops, x, w)
+    assert ((out.double() - ref).abs() <= bound).all()
+    res = torch.randn(M, N, device="cuda", generator=g)
+    total = run(ops, x, w, add=res)
+    assert ((total.double() - res.double() - ref).abs() <= bound + 2.0 ** -24 * total.double().abs()).all()
+    if ops.gemm_split_supported(x, w, M):       # where it stands in for the tiled kernel it is the closer of the two
+        plain = torch.empty(M, N, device="cuda")
+        ops.gemm_generic(x, w, plain, ops.EPI_STORE_F32)
+        assert (out.double() - ref).norm() <= (plain.double() - ref).norm()
+    # a token's result does not depend on the tokens beside it, nor on the row stride
+    pick = [M - 1] + [i for i in (0, 3, 7) if i < M - 1]
+    wide = torch.randn(len(pick), K + 12, device="cuda", generator=g)
+    wide[:, :K] = x[pick]
+    assert torch.equal(run(ops, wide[:, :K], w), out[pick])
+
+
+def test_gemm_split_values(ops):
+    """Large and small magnitudes keep their relative error; what is not finite comes out as the CUDA cores' kernel gives it."""
+    g = torch.Generator(device="cuda").manual_seed(5)
+    x = torch.randn(70, 1024, device="cuda", generator=g) * 1e18
+    w = torch.randn(256, 1024, device="cuda", generator=g) * 1e-22
+    ref = x.double() @ w.double().T
+    assert ((run(ops, x, w).double() - ref).abs() <= (x.double().abs() @ w.double().abs().T) * 2.0 ** -20).all()
+    x = torch.randn(70, 1024, device="cuda", generator=g)
+    w = torch.randn(256, 1024, device="cuda", generator=g)
+    x[3, 17], x[9, 1000], x[20, 5], x[20, 6] = float("inf"), float("-inf"), float("nan"), 2.0
+    w[100, 40], w[7, 900] = float("inf"), torch.tensor(0x7F800001, dtype=torch.int32).view(torch.float32).item()
+    w[50, 3] = 3.4e38
+    x[30] = 0.0
+    x[31, 3] = 3.4e38
+    w[60] = 0.0
+    got, want = run(ops, x, w), torch.empty(70, 256, device="cuda")
+    ops.gemm_generic(x, w, want, ops.EPI_STORE_F32)
+    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.isinf())
+    inf = want.isinf()
+    assert torch.equal(got[inf], want[inf])
+    fine = want.isfinite()
+    scale = x.nan_to_num(0, 0, 0).double().abs() @ w.nan_to_num(0, 0, 0).double().abs().T
+    assert ((got - want).abs()[fine].double() <= 2.0 ** -14 * scale[fine]).all()
+
+
+def test_gemm_split_linear(ops):
+    """The layers' entry point takes this kernel where its rule says so, and both lanes' scratch is their own."""
+    from ferrum_b200.engine.batch import StepContext
+    from ferrum_b200.parts.linear import RESIDUAL, STORE, linear
+    ctx = StepContext("cuda", 128, 4, [])
+    g = torch.Generator(device="cuda").manual_seed(6)
+    for M, N, K, split in ((64, 2048, 2048, False), (65, 2048, 2048, True), (65, 128, 512, True), (65, 127, 512, False), (65, 128, 508, False)):
+        x = torch.randn(M, K, device="cuda", generator=g)
+        w = torch.randn(N, K, device="cuda", generator=g)
+        assert ops.gemm_split_supported(x, w, M) == split
+        out = torch.zeros(M, N, device="cuda")
+        linear(x, w, out, STORE, ctx, M=M)
+        linear(x, w, out, RESIDUAL, ctx, M=M)
+        assert ((out.double() - 2 * (x.double() @ w.double().T)).abs() <= 2.5e-7 * K * out.abs().max()).all()
+    assert ctx.err.item() == 0
+    a = ctx.gemm_split_scratch(65, 2048, 2048)
+    ctx.lane = 1
+    b = ctx.gemm_split_scratch(65, 2048, 2048)
+    assert {t.data_ptr() for t in a}.isdisjoint({t.data_ptr() for t in b})
