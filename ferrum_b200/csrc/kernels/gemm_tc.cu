@@ -64,6 +64,8 @@ struct TcParams {
   int drop_loads;      // test hook: the producer requests no tile at all, so that the waits for them run out
   int glu_act;         // activation of the gate in the SwiGLU epilogues: 0 silu, 1 gelu (tanh form), 2 the clamped unit
   float glu_limit;     // the clamp of activation 2
+  int bt;              // pair kernel: tokens per tile (a multiple of 32, at most PAIR_BT)
+  int cut;             // pair kernel: left-over tiles are cut among the pairs
   int store_act;       // what the plain 16-bit store applies: 0 nothing, 1 the square of relu
 };
 
@@ -438,8 +440,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
 // ------------------------------------------------------------------ the CTA-pair kernel
 // For many tokens the single-CTA tile (128 weight rows x 256 tokens) asks the L2 for 48 KB
 // per 4.2 MFLOP and the tensor cores wait for operands half of the time.  Here two CTAs of a
-// cluster compute a 256 x 256 tile with one tcgen05.mma.cta_group::2 per K step: each CTA
-// loads its own 128 weight rows and its own 128 tokens (32 KB per stage instead of 48 KB for
+// cluster compute a tile of 256 rows x up to 256 tokens with one tcgen05.mma.cta_group::2 per K step: each CTA
+// loads its own 128 weight rows and its own half of the tokens (at 256, 32 KB per stage instead of 48 KB for
 // the same flops), the leader issues the MMAs, and each CTA's tensor memory receives its 128
 // rows of the product, which its own epilogue warps read back.  Partial tiles are handled as
 // in the single-CTA kernel with the cluster in the role of the CTA and the 128-row half tile
@@ -449,23 +451,23 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
 // on neighbouring tiles at the same k-block and share their operands in the L2.  For the R
 // tiles that are left (fewer than P) there are two ways.  As a rule R clusters take one more
 // whole tile each and the others are done.  Only where that idles much (long tiles, few of
-// them: (P - R) / P of a tile is PAIR_STREAMK_MIN_KB k-blocks or more) the left-over tiles are cut
+// them: the caller decides, see `pair_plan`) the left-over tiles are cut
 // stream-K fashion: their units (tile, k-block) form a line that is divided evenly among the
 // first Pr clusters, and a tile that several clusters share is summed from float32 partials
 // by the cluster that holds its first k-blocks.  That costs some 20 us at the end of the
 // kernel (partials out, a wait, partials in), which is why short tiles are not cut: measured
 // on 2048 x [4096, 14336], cutting 54 left-over tiles of 224 k-blocks (60 k-blocks saved)
-// gains nothing, on 512 x [4096, 14336] (127 saved) it takes 74 us to 60.  Tiles are numbered through groups of
+// gains nothing, on 512 x [4096, 14336] (127 saved) it takes 74 us to 60.  (`pair_plan` mostly finds a narrower token tile
+// that does without; what it cuts is what that cannot fill, as 300 x [4096, 14336]: 71 us whole, 63 cut.)  Tiles are numbered through groups of
 // PAIR_GROUP_T token tiles, token tile fastest: a wave then reads about P / 8 weight tiles and
 // 8 token tiles instead of P weight tiles and one token tile, and with many tokens the
 // weights stream from memory once per group instead of once per token tile.
 constexpr int PAIR_GROUP_T = 8;
-constexpr int PAIR_STREAMK_MIN_KB = 80;
 constexpr int PAIR_FINISHER_POLLS = 200;  // of about a microsecond each: how long a tile's finisher waits for the other partials
 struct PairSchedule {
   int nkb, tiles_n, tiles_t, P, cluster, waves, Pr, whole_extra;
   long long full_tiles, Ur, r_begin, r_end;
-  __host__ __device__ PairSchedule(int tiles_n_, int tiles_t_, int nkb_, int P_, int cluster_)
+  __host__ __device__ PairSchedule(int tiles_n_, int tiles_t_, int nkb_, int P_, int cluster_, bool cut)
       : nkb(nkb_), tiles_n(tiles_n_), tiles_t(tiles_t_), P(P_), cluster(cluster_) {
     const long long tiles = (long long)tiles_n * tiles_t;
     const int R = (int)(tiles % P);
@@ -474,7 +476,7 @@ struct PairSchedule {
     Ur = 0;
     Pr = 0;
     r_begin = r_end = 0;
-    if (R > 0 && (long long)(P - R) * nkb < (long long)PAIR_STREAMK_MIN_KB * P) {
+    if (R > 0 && !cut) {
       whole_extra = R;
     } else if (R > 0) {
       // few tiles left over would each be cut among many clusters: cut the last whole wave with them
@@ -525,27 +527,26 @@ struct PairSchedule {
   __host__ __device__ int slot_of(int cc, long long tile) const { return (Ur * cc / Pr) / nkb == tile - full_tiles ? 0 : 1; }
 };
 
-constexpr int PAIR_BT = 256;                              // tokens per tile pair
-constexpr int PAIR_B_BYTES = (PAIR_BT / 2) * TILE_K * 2;  // each CTA stages half of the tokens
-constexpr int PAIR_STAGE_BYTES = A_BYTES + PAIR_B_BYTES;
-constexpr int PAIR_STAGES = 6;
+constexpr int PAIR_BT = 256;                              // tokens per tile pair at most
+constexpr int PAIR_RING_BYTES = 192 * 1024;               // the ring of operand stages: 6 of 256 tokens, 9 of 64
+constexpr int PAIR_MAX_STAGES = PAIR_RING_BYTES / (A_BYTES + 16 * TILE_K * 2);
 // The epilogue's staging: two buffers of 32 tokens x 128 features (float32 at most).  A thread
 // owns one feature of 32 tokens at a time; written to `out` directly that is 32 scattered
 // read-modify-writes per thread and the epilogue, not the tensor cores, sets the pace of short
 // products.  Staged, the tile leaves as one bulk store (or float32 add) per 32 tokens.
 constexpr int PAIR_OUT_ROWS = 32;
 constexpr int PAIR_OUT_BYTES = PAIR_OUT_ROWS * TILE_N * 4;
-constexpr int PAIR_SMEM_BYTES = PAIR_STAGES * PAIR_STAGE_BYTES + 1024 + 256 + 2 * PAIR_OUT_BYTES;
+constexpr int PAIR_SMEM_BYTES = PAIR_RING_BYTES + 1024 + 256 + 2 * PAIR_OUT_BYTES;
+static_assert((2 * PAIR_MAX_STAGES + 5) * 8 <= 256, "the barriers do not fit their place");
 
 __global__ void __launch_bounds__(192, 1)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                     const __grid_constant__ CUtensorMap tmap_out, const __grid_constant__ CUtensorMap tmap_ws,
                     const TcParams p) {
-  constexpr int STAGES = PAIR_STAGES;
   constexpr int ACC_COLS = PAIR_BT;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  uint64_t* bars = (uint64_t*)(smem + STAGES * PAIR_STAGE_BYTES);  // full[S], empty[S], acc_full[2], acc_empty[2]
+  uint64_t* bars = (uint64_t*)(smem + PAIR_RING_BYTES);  // full[S], empty[S], acc_full[2], acc_empty[2]
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
   __shared__ int is_last;
@@ -555,8 +556,11 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
   const int P = gridDim.x / 2, cluster = blockIdx.x / 2;
   const int nkb = (p.K + TILE_K - 1) / TILE_K;
   const int tiles_n = (p.N + 2 * TILE_N - 1) / (2 * TILE_N);  // 256-row tiles
-  const int tiles_t = (p.M + PAIR_BT - 1) / PAIR_BT;
-  const PairSchedule sched(tiles_n, tiles_t, nkb, P, cluster);
+  const int bt = p.bt;
+  const int tiles_t = (p.M + bt - 1) / bt;
+  const PairSchedule sched(tiles_n, tiles_t, nkb, P, cluster, p.cut != 0);
+  const int stage_bytes = A_BYTES + bt / 2 * TILE_K * 2;   // each CTA stages half of the tile's tokens
+  const int STAGES = PAIR_RING_BYTES / stage_bytes;
 
   const uint32_t smem_base = smem_u32(smem);
   const uint32_t bar_base = smem_u32(bars);
@@ -612,7 +616,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         int n_idx, t_idx;
         sched.coords(tile, n_idx, t_idx);
         const int n0 = n_idx * 2 * TILE_N + (int)rank * TILE_N;
-        const int t0 = t_idx * PAIR_BT + (int)rank * (PAIR_BT / 2);
+        const int t0 = t_idx * bt + (int)rank * (bt / 2);
         for (int kb = kb0; kb < kb1; ++kb) {
           if (!mbar_wait(empty_bar(s), phase ^ 1, abort_p, wait_limit)) {
             abort_flag = 1;
@@ -620,9 +624,9 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             ok = false;
             break;
           }
-          const uint32_t a = smem_base + s * PAIR_STAGE_BYTES;
+          const uint32_t a = smem_base + s * stage_bytes;
           const uint32_t leader_full = map_to_cta(full_bar(s), 0);  // (measured: this loop is not the limit; the copies are)
-          if (rank == 0) mbar_expect_tx(full_bar(s), 2 * PAIR_STAGE_BYTES);
+          if (rank == 0) mbar_expect_tx(full_bar(s), 2 * stage_bytes);
           if (p.gated) tma_load_3d_pair(a, &tmap_w, leader_full, kb * TILE_K, 0, n0 >> 1);  // (k, gate | up, feature)
           else tma_load_2d_pair(a, &tmap_w, leader_full, kb * TILE_K, n0);
           tma_load_2d_pair(a + A_BYTES, &tmap_x, leader_full, kb * TILE_K, t0);
@@ -636,7 +640,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (leader only)
     if (rank == 0 && elect_one()) {
-      const uint32_t idesc = umma_idesc_16bit(2 * TILE_N, PAIR_BT, p.half != 0);
+      const uint32_t idesc = umma_idesc_16bit(2 * TILE_N, bt, p.half != 0);
       const uint64_t desc0 = umma_desc_k_sw128(smem_base);
       int s = 0;
       uint32_t phase = 0;
@@ -661,7 +665,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             break;
           }
           tc_fence_after();
-          const uint64_t a_desc = desc0 + (uint64_t)(s * (PAIR_STAGE_BYTES >> 4));
+          const uint64_t a_desc = desc0 + (uint64_t)(s * (stage_bytes >> 4));
           const uint64_t b_desc = a_desc + (A_BYTES >> 4);
 #pragma unroll
           for (int kk = 0; kk < TILE_K / UMMA_K; ++kk) {
@@ -685,7 +689,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
     const int ep_tid = threadIdx.x - 64;
     const uint32_t lane_addr = tmem_base + ((uint32_t)(quarter * 32) << 16);
     const size_t tile_floats = (size_t)ACC_COLS * TILE_N;
-    uint8_t* out_stage = smem + STAGES * PAIR_STAGE_BYTES + 256;
+    uint8_t* out_stage = smem + PAIR_RING_BYTES + 256;
     const bool staged = p.out_tma != 0;
     int emitted = 0;  // staged stores issued so far; buffer = emitted & 1
     pdl_wait();
@@ -766,7 +770,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
       tc_fence_after();
       int n_idx, t_idx;
       sched.coords(tile, n_idx, t_idx);
-      const int n0 = n_idx * 2 * TILE_N + (int)rank * TILE_N, t0 = t_idx * PAIR_BT;
+      const int n0 = n_idx * 2 * TILE_N + (int)rank * TILE_N, t0 = t_idx * bt;
       const int n = n0 + n_local;
       const uint32_t acc_addr = lane_addr + buf * ACC_COLS;
       const uint32_t leader_acc_empty = map_to_cta(acc_empty_bar(buf), 0);
@@ -776,7 +780,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         float* out = (float*)p.out + (size_t)t0 * p.ldo + n;
         const size_t ld = (size_t)p.ldo;
 #pragma unroll 1
-        for (int c0 = 0; c0 < PAIR_BT; c0 += 32) {
+        for (int c0 = 0; c0 < bt; c0 += 32) {
           const int valid = n < p.N ? p.M - t0 - c0 : 0;
           float r[32], v[32];
 #pragma unroll
@@ -792,7 +796,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         if (lane == 0) mbar_arrive_cluster(leader_acc_empty);
       } else if (whole && p.gated) {
 #pragma unroll 1
-        for (int c0 = 0; c0 < PAIR_BT && t0 + c0 < p.M; c0 += 32) {
+        for (int c0 = 0; c0 < bt && t0 + c0 < p.M; c0 += 32) {
           float v[32];
           tmem_ld16(acc_addr + c0, &v[0]);
           tmem_ld16(acc_addr + c0 + 16, &v[16]);
@@ -803,7 +807,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         if (lane == 0) mbar_arrive_cluster(leader_acc_empty);
       } else if (whole) {
 #pragma unroll 1
-        for (int c0 = 0; c0 < PAIR_BT && t0 + c0 < p.M; c0 += 32) {
+        for (int c0 = 0; c0 < bt && t0 + c0 < p.M; c0 += 32) {
           float v[32];
           tmem_ld16(acc_addr + c0, &v[0]);
           tmem_ld16(acc_addr + c0 + 16, &v[16]);
@@ -830,7 +834,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
           int a2, b2;
           const int others = n_contrib - 1;
           // columns per pass: what the stages hold of `others` partials (512 bytes per column)
-          const int pass_cols = min(PAIR_BT, (int)((STAGES * PAIR_STAGE_BYTES) / (others * TILE_N * 4)) & ~31);
+          const int pass_cols = min(bt, (int)(PAIR_RING_BYTES / (others * TILE_N * 4)) & ~31);
           const bool finisher = staged && cluster == c_first && pass_cols >= 32 && !sched.segment(seg + 1, t2, a2, b2);
           if (finisher) {
             if (ep_tid == 0) {
@@ -845,8 +849,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
           if (fast) {
             const float* fetched = (const float*)smem;  // [contributor][column][128 rows]
             bool fine = true;
-            for (int cb = 0; cb < PAIR_BT && t0 + cb < p.M && fine; cb += pass_cols) {
-              const int ncols = min(pass_cols, PAIR_BT - cb);
+            for (int cb = 0; cb < bt && t0 + cb < p.M && fine; cb += pass_cols) {
+              const int ncols = min(pass_cols, bt - cb);
               if (ep_tid == 0) {
                 fence_proxy_async();  // the threads' reads of the pass before precede these copies
                 mbar_expect_tx(fetch_bar, (uint32_t)(others * ncols * TILE_N * 4));
@@ -893,7 +897,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
           // the partial leaves like the output: 32 columns at a time through shared memory, as bulk
           // stores into the workspace seen as rows of 128 floats
 #pragma unroll 1
-          for (int c0 = 0; c0 < ACC_COLS; c0 += 32) {
+          for (int c0 = 0; c0 < bt; c0 += 32) {
             float v[32];
             tmem_ld16(acc_addr + c0, &v[0]);
             tmem_ld16(acc_addr + c0 + 16, &v[16]);
@@ -905,7 +909,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
           if (ep_tid == 0) bulk_wait_all();  // the partial is written before it is announced
         } else {
 #pragma unroll 1
-          for (int c0 = 0; c0 < ACC_COLS; c0 += 16) {
+          for (int c0 = 0; c0 < bt; c0 += 16) {
             float v[16];
             tmem_ld16(acc_addr + c0, v);
 #pragma unroll
@@ -932,7 +936,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
           const int q4 = (ep_tid & 31) * 4, cg = (ep_tid >> 5) * 8;
           auto slot_of = [&](int cc) { return ((size_t)cc * 2 + sched.slot_of(cc, tile)) * 2 + rank; };
 #pragma unroll 1
-          for (int c0 = 0; c0 < PAIR_BT && t0 + c0 < p.M; c0 += 32) {
+          for (int c0 = 0; c0 < bt && t0 + c0 < p.M; c0 += 32) {
             float4 acc[8];
 #pragma unroll
             for (int k = 0; k < 8; ++k) acc[k] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -980,7 +984,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         } else if (is_last) {  // the same for the four warps: they go through emit32 together
           __threadfence();
 #pragma unroll 1
-          for (int c0 = 0; c0 < PAIR_BT && t0 + c0 < p.M; c0 += 32) {
+          for (int c0 = 0; c0 < bt && t0 + c0 < p.M; c0 += 32) {
             float a0[32];
 #pragma unroll
             for (int j = 0; j < 32; ++j) a0[j] = 0.f;
@@ -1169,6 +1173,46 @@ static int sm_count() {
   return n;
 }
 
+// How the pair kernel cuts M tokens x `rows` weight rows over K among `pairs` pairs: the width of its token tiles, and
+// whether left-over tiles are cut along K.  256 tokens a tile is the cheapest per token, but a step of a few hundred
+// tokens has too few such tiles for the pairs (12 tiles of [3072, K] on 74 pairs), or a last wave that is nearly empty.
+// The estimate behind the choice: a pair's time is its k-blocks times what one costs.  A k-block of 64 elements took, in
+// units of one at 128 tokens (0.26 us): 0.92 at 64 tokens, 0.96 at 96, 1.07 at 160, 1.16 at 192, 1.33 at 224, 1.50 at
+// 256 (single waves of K = 3,072 to 14,336 and 49 to 13 waves of 2,048 x [28672, 4096]): up to 160 tokens it is the copies of
+// the weight tiles, the same whatever the tile, above that the products and the token tiles.  Cutting costs the partials
+// and the wait for them, some 15 k-blocks for every 32 tokens of a tile.  A narrower tile has to promise 5 %: on long steps
+// the power limit sets the clock, and the wider tile moves fewer bytes (192 tokens a tile for 2,048 x [28672, 4096]: 2 %
+// by the estimate, and a whole 2,048-token step 4 % slower).
+// Measured on a B200, us, 256 tokens a tile with the cut -> this choice: 391 x [5120, 3072] 24.5 -> 18.5, 391 x [3072, 3072]
+// 22.0 -> 15.5, 391 x [3072, 8192] 45 -> 28..38, 512 x [12288, 4096] 60 -> 45, 512 x [4096, 4096] 37 -> 19..26, 300 x 2 x [8192, 3072]
+// 47 -> 38, 1,024 x [6144, 4096] 74..81 -> 41..65, 2,048 x [3072, 8192] 90 -> 80; 2,048 x [4096, 4096] stays at 51..54.
+struct PairPlan {
+  int bt, tiles_t;
+  bool cut;
+};
+static long long pair_cost(long long tiles, long long nkb, int pairs, int bt, bool* cut) {
+  const long long block = std::max(672 + bt, 47 * bt / 10);      // (a k-block at 128 tokens: 800)
+  const long long whole = (tiles + pairs - 1) / pairs * nkb * block;
+  const long long shared = (tiles * nkb + pairs - 1) / pairs * block + 380LL * bt;
+  *cut = tiles % pairs != 0 && shared < whole;
+  return *cut ? shared : whole;
+}
+static PairPlan pair_plan(int M, long long rows, int K, int pairs) {
+  const long long tiles_n = (rows + 2 * TILE_N - 1) / (2 * TILE_N);
+  PairPlan best{PAIR_BT, 1, false};
+  long long best_cost = -1;
+  for (int bt = PAIR_BT; bt >= 64; bt -= 32) {
+    const int tiles_t = (M + bt - 1) / bt;
+    bool cut;
+    const long long cost = pair_cost(tiles_n * tiles_t, (K + TILE_K - 1) / TILE_K, pairs, bt, &cut);
+    if (best_cost < 0 || cost * 20 < best_cost * 19) {      // (5 %: of two that are as quick the wider one moves less)
+      best_cost = cost;
+      best = PairPlan{bt, tiles_t, cut};
+    }
+  }
+  return best;
+}
+
 // The token-tile width the kernel uses for M tokens.
 FERRUM_API int ferrum_gemm_tc_token_tile(int M, int dual) {
   if (M <= 16) return 16;
@@ -1181,15 +1225,21 @@ FERRUM_API int ferrum_gemm_tc_token_tile(int M, int dual) {
 // The grid the kernel runs with when the caller passes n_ctas = 0: one CTA per SM.
 FERRUM_API int ferrum_gemm_tc_default_ctas() { return sm_count(); }
 
+// The single-CTA kernel's counters: one per 128-row tile (rounded up to pairs of them).
+static long long single_cta_tiles(int M, int N, int bt) { return 2LL * ((N + 2 * TILE_N - 1) / (2 * TILE_N)) * ((M + bt - 1) / bt); }
+
 // Workspace floats and tile counters a launch needs.  Partial tiles arise where a CTA's
 // range of units begins or ends inside a tile, so every CTA has two partial slots.
 FERRUM_API long long ferrum_gemm_tc_workspace(int M, int N, int K, int dual, int n_ctas, int* n_tiles) {
   const int bt = ferrum_gemm_tc_token_tile(M, dual);
   if (n_ctas <= 0) n_ctas = sm_count();
-  // counters: one per 128-row tile; the pair kernel numbers them by 256-row tile and half
-  long long tiles = 2LL * ((N + 2 * TILE_N - 1) / (2 * TILE_N)) * ((M + bt - 1) / bt);
-  if (dual && M > TILE_N)  // may run on the pair kernel as one product of 2 N interleaved rows
-    tiles = std::max(tiles, 2LL * ((2LL * N + 2 * TILE_N - 1) / (2 * TILE_N)) * ((M + PAIR_BT - 1) / PAIR_BT));
+  long long tiles = single_cta_tiles(M, N, bt);
+  if (M > 0 && n_ctas >= 2 && (dual ? M > TILE_N : bt == PAIR_BT)) {
+    // may run on the pair kernel (gate and up as one product of 2 N interleaved rows): it numbers the counters by 256-row tile and half
+    const long long rows = dual ? 2LL * N : N;
+    const PairPlan plan = pair_plan(M, rows, K, n_ctas / 2);
+    if (plan.cut) tiles = std::max(tiles, 2LL * ((rows + 2 * TILE_N - 1) / (2 * TILE_N)) * plan.tiles_t);
+  }
   if (n_tiles) *n_tiles = (int)tiles;
   return 2LL * n_ctas * (long long)(bt * (dual ? 2 : 1)) * TILE_N;
 }
@@ -1224,6 +1274,7 @@ FERRUM_API int ferrum_gemm_tc(const void* x, const void* w, void* out, int dtype
   const long long need = ferrum_gemm_tc_workspace(M, N, K, dual, n_ctas, &tiles);
   FERRUM_CHECK_ARG(workspace && workspace_floats >= need, "gemm_tc: needs %lld workspace floats, got %lld", need, workspace_floats);
   FERRUM_CHECK_ARG(counters && n_counters >= tiles, "gemm_tc: needs %d tile counters, got %d", tiles, n_counters);
+  const int asked_ctas = n_ctas;      // (what the workspace was sized with)
   {
     // every CTA must own at least one unit, or the CTAs that share a tile are not consecutive
     const long long units = (long long)((N + TILE_N - 1) / TILE_N) * ((M + bt - 1) / bt) * ((K + TILE_K - 1) / TILE_K);
@@ -1245,12 +1296,15 @@ FERRUM_API int ferrum_gemm_tc(const void* x, const void* w, void* out, int dtype
     p.N = 2 * N;
     p.gated = 1;
     p.stream_weights = 0;
-    const long long units = (long long)((p.N + 2 * TILE_N - 1) / (2 * TILE_N)) * ((M + PAIR_BT - 1) / PAIR_BT) * ((K + TILE_K - 1) / TILE_K);
-    int pairs = n_ctas / 2;
+    const PairPlan plan = pair_plan(M, p.N, K, asked_ctas / 2);
+    p.bt = plan.bt;
+    p.cut = plan.cut;
+    const long long units = (long long)((p.N + 2 * TILE_N - 1) / (2 * TILE_N)) * plan.tiles_t * ((K + TILE_K - 1) / TILE_K);
+    int pairs = asked_ctas / 2;
     if (pairs > units) pairs = (int)units;
     CUtensorMap mo, ms;
     if (int r = get_tensor_map(w, N, K, ldw, dual_offset, &mw, 4)) return r;
-    if (int r = get_tensor_map(x, M, K, ldx, PAIR_BT / 2, &mx)) return r;
+    if (int r = get_tensor_map(x, M, K, ldx, plan.bt / 2, &mx)) return r;
     if (int r = get_tensor_map(out, M, N, ldo, PAIR_OUT_ROWS, &mo, 3)) return r;
     FERRUM_CHECK_ARG(((uintptr_t)workspace & 15) == 0, "gemm_tc: the workspace must be 16-byte aligned");
     if (int r = get_tensor_map(workspace, workspace_floats / TILE_N, TILE_N, TILE_N, PAIR_OUT_ROWS, &ms, 1)) return r;
@@ -1260,10 +1314,13 @@ FERRUM_API int ferrum_gemm_tc(const void* x, const void* w, void* out, int dtype
   if (int r = get_tensor_map(w, w_rows, K, ldw, TILE_N, &mw)) return r;
   if (bt == PAIR_BT && !dual && g_pair_kernel && n_ctas >= 2) {
     // many tokens: pairs of CTAs on 256 x 256 tiles; each CTA stages 128 tokens
-    const long long units = (long long)((N + 2 * TILE_N - 1) / (2 * TILE_N)) * ((M + PAIR_BT - 1) / PAIR_BT) * ((K + TILE_K - 1) / TILE_K);
-    int pairs = n_ctas / 2;
+    const PairPlan plan = pair_plan(M, N, K, asked_ctas / 2);
+    p.bt = plan.bt;
+    p.cut = plan.cut;
+    const long long units = (long long)((N + 2 * TILE_N - 1) / (2 * TILE_N)) * plan.tiles_t * ((K + TILE_K - 1) / TILE_K);
+    int pairs = asked_ctas / 2;
     if (pairs > units) pairs = (int)units;
-    if (int r = get_tensor_map(x, M, K, ldx, PAIR_BT / 2, &mx)) return r;
+    if (int r = get_tensor_map(x, M, K, ldx, plan.bt / 2, &mx)) return r;
     // the output through a tensor map where its rows are 16-byte multiples; else by the threads
     CUtensorMap mo = mw;
     const int esize = epilogue == TC_RESIDUAL ? 4 : 2;
@@ -1295,15 +1352,25 @@ FERRUM_API int ferrum_gemm_tc(const void* x, const void* w, void* out, int dtype
   FERRUM_CHECK_ARG(false, "gemm_tc: no kernel for token tile %d", bt);
 }
 
+// For tests on the host: out[0..2] = tokens per tile, token tiles and whether tiles are cut, as `pair_plan` chooses.
+FERRUM_API void ferrum_gemm_pair_plan(int M, long long rows, int K, int pairs, int* out) {
+  const PairPlan plan = pair_plan(M, rows, K, pairs);
+  out[0] = plan.bt;
+  out[1] = plan.tiles_t;
+  out[2] = plan.cut;
+}
+
 // For tests of the schedule on the host: pair `cluster`'s s-th segment when `pairs` pairs
-// compute M tokens x `rows` weight rows (for gate and up as one product: both) over K.
+// compute M tokens x `rows` weight rows (for gate and up as one product: both) over K in tiles of 256 tokens.
 // out[0..7] = tile, first k-block, one past the last, weight tile index, token tile index, and
 // for a tile that pairs share its first and last contributor and the slot (0 or 1) of this
 // pair's partial (-1 each for a whole tile).  Returns 0 when the pair has no such segment.
 FERRUM_API int ferrum_gemm_pair_schedule(int M, long long rows, int K, int pairs, int cluster, int s, long long* out) {
   const int nkb = (K + TILE_K - 1) / TILE_K;
   const int tiles_n = (int)((rows + 2 * TILE_N - 1) / (2 * TILE_N)), tiles_t = (M + PAIR_BT - 1) / PAIR_BT;
-  const PairSchedule sched(tiles_n, tiles_t, nkb, pairs, cluster);
+  bool cut;
+  pair_cost((long long)tiles_n * tiles_t, nkb, pairs, PAIR_BT, &cut);
+  const PairSchedule sched(tiles_n, tiles_t, nkb, pairs, cluster, cut);
   long long tile;
   int kb0, kb1, n_idx, t_idx;
   if (!sched.segment(s, tile, kb0, kb1)) return 0;
@@ -1445,6 +1512,7 @@ FERRUM_API int ferrum_gemm_tc_noalloc(const void* x, const void* w, void* out, i
   const int bt = ferrum_gemm_tc_token_tile(M, dual);
   int tiles = 0;
   const long long need_floats = ferrum_gemm_tc_workspace(M, N, K, dual, n_ctas, &tiles);
+  tiles = (int)single_cta_tiles(M, N, bt);       // (this entry never takes the pair kernel)
   FERRUM_CHECK_ARG(need_floats * (long long)sizeof(float) <= (long long)FERRUM_NOALLOC_SCRATCH_BYTES,
                    "gemm_tc_noalloc: %d tokens%s need %lld bytes of scratch, the built-in array holds %u; use ferrum_gemm_tc "
                    "with a caller-provided workspace", M, dual ? " with the SwiGLU epilogue" : "",
