@@ -17,6 +17,8 @@ from typing import Dict, List, Sequence
 import numpy as np
 import torch
 
+from ..ops import lib as ops
+
 
 @dataclass
 class StepEntry:
@@ -41,11 +43,20 @@ class Scratch:
     def __init__(self, device, guard=None):
         self.device = device
         self._bufs: Dict[str, torch.Tensor] = {}
+        self._views: Dict[str, tuple] = {}     # name -> (shape, dtype, view): the last view handed out (a step asks for the same one in every layer)
         self._guards: Dict[str, torch.Tensor] = {}
         self.generation = 0      # bumped whenever a buffer is (re)allocated and so may have moved
         self.guard = int(os.environ.get("FERRUM_CANARY", "0") == "1") * 64 if guard is None else int(guard)
 
     def get(self, name, shape, dtype):
+        last = self._views.get(name)
+        if last is not None and last[0] == shape and last[1] is dtype:
+            return last[2]
+        view = self._get(name, shape, dtype)
+        self._views[name] = (shape, dtype, view)
+        return view
+
+    def _get(self, name, shape, dtype):
         n = 1
         for s in shape:
             n *= int(s)
@@ -98,7 +109,7 @@ class PinnedRing:
         if self.cuda:
             if self.events[self.i] is None:
                 self.events[self.i] = torch.cuda.Event()
-            self.events[self.i].record()
+            self.events[self.i].record(ops.current_stream())
 
 
 class PlanStore:
@@ -280,22 +291,18 @@ class StepContext:
         into several residual streams."""
         p = self.pending_residual
         if p is not None:
-            from ..ops import lib as ops
             self.pending_residual = None
             ops.residual_reduce(p[0], self.n_tokens, p[1])
         p = self.pending_streams
         if p is not None:
-            from ..ops import lib as ops
             self.pending_streams = None
             ops.hyper_step(p[0], p[1], p[2], self.n_tokens, write=p[3], store=True)
         p = self.pending_add
         if p is not None:
-            from ..ops import lib as ops
             self.pending_add = None
             ops.norm_scaled_add(p[0], p[1].y, p[1].w, p[1].mult, p[1].eps, self.n_tokens, partials=p[1].partials)
         p = self.pending_experts
         if p is not None:
-            from ..ops import lib as ops
             self.pending_experts = None
             ops.moe_combine(p[1].rows, p[1].row_of, p[1].top, self.n_tokens, p[0], weight_of=p[1].weight_of, accumulate=True)
 
@@ -345,19 +352,15 @@ class StepContext:
 
     def gemm_scratch(self, M, N, K, dual):
         """(float32 workspace, zeroed int32 tile counters) for the tensor-core product."""
-        from ..ops import lib as ops
         floats, tiles = ops.gemm_tc_workspace(M, N, K, dual)
-        if self.lane:
-            if tiles > self._splitk_counters_side.numel():
-                self._splitk_counters_side = torch.zeros(2 * tiles, dtype=torch.int32, device=self.device)
-            return self.scratch.get("gemm_partials_side", (floats,), torch.float32), self._splitk_counters_side
-        if tiles > self._splitk_counters.numel():
-            self._splitk_counters = torch.zeros(2 * tiles, dtype=torch.int32, device=self.device)
-        return self.scratch.get("gemm_partials", (floats,), torch.float32), self._splitk_counters
+        name = "_splitk_counters_side" if self.lane else "_splitk_counters"
+        if tiles > getattr(self, name).numel():
+            setattr(self, name, torch.zeros(2 * tiles, dtype=torch.int32, device=self.device))
+            self.scratch.generation += 1       # (a captured graph would go on counting in the old ones)
+        return self.scratch.get("gemm_partials_side" if self.lane else "gemm_partials", (floats,), torch.float32), getattr(self, name)
 
     def gemm_split_scratch(self, M, N, K):
         """(tokens' parts, partial sums) for the float32 product on the tensor cores."""
-        from ..ops import lib as ops
         parts, partials = ops.gemm_split_workspace(M, N, K)
         lane = "_side" if self.lane else ""
         return (self.scratch.get("gemm_split_parts" + lane, (parts,), torch.float32),

@@ -50,6 +50,21 @@ def lib():
     return _lib
 
 
+_streams = {}
+
+
+def current_stream():
+    """The current CUDA stream as a torch object, made once per handle (torch makes a new one on every call)."""
+    if _raw_stream is None:
+        return torch.cuda.current_stream()
+    key = _device_index()
+    raw = _raw_stream(key)
+    known = _streams.get(key)
+    if known is None or known.cuda_stream != raw:
+        known = _streams[key] = torch.cuda.current_stream()
+    return known
+
+
 def require_cuda(device=None):
     if not torch.cuda.is_available():
         raise KernelError("ferrum_b200 runs on a CUDA device only (sm_100a); none is visible")
@@ -171,16 +186,23 @@ def _ptr(t):
 
 
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_device_index = getattr(torch._C, "_cuda_getDevice", None) or torch.cuda.current_device
 
 
 def _stream():
     """The current CUDA stream's handle (the capture stream inside a graph capture)."""
     if _raw_stream is not None:
-        return c_void_p(_raw_stream(torch.cuda.current_device()))
+        return c_void_p(_raw_stream(_device_index()))
     return c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
+# The entry points are called a few hundred times a step, and a step of a few hundred tokens that is launched kernel by
+# kernel waits for them: Python's share of a launch was some 16 us.  So the wrappers of the kernels that every layer launches
+# hand plain integers to ctypes (it passes them as C ints; a c_int object each is another 0.1 us), and the checks
+# below answer for the usual operand, a contiguous tensor, with a few attribute reads.
 def _need(t, dtype, name, ndim=None):
+    if type(t) is torch.Tensor and t.is_cuda and (dtype is None or t.dtype is dtype) and (ndim is None or t.ndim == ndim) and t.is_contiguous():
+        return
     if not isinstance(t, torch.Tensor) or not t.is_cuda:
         raise KernelError(f"{name} must be a CUDA tensor")
     if dtype is not None and t.dtype != dtype:
@@ -222,13 +244,13 @@ def embedding(table, ids, out, err, scale=1.0, pos_table=None, positions=None, c
             _need(pos_table, table.dtype, "pos_table", 2); _need(positions, torch.int32, "positions", 1)
             if pos_table.shape[1] != E or not pos_table.is_contiguous() or positions.shape[0] < T:
                 raise KernelError("embedding: pos_table must be contiguous [positions, E]")
-        _check(lib().ferrum_embedding_scaled(_ptr(table), dtype_code(table.dtype), _ptr(ids), _ptr(out), c_int(T), c_int(E),
-                                             c_int(V), c_float(scale), _ptr(pos_table), _ptr(positions),
-                                             c_int(pos_table.shape[0] if pos_table is not None else 0), _ptr(err),
+        _check(lib().ferrum_embedding_scaled(_ptr(table), dtype_code(table.dtype), _ptr(ids), _ptr(out), T, E,
+                                             V, c_float(scale), _ptr(pos_table), _ptr(positions),
+                                             pos_table.shape[0] if pos_table is not None else 0, _ptr(err),
                                              _stream()), "embedding_scaled")
         return
-    _check(lib().ferrum_embedding(_ptr(table), dtype_code(table.dtype), _ptr(ids), _ptr(out), c_int(T), c_int(E),
-                                  c_int(V), _ptr(err), c_int(copies), _stream()), "embedding")
+    _check(lib().ferrum_embedding(_ptr(table), dtype_code(table.dtype), _ptr(ids), _ptr(out), T, E,
+                                  V, _ptr(err), copies, _stream()), "embedding")
 
 
 def embedding_norm(table, ids, w, eps, out, err, copy=None):
@@ -346,29 +368,29 @@ def rmsnorm(x, weight, out, eps, rows=None, n_rows=None, partials=None, groups=1
     if groups != 1:
         if partials is not None:
             raise KernelError("rmsnorm: a grouped norm takes no pending product")
-        _check(lib().ferrum_group_norm(_ptr(x), _ptr(weight), _ptr(out), dtype_code(out.dtype), _ptr(rows), c_int(n_rows),
-                                       c_int(E), c_int(groups), c_float(eps), _stream()), "group_norm")
+        _check(lib().ferrum_group_norm(_ptr(x), _ptr(weight), _ptr(out), dtype_code(out.dtype), _ptr(rows), n_rows,
+                                       E, groups, c_float(eps), _stream()), "group_norm")
         return
     if partials is not None:
         _check(lib().ferrum_rmsnorm_reduce(_ptr(x), _ptr(weight), _ptr(out), dtype_code(out.dtype), _ptr(rows),
-                                           c_int(n_rows), c_int(E), c_float(eps), _ptr(partials.workspace), partials._c,
+                                           n_rows, E, c_float(eps), _ptr(partials.workspace), partials._c,
                                            _stream()), "rmsnorm_reduce")
         return
-    _check(lib().ferrum_rmsnorm(_ptr(x), _ptr(weight), _ptr(out), dtype_code(out.dtype), _ptr(rows), c_int(n_rows),
-                                c_int(E), c_float(eps), _stream()), "rmsnorm")
+    _check(lib().ferrum_rmsnorm(_ptr(x), _ptr(weight), _ptr(out), dtype_code(out.dtype), _ptr(rows), n_rows,
+                                E, c_float(eps), _stream()), "rmsnorm")
 
 
 def residual_reduce(h, n_rows, partials):
     """h[:n_rows] += the deferred product."""
     _need(h, torch.float32, "h", 2)
-    _check(lib().ferrum_residual_reduce(_ptr(h), c_int(n_rows), c_int(h.shape[1]), _ptr(partials.workspace), partials._c,
+    _check(lib().ferrum_residual_reduce(_ptr(h), n_rows, h.shape[1], _ptr(partials.workspace), partials._c,
                                         _stream()), "residual_reduce")
 
 
 def swiglu_reduce(act, n_tokens, F, partials):
     """act[t, f] = silu(gate) * up from a deferred two-product launch."""
     _need16(act, "act", 2)
-    _check(lib().ferrum_swiglu_reduce(_ptr(act), dtype_code(act.dtype), c_int(n_tokens), c_int(F), c_int(act.stride(0)), _ptr(partials.workspace),
+    _check(lib().ferrum_swiglu_reduce(_ptr(act), dtype_code(act.dtype), n_tokens, F, act.stride(0), _ptr(partials.workspace),
                                       partials._c, _stream()), "swiglu_reduce")
 
 
@@ -389,8 +411,8 @@ def gemm_tc_deferred(x, w, err, workspace, M=None, N=None, dual_offset=0, n_ctas
         raise KernelError(f"gemm_tc_deferred: shapes do not agree: x {tuple(x.shape)} w {tuple(w.shape)}")
     layout = (c_int * 4)()
     _gemm_work(x, w, workspace, M, N, K, 2 if dual_offset else 1)
-    _check(lib().ferrum_gemm_tc_deferred(_ptr(x), _ptr(w), dtype_code(x.dtype), c_int(M), c_int(N), c_int(K), c_int(x.stride(0)),
-                                         c_int(w.stride(0)), c_int(w.shape[0]), c_int(dual_offset), c_int(n_ctas),
+    _check(lib().ferrum_gemm_tc_deferred(_ptr(x), _ptr(w), dtype_code(x.dtype), M, N, K, x.stride(0),
+                                         w.stride(0), w.shape[0], dual_offset, n_ctas,
                                          _ptr(workspace), c_longlong(workspace.numel()), layout, _ptr(err), _stream()),
            "gemm_tc_deferred")
     return Partials(workspace, tuple(layout))
@@ -407,8 +429,8 @@ def gemm_generic(x, w, out, epilogue, M=None):
     if out.dtype != want:
         raise KernelError(f"gemm: out must be {want} for epilogue {epilogue}")
     _gemm_work(x, w, out, M, N, K)
-    _check(lib().ferrum_gemm_generic(_ptr(x), _ptr(w), _ptr(out), dtype_code(x.dtype), c_int(M), c_int(N), c_int(K),
-                                     c_int(x.stride(0)), c_int(w.stride(0)), c_int(out.stride(0)), c_int(epilogue),
+    _check(lib().ferrum_gemm_generic(_ptr(x), _ptr(w), _ptr(out), dtype_code(x.dtype), M, N, K,
+                                     x.stride(0), w.stride(0), out.stride(0), epilogue,
                                      _stream()), "gemm_generic")
 
 
@@ -448,8 +470,8 @@ def gemm_split(x, w, out, err, parts, partials, M=None, add=False):
     if x.shape[1] != K or out.shape[1] < N or out.shape[0] < M or x.shape[0] < M:
         raise KernelError(f"gemm_split: shapes do not agree: x {tuple(x.shape)} w {tuple(w.shape)} out {tuple(out.shape)}")
     _gemm_work(x, w, out, M, N, K)
-    _check(lib().ferrum_gemm_split(_ptr(x), _ptr(w), _ptr(out), c_int(M), c_int(N), c_int(K), c_int(x.stride(0)), c_int(w.stride(0)),
-                                   c_int(out.stride(0)), c_int(1 if add else 0), _ptr(parts), c_longlong(parts.numel()), _ptr(partials),
+    _check(lib().ferrum_gemm_split(_ptr(x), _ptr(w), _ptr(out), M, N, K, x.stride(0), w.stride(0),
+                                   out.stride(0), 1 if add else 0, _ptr(parts), c_longlong(parts.numel()), _ptr(partials),
                                    c_longlong(partials.numel()), _ptr(err), _stream()), "gemm_split")
     launches += (1 + (partials.numel() > 0)) if M else 0      # (the tokens' parts and the sum of the ranges have kernels of their own)
 
@@ -483,9 +505,9 @@ def thin_linear(x, w, out, M, err, table=None, offset=0, token_ids=None):
     if x.shape[1] != K or out.shape[1] < N or min(x.shape[0], out.shape[0]) < M or (kind and out.dtype != x.dtype):
         raise KernelError("thin_linear: shapes do not agree")
     _gemm_work(x, w, out, M, N, K)
-    _check(lib().ferrum_thin_linear(_ptr(x), c_int(x.stride(0)), _ptr(w), dtype_code(x.dtype), c_int(M), c_int(N), c_int(K), c_int(kind),
-                                    _ptr(out), c_int(out.stride(0)), _ptr(table), c_int(table.stride(0) if table is not None else 0),
-                                    c_int(table.shape[0] if table is not None else 0), c_int(offset), _ptr(token_ids), _ptr(err),
+    _check(lib().ferrum_thin_linear(_ptr(x), x.stride(0), _ptr(w), dtype_code(x.dtype), M, N, K, kind,
+                                    _ptr(out), out.stride(0), _ptr(table), table.stride(0) if table is not None else 0,
+                                    table.shape[0] if table is not None else 0, offset, _ptr(token_ids), _ptr(err),
                                     _stream()), "thin_linear")
 
 
@@ -526,10 +548,10 @@ def gemm_tc(x, w, out, epilogue, err, workspace, counters, M=None, N=None, dual_
     _need(workspace, torch.float32, "workspace")
     _need(counters, torch.int32, "counters")
     _gemm_work(x, w, out, M, N, K, 2 if dual_offset else 1)
-    _check(lib().ferrum_gemm_tc(_ptr(x), _ptr(w), _ptr(out), dtype_code(x.dtype), c_int(M), c_int(N), c_int(K), c_int(x.stride(0)),
-                                c_int(w.stride(0)), c_int(out.stride(0)), c_int(w.shape[0]), c_int(epilogue),
-                                c_int(dual_offset), c_int(n_ctas), _ptr(workspace), c_longlong(workspace.numel()),
-                                _ptr(counters), c_int(counters.numel()), _ptr(err), c_float(glu_limit), _stream()), "gemm_tc")
+    _check(lib().ferrum_gemm_tc(_ptr(x), _ptr(w), _ptr(out), dtype_code(x.dtype), M, N, K, x.stride(0),
+                                w.stride(0), out.stride(0), w.shape[0], epilogue,
+                                dual_offset, n_ctas, _ptr(workspace), c_longlong(workspace.numel()),
+                                _ptr(counters), counters.numel(), _ptr(err), c_float(glu_limit), _stream()), "gemm_tc")
 
 
 def rope_cache_write(qkv, n_tokens, positions, req_of_token, block_table, cos_sin, kv_plane, page_stride, page_size,
@@ -549,12 +571,12 @@ def rope_cache_write(qkv, n_tokens, positions, req_of_token, block_table, cos_si
     global _work
     if _profile is not None and partials is None:
         _work = (n_tokens * (2 * Hq + (3 * Hkv if write_kv else 0)) * D * qkv.element_size(), 0.0)
-    _check(lib().ferrum_rope_cache_write(_ptr(qkv), dtype_code(qkv.dtype), c_int(n_tokens), c_int(qkv.stride(0)),
+    _check(lib().ferrum_rope_cache_write(_ptr(qkv), dtype_code(qkv.dtype), n_tokens, qkv.stride(0),
                                          _ptr(positions), _ptr(req_of_token), _ptr(block_table),
-                                         c_int(block_table.shape[1]), _ptr(cos_sin if R else None),
-                                         c_int(cos_sin.shape[0] if R else 0), _ptr(kv_plane if write_kv else None),
-                                         c_longlong(page_stride), c_int(page_size), c_int(Hq), c_int(Hkv), c_int(D),
-                                         c_int(R), c_int(pairing), c_int(1 if write_kv else 0), _ptr(err),
+                                         block_table.shape[1], _ptr(cos_sin if R else None),
+                                         cos_sin.shape[0] if R else 0, _ptr(kv_plane if write_kv else None),
+                                         c_longlong(page_stride), page_size, Hq, Hkv, D,
+                                         R, pairing, 1 if write_kv else 0, _ptr(err),
                                          _ptr(partials.workspace if partials is not None else None),
                                          partials._c if partials is not None else None, _stream()),
            "rope_cache_write")
@@ -602,18 +624,19 @@ def attention_generic(q, out, n_tokens, positions, req_of_token, block_table, kv
         _need(part, torch.float32, "part")
         if part.numel() < n_tokens * Hq * split_slots * (D + 2):
             raise KernelError("attention: the partials buffer is too small")
-    _check(lib().ferrum_attention_generic(_ptr(q), c_int(q.stride(0)), _ptr(out), c_int(out.stride(0)),
-                                          dtype_code(q.dtype), c_int(n_tokens), _ptr(positions), _ptr(req_of_token),
-                                          _ptr(block_table), c_int(block_table.shape[1]), _ptr(kv_plane),
-                                          c_longlong(page_stride), c_int(page_size), c_int(Hq), c_int(Hkv), c_int(D),
-                                          c_float(scale), c_int(window), _ptr(err), _ptr(part), c_int(split_slots),
-                                          _ptr(q_start) if part is None else None, c_int(n_reqs), _ptr(r1), _ptr(r2),
-                                          c_int(1 if out.dtype == torch.float32 and q.dtype != torch.float32 else 0),
-                                          c_int(1 if chunked else 0), c_float(softcap or 0.0), c_int(1 if sink else 0), c_int(int(keep_first)),
+    _check(lib().ferrum_attention_generic(_ptr(q), q.stride(0), _ptr(out), out.stride(0),
+                                          dtype_code(q.dtype), n_tokens, _ptr(positions), _ptr(req_of_token),
+                                          _ptr(block_table), block_table.shape[1], _ptr(kv_plane),
+                                          c_longlong(page_stride), page_size, Hq, Hkv, D,
+                                          c_float(scale), window, _ptr(err), _ptr(part), split_slots,
+                                          _ptr(q_start) if part is None else None, n_reqs, _ptr(r1), _ptr(r2),
+                                          1 if out.dtype == torch.float32 and q.dtype != torch.float32 else 0,
+                                          1 if chunked else 0, c_float(softcap or 0.0), 1 if sink else 0, int(keep_first),
                                           c_float(out_scale), _stream()),
            "attention_generic")
 
 
+@functools.lru_cache(maxsize=256)
 def attention_flash_supported(dtype, D, page_stride=0):
     """True when the tensor-core attention kernel is built for this dtype and head size."""
     return dtype in SIXTEEN_BIT and bool(lib().ferrum_attention_flash_supported(c_int(D), c_int(16)))
@@ -654,14 +677,14 @@ def attention_flash(q, out, kv_plane, page_stride, page_size, block_table, q_sta
     keep float32 precision (a 16-bit head and a 16-bit remainder) instead of being rounded for the second product."""
     _need16(q, "q", 2); _need16(out, "out", 2, like=q); _need16(kv_plane, "kv_plane", like=q)
     _need(block_table, torch.int32, "block_table", 2); _need(work, torch.int32, "work", 1)
-    _check(lib().ferrum_attention_flash(_ptr(q), c_int(q.stride(0)), _ptr(out), c_int(out.stride(0)), dtype_code(q.dtype),
+    _check(lib().ferrum_attention_flash(_ptr(q), q.stride(0), _ptr(out), out.stride(0), dtype_code(q.dtype),
                                         _ptr(kv_plane),
-                                        c_longlong(page_stride), c_int(page_size), _ptr(block_table),
-                                        c_int(block_table.shape[1]), _ptr(q_start), _ptr(pos0), _ptr(work),
-                                        c_int(n_work), _ptr(cta_items), c_int(n_ctas), _ptr(part_o), _ptr(part_ml),
-                                        c_int(Hq), c_int(Hkv), c_int(D),
-                                        c_float(scale), c_int(window), c_int(bm), c_int(1 if trigger_early else 0),
-                                        _ptr(err), c_int(1 if wide_weights else 0), _stream()), "attention_flash")
+                                        c_longlong(page_stride), page_size, _ptr(block_table),
+                                        block_table.shape[1], _ptr(q_start), _ptr(pos0), _ptr(work),
+                                        n_work, _ptr(cta_items), n_ctas, _ptr(part_o), _ptr(part_ml),
+                                        Hq, Hkv, D,
+                                        c_float(scale), window, bm, 1 if trigger_early else 0,
+                                        _ptr(err), 1 if wide_weights else 0, _stream()), "attention_flash")
 
 
 def attention_tc_tokens(D, G, page_size, kv_plane=None, page_stride=0):
@@ -685,11 +708,11 @@ def attention_tc(q, out, kv_plane, page_stride, page_size, block_table, q_start,
     """tcgen05 attention over work items of attention_tc_tokens * G rows (prompt portions).  wide_weights: as in `attention_flash`."""
     _need16(q, "q", 2); _need16(out, "out", 2, like=q); _need16(kv_plane, "kv_plane", like=q)
     _need(block_table, torch.int32, "block_table", 2); _need(work, torch.int32, "work", 1)
-    _check(lib().ferrum_attention_tc(_ptr(q), c_int(q.stride(0)), c_longlong(q.shape[0]), _ptr(out), c_int(out.stride(0)),
+    _check(lib().ferrum_attention_tc(_ptr(q), q.stride(0), c_longlong(q.shape[0]), _ptr(out), out.stride(0),
                                      dtype_code(q.dtype), _ptr(kv_plane), c_longlong(page_stride), c_longlong(kv_plane.shape[0]),
-                                     c_int(page_size), _ptr(block_table), c_int(block_table.shape[1]), _ptr(q_start),
-                                     _ptr(pos0), _ptr(work), c_int(n_work), _ptr(part_o), _ptr(part_ml), c_int(Hq),
-                                     c_int(Hkv), c_int(D), c_float(scale), c_int(window), _ptr(err), c_int(1 if wide_weights else 0), _stream()),
+                                     page_size, _ptr(block_table), block_table.shape[1], _ptr(q_start),
+                                     _ptr(pos0), _ptr(work), n_work, _ptr(part_o), _ptr(part_ml), Hq,
+                                     Hkv, D, c_float(scale), window, _ptr(err), 1 if wide_weights else 0, _stream()),
            "attention_tc")
 
 
@@ -698,17 +721,17 @@ def attention_combine(out, part_o, part_ml, q_start, req_of_token, req_tile0, ti
     """Merges the key-range splits written by attention_flash into `out`.  n_warps (1..8): warps
     per (token, head) that share its splits; more than one pays from about 16 splits on."""
     _need16(out, "out", 2)
-    _check(lib().ferrum_attention_combine(_ptr(out), c_int(out.stride(0)), dtype_code(out.dtype), _ptr(part_o), _ptr(part_ml), _ptr(q_start),
+    _check(lib().ferrum_attention_combine(_ptr(out), out.stride(0), dtype_code(out.dtype), _ptr(part_o), _ptr(part_ml), _ptr(q_start),
                                           _ptr(req_of_token), _ptr(req_tile0), _ptr(tile_info), _ptr(token_list),
-                                          c_int(n_tokens), c_int(Hq), c_int(Hkv), c_int(D), c_int(bm), c_int(n_warps), _stream()),
+                                          n_tokens, Hq, Hkv, D, bm, n_warps, _stream()),
            "attention_combine")
 
 
 def swiglu(gu, act, n_tokens, F):
     """act[t, f] = silu(gu[t, f]) * gu[t, F + f]."""
     _need(gu, None, "gu", 2); _need(act, gu.dtype, "act", 2)
-    _check(lib().ferrum_swiglu(_ptr(gu), _ptr(act), dtype_code(gu.dtype), c_int(n_tokens), c_int(F),
-                               c_int(gu.stride(0)), c_int(act.stride(0)), _stream()), "swiglu")
+    _check(lib().ferrum_swiglu(_ptr(gu), _ptr(act), dtype_code(gu.dtype), n_tokens, F,
+                               gu.stride(0), act.stride(0), _stream()), "swiglu")
 
 
 def sample(logits, n_rows, out_ids, err, inv_temperature=None, seeds=None, counters=None, also_to=None):
@@ -718,7 +741,7 @@ def sample(logits, n_rows, out_ids, err, inv_temperature=None, seeds=None, count
     if inv_temperature is not None:
         _need(inv_temperature, torch.float32, "inv_temperature", 1)
         _need(seeds, torch.int64, "seeds", 1); _need(counters, torch.int32, "counters", 1)
-    _check(lib().ferrum_sample(_ptr(logits), c_int(logits.stride(0)), c_int(n_rows), c_int(logits.shape[1]),
+    _check(lib().ferrum_sample(_ptr(logits), logits.stride(0), n_rows, logits.shape[1],
                                _ptr(inv_temperature), _ptr(seeds), _ptr(counters), _ptr(out_ids), _ptr(also_to),
                                _ptr(err), _stream()), "sample")
 

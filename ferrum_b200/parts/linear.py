@@ -19,11 +19,10 @@ def linear_deferred(x, w, ctx, M, N=None, dual_offset=0):
     """The product as float32 partials for the next kernel to sum (`ops.Partials`), or None
     when the shape or the operands do not allow it.  The partials live in the step's product
     workspace: they must be consumed before the next tensor-core product runs."""
-    if M == 0 or not ops.gemm_tc_supported(x, w) or (N is None and not dual_offset and ops.thin_linear_supported(x, w, M)):
-        return None
+    thin = N is None and not dual_offset
     N = (w.shape[0] - dual_offset) if N is None else N
     K = w.shape[1]
-    if not ops.gemm_tc_can_defer(M, N, K, dual_offset > 0):
+    if M == 0 or not ops.gemm_tc_can_defer(M, N, K, dual_offset > 0) or not ops.gemm_tc_supported(x, w) or (thin and ops.thin_linear_supported(x, w, M)):
         return None
     ctx.flush_residual()
     ws, _ = ctx.gemm_scratch(M, N, K, dual_offset > 0)

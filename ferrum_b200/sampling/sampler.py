@@ -76,7 +76,7 @@ class DeviceSampler:
         self._turn = (self._turn + 1) % self.DEPTH
         host, event = self._ids_host[self._turn], self._events[self._turn]
         host.copy_(ids_d, non_blocking=True)
-        event.record()
+        event.record(ops.current_stream())
         self.d2h_bytes = 4 * (self.max_rows + 1)
         return Ticket(n, host, event)
 
