@@ -55,6 +55,7 @@
 
 #include "common.cuh"
 #include "ptx_sm100.cuh"
+#include "softmax_sink.cuh"
 
 using namespace sm100;
 
@@ -74,19 +75,25 @@ struct AttnTcParams {
   int ldo, page_size, page_shift, table_width;
   int Hkv, G, tok, window;
   float scale_log2;
+  // keys and values that lie as rows (ROWS): see ferrum_attention_rows
+  const int* key_row;   // [R] row of a request's key 0 (may lie before its first row: only the keys in use have rows)
+  const float* gate;    // [tokens][Hkv] factor of a head's output, or null
+  const float* sink;    // [Hkv], or null
+  int k_cols, v_cols;   // columns of a row where head 0's keys and values begin; its shared key part begins at rot_col of the other map
+  int rot_col;
 };
 
-// NT row tiles per CTA, BN keys per stage, NS stages of keys and of values.
-template <int D, int NT, int BN, int NS>
+// D value columns and DK query and key columns of a head, NT row tiles per CTA, BN keys per stage, NS stages of keys and of values.
+template <int D, int DK, int NT, int BN, int NS>
 struct AttnTcConfig {
-  static constexpr int HALVES = D / 64;                          // 64-column spans of a head
-  static constexpr int Q_TILE_BYTES = HALVES * 128 * 128;       // 128 rows x 128 bytes per 64 columns
+  static constexpr int HALVES = D / 64, K_HALVES = DK / 64;      // 64-column spans of a head
+  static constexpr int Q_TILE_BYTES = K_HALVES * 128 * 128;     // 128 rows x 128 bytes per 64 columns
   static constexpr int KV_HALF_BYTES = BN * 128;
-  static constexpr int KV_STAGE_BYTES = HALVES * KV_HALF_BYTES;
+  static constexpr int K_STAGE_BYTES = K_HALVES * KV_HALF_BYTES, V_STAGE_BYTES = HALVES * KV_HALF_BYTES;
   static constexpr int OFF_Q = 0;
   static constexpr int OFF_K = OFF_Q + NT * Q_TILE_BYTES;
-  static constexpr int OFF_V = OFF_K + NS * KV_STAGE_BYTES;
-  static constexpr int OFF_BARS = OFF_V + NS * KV_STAGE_BYTES;
+  static constexpr int OFF_V = OFF_K + NS * K_STAGE_BYTES;
+  static constexpr int OFF_BARS = OFF_V + NS * V_STAGE_BYTES;
   static constexpr int N_BARS = 1 + 4 * NS + 6 * NT;
   static constexpr int SMEM_BYTES = OFF_BARS + N_BARS * 8 + 1024 /*alignment slack*/;
   static constexpr int S_COL = 0;                 // S of tile t, buffer b: columns (2 t + b) * BN ..
@@ -179,11 +186,14 @@ __device__ __forceinline__ float unpack_16(uint32_t bits) {
   return HALF ? __half2float(__ushort_as_half((unsigned short)bits)) : __uint_as_float(bits << 16);
 }
 
-template <int D, int NT, int BN, int NS, bool HALF, bool WIDE>
-__global__ void __launch_bounds__(AttnTcConfig<D, NT, BN, NS>::THREADS, 1)
-attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_kv, const AttnTcParams p) {
-  using Cfg = AttnTcConfig<D, NT, BN, NS>;
-  constexpr int HALVES = Cfg::HALVES;
+// ROWS: keys and values are rows of a matrix (a head's keys and values at columns of their own) instead of pages, one query
+// head per KV head; the last 64 columns of a key are shared by all heads and come from the rows of `map_rot`.
+template <int D, int DK, int NT, int BN, int NS, bool HALF, bool WIDE, bool ROWS>
+__global__ void __launch_bounds__(AttnTcConfig<D, DK, NT, BN, NS>::THREADS, 1)
+attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_kv,
+                    const __grid_constant__ CUtensorMap map_rot, const AttnTcParams p) {
+  using Cfg = AttnTcConfig<D, DK, NT, BN, NS>;
+  constexpr int HALVES = Cfg::HALVES, K_HALVES = Cfg::K_HALVES;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   __shared__ uint32_t tmem_slot;
@@ -262,16 +272,17 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     // is read one stage ahead, so that the lookups of a stage overlap instead of queueing).  The
     // keys of stage j + 1 are requested before the values of stage j: the scores run ahead.
     if (lane == 0) {
-      mbar_expect_tx(q_full, NT * HALVES * tok * G * 128);
+      mbar_expect_tx(q_full, NT * K_HALVES * tok * G * 128);
       for (int t = 0; t < NT; ++t)
-        for (int h = 0; h < HALVES; ++h)
+        for (int h = 0; h < K_HALVES; ++h)
           tma_load_3d(smem_base + Cfg::OFF_Q + t * Cfg::Q_TILE_BYTES + h * 128 * 128, &map_q, q_full, h * 64, kvh * G,
                       qs + tok0 + t * tok);
     }
     const int ps = p.page_size;
-    const int pages_per_stage = BN / ps;
+    const int pages_per_stage = ROWS ? 0 : BN / ps;
     const int* bt = p.block_table + (size_t)req * p.table_width;
     auto page_of = [&](int j) {  // this lane's page of stage j; a page past the key range reads as zeros (masked keys)
+      if (ROWS) return -1;
       const int lp = ((kv0 + j * BN) >> p.page_shift) + lane;
       if (!(lane < pages_per_stage && j >= 0 && j < n_j)) return -1;
       const int page = lp < p.table_width ? bt[lp] : -1;
@@ -287,13 +298,24 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       bool ok = true;
       if (lane == 0) {
         ok = mbar_wait(kv ? v_empty(s) : k_empty(s), parity, abort_p);
-        if (ok) mbar_expect_tx(full, Cfg::KV_STAGE_BYTES);
+        if (ok) mbar_expect_tx(full, kv ? Cfg::V_STAGE_BYTES : Cfg::K_STAGE_BYTES);
+        if (ROWS && ok) {
+          const int y = p.key_row[req] + kv0 + j * BN;     // (rows past the last one read as zeros, other requests' rows are masked)
+          const uint32_t dst = smem_base + (kv ? Cfg::OFF_V + s * Cfg::V_STAGE_BYTES : Cfg::OFF_K + s * Cfg::K_STAGE_BYTES);
+          if (kv) {
+            for (int h = 0; h < HALVES; ++h) tma_load_2d(dst + h * Cfg::KV_HALF_BYTES, &map_kv, full, p.v_cols + kvh * D + h * 64, y);
+          } else {
+            for (int h = 0; h < K_HALVES - 1; ++h)
+              tma_load_2d(dst + h * Cfg::KV_HALF_BYTES, &map_kv, full, p.k_cols + kvh * (DK - 64) + h * 64, y);
+            tma_load_2d(dst + (K_HALVES - 1) * Cfg::KV_HALF_BYTES, &map_rot, full, p.rot_col, y);
+          }
+        }
       }
       ok = __shfl_sync(0xffffffffu, ok, 0);
       if (!ok) return false;
       if (lane < pages_per_stage) {
         const int y = page < 0 ? -ps : ((page * 2 + kv) * p.Hkv + kvh) * ps;   // a negative row: the box reads as zeros
-        const uint32_t dst = smem_base + (kv ? Cfg::OFF_V : Cfg::OFF_K) + s * Cfg::KV_STAGE_BYTES + lane * ps * 128;
+        const uint32_t dst = smem_base + (kv ? Cfg::OFF_V + s * Cfg::V_STAGE_BYTES : Cfg::OFF_K + s * Cfg::K_STAGE_BYTES) + lane * ps * 128;
         for (int h = 0; h < HALVES; ++h) tma_load_2d(dst + h * Cfg::KV_HALF_BYTES, &map_kv, full, h * 64, y);
       }
       return true;
@@ -322,17 +344,17 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       const uint64_t q_desc = umma_desc_k_sw128(q_addr), k_desc0 = umma_desc_k_sw128(smem_base + Cfg::OFF_K);
       const uint64_t v_desc0 = umma_desc_mn_sw128(smem_base + Cfg::OFF_V, Cfg::KV_HALF_BYTES, 1024);
       auto issue_qk = [&](int s, int buf) {
-        const uint64_t k_desc = k_desc0 + (uint64_t)(s * (Cfg::KV_STAGE_BYTES >> 4));
+        const uint64_t k_desc = k_desc0 + (uint64_t)(s * (Cfg::K_STAGE_BYTES >> 4));
         const uint32_t s_tmem = tmem_base + Cfg::S_COL + (2 * t + buf) * BN;
 #pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) {
+        for (int kk = 0; kk < DK / 16; ++kk) {
           const int h = kk >> 2, in = kk & 3;
           umma_bf16(s_tmem, q_desc + (uint64_t)((h * 128 * 128 >> 4) + in * 2),
                     k_desc + (uint64_t)((h * Cfg::KV_HALF_BYTES >> 4) + in * 2), idesc_qk, kk > 0);
         }
       };
       auto issue_pv = [&](int s, int buf, bool accumulate) {
-        const uint64_t v_desc = v_desc0 + (uint64_t)(s * (Cfg::KV_STAGE_BYTES >> 4));
+        const uint64_t v_desc = v_desc0 + (uint64_t)(s * (Cfg::V_STAGE_BYTES >> 4));
         const uint32_t p_tmem = tmem_base + Cfg::S_COL + (2 * t + buf) * BN;  // P lies over the scores it came from
 #pragma unroll
         for (int kk = 0; kk < BN / 16; ++kk)  // 16 keys on: 8 columns of P, 16 rows of V
@@ -503,7 +525,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
           break;
         }
         const int first_bad = kv_end - key0;
-        uint8_t* v = smem + Cfg::OFF_V + s_last * Cfg::KV_STAGE_BYTES;
+        uint8_t* v = smem + Cfg::OFF_V + s_last * Cfg::V_STAGE_BYTES;
         const int n16 = (BN - first_bad) * 8;  // 16-byte pieces per 64-column half
         for (int h = 0; h < HALVES; ++h)
           for (int i = r; i < n16; i += 128)
@@ -538,7 +560,12 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     } else {
       tc_fence_after();
       const bool whole = n_splits == 1;
-      const float inv = l_run > 0.f ? 1.0f / l_run : 0.f;
+      float inv = l_run > 0.f ? 1.0f / l_run : 0.f;
+      if constexpr (ROWS) {
+        // (m_run is in units of log2, and may lag behind the row's maximum by TC_LAZY: the factor does not depend on it)
+        if (p.sink != nullptr) inv = softmax_sink_factor(m_run * 0.6931471805599453f, l_run, p.sink, kvh);
+        if (p.gate != nullptr && row_valid) inv *= p.gate[(size_t)(qs + tok_in_req) * p.Hkv + kvh];
+      }
       uint16_t* orow = p.out + (size_t)(qs + tok_in_req) * p.ldo + (size_t)(kvh * G + r % G) * D;
       const size_t prow = (size_t)part * (NT * tok * G) + t * tok * G + r;
 #pragma unroll 1
@@ -1106,24 +1133,25 @@ int cache_map(const void* plane, long long n_pages, int Hkv, int page_size, int 
   return 0;
 }
 
-template <int D, int NT, int BN, int NS, bool HALF, bool WIDE>
-int launch_attention_tc_as(const CUtensorMap& mq, const CUtensorMap& mkv, const AttnTcParams& p, int n_work, cudaStream_t stream) {
-  using Cfg = AttnTcConfig<D, NT, BN, NS>;
+template <int D, int DK, int NT, int BN, int NS, bool HALF, bool WIDE, bool ROWS>
+int launch_attention_tc_as(const CUtensorMap& mq, const CUtensorMap& mkv, const CUtensorMap& mrot, const AttnTcParams& p, int n_work,
+                           cudaStream_t stream) {
+  using Cfg = AttnTcConfig<D, DK, NT, BN, NS>;
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(attention_tc_kernel<D, NT, BN, NS, HALF, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES);
+    cudaError_t e = cudaFuncSetAttribute(attention_tc_kernel<D, DK, NT, BN, NS, HALF, WIDE, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES);
     FERRUM_CHECK_ARG(e == cudaSuccess, "attention_tc: cannot reserve %d bytes of shared memory: %s", Cfg::SMEM_BYTES, cudaGetErrorString(e));
     configured = true;
   }
-  launch_kernel(attention_tc_kernel<D, NT, BN, NS, HALF, WIDE>, dim3(p.Hkv, n_work), dim3(Cfg::THREADS), Cfg::SMEM_BYTES, stream, mq, mkv, p);
+  launch_kernel(attention_tc_kernel<D, DK, NT, BN, NS, HALF, WIDE, ROWS>, dim3(p.Hkv, n_work), dim3(Cfg::THREADS), Cfg::SMEM_BYTES, stream, mq, mkv, mrot, p);
   FERRUM_CHECK_LAUNCH("attention_tc");
   return 0;
 }
 
 template <int D, int NT, int BN, int NS, bool HALF>
 int launch_attention_tc(const CUtensorMap& mq, const CUtensorMap& mkv, const AttnTcParams& p, int n_work, int wide, cudaStream_t stream) {
-  return wide ? launch_attention_tc_as<D, NT, BN, NS, HALF, true>(mq, mkv, p, n_work, stream)
-              : launch_attention_tc_as<D, NT, BN, NS, HALF, false>(mq, mkv, p, n_work, stream);
+  return wide ? launch_attention_tc_as<D, D, NT, BN, NS, HALF, true, false>(mq, mkv, mkv, p, n_work, stream)
+              : launch_attention_tc_as<D, D, NT, BN, NS, HALF, false, false>(mq, mkv, mkv, p, n_work, stream);
 }
 
 template <int NS, bool HALF>
@@ -1201,7 +1229,7 @@ FERRUM_API int ferrum_attention_tc(const void* q, int ldq, long long q_rows, voi
   FERRUM_CHECK_ARG(table_width > 0 && window >= 0 && n_work >= 0 && q_rows > 0, "attention_tc: bad arguments");
   if (n_work == 0) return 0;
   FERRUM_CHECK_ARG(n_work <= 65535, "attention_tc: %d work items are more than one launch takes", n_work);
-  AttnTcParams p;
+  AttnTcParams p = {};
   p.out = (uint16_t*)out; p.block_table = block_table; p.q_start = q_start; p.pos0 = pos0; p.work = work;
   p.part_o = part_o; p.part_ml = part_ml; p.err = err_flag;
   p.ldo = ldo; p.page_size = page_size; p.table_width = table_width;
@@ -1222,4 +1250,98 @@ FERRUM_API int ferrum_attention_tc(const void* q, int ldq, long long q_rows, voi
   }
   if (D == 64) return launch_attention_tc<64, TC_TILES, TC_BN, TC_STAGES, false>(mq, mkv, p, n_work, wide, stream);
   return launch_attention_tc<128, TC_TILES, TC_BN, TC_STAGES, false>(mq, mkv, p, n_work, wide, stream);
+}
+
+// ------------------------------------------------------------------ expanded latent keys and values
+namespace {
+
+// Rows of a 16-bit matrix [rows, cols]; a box is 64 columns x TC_BN rows.
+int rows_map(const void* p, long long rows, long long cols, long long ld, CUtensorMap* out) {
+  EncodeTiledFn fn = encode_fn();
+  FERRUM_CHECK_ARG(fn != nullptr, "attention_rows: the driver does not export cuTensorMapEncodeTiled");
+  cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+  cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
+  cuuint32_t box[2] = {64, (cuuint32_t)TC_BN};
+  cuuint32_t estr[2] = {1, 1};
+  CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(p), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  FERRUM_CHECK_ARG(r == CUDA_SUCCESS, "attention_rows: encoding a row map failed with code %d", (int)r);
+  return 0;
+}
+
+template <bool HALF>
+int launch_attention_rows(const CUtensorMap& mq, const CUtensorMap& mkv, const CUtensorMap& mrot, const AttnTcParams& p, int n_work, int wide,
+                          cudaStream_t stream) {
+  return wide ? launch_attention_tc_as<128, 192, TC_TILES, TC_BN, TC_STAGES, HALF, true, true>(mq, mkv, mrot, p, n_work, stream)
+              : launch_attention_tc_as<128, 192, TC_TILES, TC_BN, TC_STAGES, HALF, false, true>(mq, mkv, mrot, p, n_work, stream);
+}
+
+// Row i of `rows` <- the cached row of key `first[r] + i - start[r]` of the request r whose rows start[r] .. start[r + 1] - 1 are;
+// zeros where the key has no page.  A warp takes a row.
+__global__ void __launch_bounds__(256)
+latent_gather_kernel(const uint16_t* __restrict__ plane, long long page_stride, int page_size, const int* __restrict__ block_table,
+                     int table_width, const int* __restrict__ start, const int* __restrict__ first, const int* __restrict__ pos0, int window,
+                     int n_reqs, int n_rows, int Dk, uint16_t* __restrict__ rows, int* __restrict__ err) {
+  pdl_launch();
+  pdl_wait();
+  const int i = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (i >= n_rows) return;
+  int r = 0;
+  while (r + 1 < n_reqs && start[r + 1] <= i) ++r;
+  const int key = first[r] + i - start[r], lp = key / page_size;
+  const int page = lp < table_width ? block_table[(size_t)r * table_width + lp] : -1;
+  // (a key before the window of the step's first query may have lost its page; any other must have one)
+  if (page < 0 && lane == 0 && (window == 0 || key > pos0[r] - window)) atomicExch(err, 5);
+  const uint4* src = reinterpret_cast<const uint4*>(plane + (size_t)max(page, 0) * page_stride + (size_t)(key % page_size) * Dk);
+  uint4* dst = reinterpret_cast<uint4*>(rows + (size_t)i * Dk);
+  for (int c = lane; c < Dk / 8; c += 32) dst[c] = page >= 0 ? src[c] : make_uint4(0, 0, 0, 0);
+}
+
+}  // namespace
+
+FERRUM_API int ferrum_latent_gather(const void* plane, long long page_stride, int page_size, const int* block_table, int table_width,
+                                    const int* start, const int* first, const int* pos0, int window, int n_reqs, int n_rows, int Dk, void* rows,
+                                    int* err_flag, cudaStream_t stream) {
+  FERRUM_CHECK_ARG(err_flag != nullptr && window >= 0 && n_reqs > 0 && n_rows >= 0 && page_size > 0 && table_width > 0, "latent_gather: bad sizes");
+  FERRUM_CHECK_ARG(Dk % 8 == 0 && page_stride % 8 == 0 && ((uintptr_t)plane & 15) == 0 && ((uintptr_t)rows & 15) == 0,
+                   "latent_gather: rows must be 16-byte multiples");
+  if (n_rows == 0) return 0;
+  launch_kernel(latent_gather_kernel, dim3((n_rows + 7) / 8), dim3(256), 0, stream, (const uint16_t*)plane, page_stride, page_size, block_table,
+                table_width, start, first, pos0, window, n_reqs, n_rows, Dk, (uint16_t*)rows, err_flag);
+  FERRUM_CHECK_LAUNCH("latent_gather");
+  return 0;
+}
+
+// Causal attention of H heads, every one with keys and values of its own: q [tokens, H * 192] (a head's 128 plain columns, then its
+// 64 rotated ones), kv [n_rows, ldkv] with head h's 128 plain key columns at h * 128 and its values at H * 128 + h * 128, rot
+// [n_rows, ldrot] with the rotated key columns of all heads at rot_col.  key_row[r] + k is the row of key k of request r.  Items of
+// 256 tokens, unsplit, as ferrum_attention_tc takes them.  out [tokens, H * 128], times gate[t, h] (or null), sink[h] in every
+// softmax (or null).
+// This is latent attention with its keys and values written out: a (query, key) pair costs 320 products a head instead of the
+// 1,088 on the cached rows, for one product of the rows with U_k and U_v ahead.  Bound by the softmax of a stage like the kernel
+// on pages; 1,500 tokens are 96 items, so a wave leaves a third of the SMs idle.  Measured on a B200, 1,500 tokens, 16 heads,
+// rows of 512 + 64, a whole layer: 670 -> 340 us (attention on the cached rows alone was 345).
+FERRUM_API int ferrum_attention_rows(const void* q, int ldq, long long q_rows, const void* kv, int ldkv, const void* rot, int ldrot, int rot_col,
+                                     int n_rows, void* out, int ldo, int dtype, const int* key_row, const int* q_start, const int* pos0,
+                                     const int* work, int n_work, int H, float scale, int window, const float* gate, const float* sink,
+                                     int* err_flag, int wide, cudaStream_t stream) {
+  FERRUM_CHECK_ARG(ferrum_is_16bit(dtype) && err_flag != nullptr && key_row != nullptr, "attention_rows: bad arguments");
+  FERRUM_CHECK_ARG(H > 0 && n_rows > 0 && window >= 0 && n_work >= 0 && n_work <= 65535 && q_rows > 0, "attention_rows: bad sizes");
+  FERRUM_CHECK_ARG(ldq >= H * 192 && ldkv >= H * 256 && ldo >= H * 128 && rot_col >= 0 && rot_col % 8 == 0 && ldrot >= rot_col + 64,
+                   "attention_rows: a row stride is too short");
+  FERRUM_CHECK_ARG(ldq % 8 == 0 && ldkv % 8 == 0 && ldrot % 8 == 0 && ldo % 8 == 0 && ((uintptr_t)q & 15) == 0 && ((uintptr_t)kv & 15) == 0 &&
+                   ((uintptr_t)rot & 15) == 0 && ((uintptr_t)out & 15) == 0, "attention_rows: operands must be 16-byte aligned");
+  if (n_work == 0) return 0;
+  AttnTcParams p = {};
+  p.out = (uint16_t*)out; p.q_start = q_start; p.pos0 = pos0; p.work = work; p.err = err_flag;
+  p.ldo = ldo; p.Hkv = H; p.G = 1; p.tok = 128; p.window = window; p.page_size = TC_BN;
+  p.scale_log2 = scale * 1.4426950408889634f;
+  p.key_row = key_row; p.gate = gate; p.sink = sink;
+  p.k_cols = 0; p.v_cols = H * 128; p.rot_col = rot_col;
+  CUtensorMap mq, mkv, mrot;
+  if (int r = query_map(q, q_rows, ldq, H, 192, 1, 128, &mq)) return r;
+  if (int r = rows_map(kv, n_rows, (long long)H * 256, ldkv, &mkv)) return r;
+  if (int r = rows_map(rot, n_rows, rot_col + 64, ldrot, &mrot)) return r;
+  return dtype == FERRUM_F16 ? launch_attention_rows<true>(mq, mkv, mrot, p, n_work, wide, stream)
+                             : launch_attention_rows<false>(mq, mkv, mrot, p, n_work, wide, stream);
 }

@@ -155,6 +155,43 @@ latent_q_rope_kernel(const T* __restrict__ q, int ldq, T* __restrict__ qf, int l
   }
 }
 
+// The same in place (q itself): a thread owns a pair of elements.
+template <typename T>
+__global__ void __launch_bounds__(LAT_THREADS)
+latent_q_rope_own_kernel(T* __restrict__ q, int ldq, const int* __restrict__ positions, const float* __restrict__ cos_sin, int n_pos,
+                         int rope_dims, int pairing, int H, int Dn, int Rr, int* __restrict__ err) {
+  pdl_launch();
+  pdl_wait();
+  const int t = blockIdx.x;
+  const int pos = positions[t];
+  if (pos < 0 || pos >= n_pos) {
+    if (threadIdx.x == 0) atomicExch(err, 2);
+    return;
+  }
+  const float* cs = cos_sin + (size_t)pos * rope_dims;
+  const int half = rope_dims >> 1;
+  for (int idx = threadIdx.x; idx < H * half; idx += blockDim.x) {
+    const int h = idx / half, k = idx % half;
+    T* row = q + (size_t)t * ldq + (size_t)h * (Dn + Rr) + Dn;
+    T* a = row + (pairing == 0 ? 2 * k : k);
+    T* b = row + (pairing == 0 ? 2 * k + 1 : k + half);
+    const float x = to_f32<T>(*a), y = to_f32<T>(*b), c = cs[2 * k], s = cs[2 * k + 1];
+    *a = from_f32<T>(x * c - y * s);
+    *b = from_f32<T>(y * c + x * s);
+  }
+}
+
+FERRUM_API int ferrum_latent_q_rope_own(void* q, int ldq, int dtype, int n_tokens, const int* positions, const float* cos_sin, int n_pos,
+                                        int rope_dims, int pairing, int H, int Dn, int Rr, int* err_flag, cudaStream_t stream) {
+  FERRUM_CHECK_ARG(n_tokens >= 0 && H > 0 && Dn >= 0 && Rr >= 0 && ldq >= H * (Dn + Rr), "latent q rope: bad sizes");
+  FERRUM_CHECK_ARG(rope_dims >= 0 && rope_dims % 2 == 0 && rope_dims <= Rr, "latent q rope: %d rotated dimensions of %d", rope_dims, Rr);
+  if (n_tokens == 0 || rope_dims == 0) return 0;
+  FERRUM_DISPATCH_DTYPE(dtype, T, launch_kernel(latent_q_rope_own_kernel<T>, n_tokens, LAT_THREADS, 0, stream, (T*)q, ldq, positions, cos_sin,
+                                                n_pos, rope_dims, pairing, H, Dn, Rr, err_flag));
+  FERRUM_CHECK_LAUNCH("latent_q_rope_own");
+  return 0;
+}
+
 FERRUM_API int ferrum_latent_q_rope(const void* q, int ldq, void* qf, int ldf, int dtype, int n_tokens, const int* positions,
                                     const float* cos_sin, int n_pos, int rope_dims, int pairing, int H, int Dn, int Rr, int R, int* err_flag,
                                     cudaStream_t stream) {

@@ -26,7 +26,7 @@ TC_STORE_BF16, TC_STORE_F32, TC_RESIDUAL, TC_SWIGLU, TC_GEGLU, TC_SWISH_CLAMP, T
 
 _lib = None
 _lock = threading.Lock()
-ABI = 22
+ABI = 23
 
 
 def lib():
@@ -860,6 +860,50 @@ def latent_q_rope(q, qf, n_tokens, positions, rot, H, Dn, Rr, R, err):
                                       c_int(cos_sin.shape[0] if rot is not None else 0),
                                       c_int(rot.rope_dim if rot is not None else 0), c_int(rot.pairing if rot is not None else 0), c_int(H), c_int(Dn), c_int(Rr), c_int(R),
                                       _ptr(err), _stream()), "latent_q_rope")
+
+
+def latent_q_rope_own(q, n_tokens, positions, rot, H, Dn, Rr, err):
+    """The rotated part of every query head of q (heads of Dn + Rr) in place."""
+    _need(q, None, "q", 2)
+    if rot is None:
+        return
+    _need(positions, torch.int32, "positions", 1)
+    _check(lib().ferrum_latent_q_rope_own(_ptr(q), q.stride(0), dtype_code(q.dtype), n_tokens, _ptr(positions), _ptr(rot.cos_sin),
+                                          rot.cos_sin.shape[0], rot.rope_dim, rot.pairing, H, Dn, Rr, _ptr(err), _stream()), "latent_q_rope_own")
+
+
+def latent_gather(plane, page_stride, page_size, block_table, start, first, pos0, window, n_rows, Dk, rows, err):
+    """rows[i] = the cached row of key first[r] + i - start[r] of request r, for start[r] <= i < start[r + 1]."""
+    _need16(plane, "plane"); _need16(rows, "rows", 2, like=plane)
+    _need(block_table, torch.int32, "block_table", 2); _need(start, torch.int32, "start", 1); _need(first, torch.int32, "first", 1)
+    if rows.shape[0] < n_rows or rows.shape[1] != Dk or not rows.is_contiguous() or not block_table.is_contiguous():
+        raise KernelError("latent_gather: rows must be contiguous [n_rows, Dk]")
+    _check(lib().ferrum_latent_gather(_ptr(plane), c_longlong(page_stride), page_size, _ptr(block_table), block_table.shape[1], _ptr(start),
+                                      _ptr(first), _ptr(pos0), window, first.shape[0], n_rows, Dk, _ptr(rows), _ptr(err), _stream()), "latent_gather")
+
+
+def attention_rows_supported(dtype, Dn, Rr, Dv, R):
+    """Whether `attention_rows` takes latent attention of these head and row sizes."""
+    return dtype in SIXTEEN_BIT and (Dn, Rr, Dv) == (128, 64, 128) and R % 8 == 0
+
+
+def attention_rows(q, kv, rot, rot_col, n_rows, out, key_row, q_start, pos0, work, n_work, H, scale, window, err, gate=None, sink=None,
+                   wide_weights=False):
+    """tcgen05 attention of heads with keys and values of their own, which lie as rows (attention_tc.cu)."""
+    _need16(q, "q", 2)
+    for t, name in ((kv, "kv"), (rot, "rot"), (out, "out")):
+        _need16(t, name, 2, like=q)
+    for t, name in ((key_row, "key_row"), (work, "work")):
+        _need(t, torch.int32, name, 1)
+    if kv.shape[0] < n_rows or rot.shape[0] < n_rows:
+        raise KernelError("attention_rows: fewer rows than keys")
+    for t, name in ((gate, "gate"), (sink, "sink")):
+        if t is not None:
+            _need(t, torch.float32, name)
+    _check(lib().ferrum_attention_rows(_ptr(q), q.stride(0), c_longlong(q.shape[0]), _ptr(kv), kv.stride(0), _ptr(rot), rot.stride(0), rot_col,
+                                       n_rows, _ptr(out), out.stride(0), dtype_code(q.dtype), _ptr(key_row), _ptr(q_start), _ptr(pos0),
+                                       _ptr(work), n_work, H, c_float(scale), window, _ptr(gate), _ptr(sink), _ptr(err),
+                                       1 if wide_weights else 0, _stream()), "attention_rows")
 
 
 @functools.lru_cache(maxsize=1)

@@ -120,6 +120,16 @@ def _grid_class(q_len, pos0, G, window, Hkv, bm, sel, R, q_start, slots=None, mi
             "cta_items": np.zeros(0, dtype=np.int32), "n_ctas": 0}
 
 
+def whole_items(q_len, pos0, window, bm):
+    """Work items [request, first row, first key, end key, 1, -1, 0, 0] of every request's tiles of bm rows (one row a token), with
+    all their keys, longest first."""
+    q_len, pos0 = np.asarray(q_len, dtype=np.int64), np.asarray(pos0, dtype=np.int64)
+    _, req, row0, lo, hi = _tiles(q_len, pos0, 1, window, bm, np.arange(len(q_len)))
+    items = np.zeros((len(req), 8), dtype=np.int32)
+    items[:, 0], items[:, 1], items[:, 2], items[:, 3], items[:, 4], items[:, 5] = req, row0, lo, hi, 1, -1
+    return items[np.argsort(lo - hi, kind="stable")]
+
+
 def _balanced_class(q_len, pos0, G, window, Hkv, bm, sel, R, q_start):
     """Requests with one row tile each (decoded tokens).  All (request, head, 64-key tile)
     units form one line; CTA slot c owns units [c*U/P, (c+1)*U/P); a share is cut into items

@@ -34,6 +34,24 @@ from .linear import RESIDUAL, STORE, STORE_F32, linear, linear_deferred
 SPLIT_BELOW = 4
 MAX_SPLITS = 1024       # what the merge kernel folds per (token, head)
 
+# Prompt portions write their requests' keys and values out (a product of the cached rows with U_k and U_v) and attend to
+# those on the tcgen05 kernel: (128 + 64 + 128) products a (query, key) pair and head instead of the (512 + 64 + 512) on the
+# cached rows, for 2 * 256 * 512 a key and head.  That pays where a key meets EXPAND_MIN_QUERIES queries of the step or
+# more on average (B200, a prompt step of four layers of 16 heads, us, cached rows -> written out: 256 tokens 975 -> 984, 400
+# 1001 -> 993, 700 1331 -> 1019, 1500 2691 -> 1373, 2048 3903 -> 1684).  The rows of EXPAND_MAX_KEYS keys are as much scratch as
+# a step may take (306 MB with 16 heads).
+EXPAND_MIN_QUERIES, EXPAND_MAX_KEYS = 192, 32768
+
+
+def rows_plan(q_len, pos0, window):
+    """(start, first): request r's keys from first[r] on lie at rows start[r] .. start[r + 1] - 1.  `first` is a multiple of the
+    kernel's 64-key stages that no query of the step sees past."""
+    import numpy as np
+    q_len, pos0 = np.asarray(q_len, dtype=np.int64), np.asarray(pos0, dtype=np.int64)
+    first = np.maximum(0, pos0 - window + 1) // 64 * 64 if window > 0 else np.zeros_like(pos0)
+    start = np.concatenate([[0], np.cumsum(pos0 + q_len - first)])
+    return start, first
+
 
 def _sink_init(shape, g, device, std):
     return torch.randn(shape, generator=g, device=device, dtype=torch.float32)
@@ -80,6 +98,11 @@ class LatentAttention(Mixer):
         # per head: U_k,h^T as [kv_rank, dim] (a linear map from the head's plain query part) and U_v,h as [vdim, kv_rank]
         self.w_uk_t = self.w_uk_weight.view(self.H, self.Dn, self.R).transpose(1, 2).contiguous()
         self.w_uv_h = self.w_uv_weight.view(self.H, self.Dv, self.R)     # (a view: contiguous [H, vdim, kv_rank])
+        self.w_ukv = None
+        if ops.attention_rows_supported(self.dtype, self.Dn, self.Rr, self.Dv, self.R):
+            self.w_ukv = torch.cat([self.w_uk_weight, self.w_uv_weight], dim=0).contiguous()     # every head's key rows, then every head's value rows
+            self.w_uv_h = self.w_ukv[self.H * self.Dn:].view(self.H, self.Dv, self.R)
+            self.w_uv_weight = None
         self.w_uk_weight = None
 
     def cache_need(self):
@@ -107,6 +130,11 @@ class LatentAttention(Mixer):
                         cache.page_stride, cache.page_size, cq, gate, self.eps, partials=part)
         q = ctx.buf("lat_q", (cap, H * (Dn + Rr)), self.dtype)
         linear(cq, self.w_uq_weight, q, STORE, ctx, M=T)
+        plan = self._expand_plan(ctx)
+        if plan is not None:
+            ov = ctx.buf("lat_ov", (cap, H * Dv), self.dtype)
+            self._expanded(q, ov, gate, plan, ctx, cache, table)
+            return self._project(ov, ctx, residual, accumulate, defer)
         qf = ctx.buf("lat_qf", (cap, H * Dk), self.dtype)
         few = T <= ops.head_linear_max_tokens()      # every head's product in one launch: a few tokens on the CUDA cores ...
         if few or ops.head_linear_mma_supported(q, Dn + Rr, self.w_uk_t, qf, Dk):     # ... many on the tensor cores
@@ -138,9 +166,49 @@ class LatentAttention(Mixer):
         else:
             for h in range(H):
                 linear(o[:, h * R:(h + 1) * R], self.w_uv_h[h], ov[:, h * Dv:(h + 1) * Dv], STORE, ctx, M=T)
+        return self._project(ov, ctx, residual, accumulate, defer)
+
+    def _project(self, ov, ctx, residual, accumulate, defer):
         if defer and not accumulate:
-            part = linear_deferred(ov, self.w_o_weight, ctx, T)
+            part = linear_deferred(ov, self.w_o_weight, ctx, ctx.n_tokens)
             if part is not None:
                 return part
-        linear(ov, self.w_o_weight, residual, RESIDUAL if accumulate else STORE_F32, ctx, M=T)
+        linear(ov, self.w_o_weight, residual, RESIDUAL if accumulate else STORE_F32, ctx, M=ctx.n_tokens)
         return None
+
+    def _expand_plan(self, ctx):
+        """Where this step's keys and values are written out: (keys, start, first, key_row, work, items), the same for every layer
+        with this window; None where attention runs on the cached rows."""
+        if self.w_ukv is None or ctx.max_q_len < EXPAND_MIN_QUERIES or ctx.fixed_shapes:
+            return None
+        key = ("latent rows", self.window)
+        if key in ctx.step_cache:
+            return ctx.step_cache[key]
+        import numpy as np
+        start, first = rows_plan(ctx.h_q_len, ctx.h_pos0, self.window)
+        n_keys = int(start[-1])
+        seen = sum(n * min(p + (n + 1) // 2, self.window if self.window > 0 else p + n) for p, n in zip(ctx.h_pos0, ctx.h_q_len))
+        plan = None
+        if n_keys <= EXPAND_MAX_KEYS and seen >= EXPAND_MIN_QUERIES * n_keys:
+            R = len(ctx.h_q_len)
+            items = attention_plan.whole_items(ctx.h_q_len, ctx.h_pos0, self.window, 256)
+            host = np.concatenate([start, first, start[:-1] - first, items.reshape(-1)]).astype(np.int32)
+            ring, dev = ctx.plan_store.buffers(key, host.size)
+            ring.next().numpy()[:host.size] = host
+            dev[:host.size].copy_(ring.bufs[ring.i][:host.size], non_blocking=True)
+            ring.sent()
+            ctx.h2d_bytes += host.size * 4
+            plan = (n_keys, dev[:R + 1], dev[R + 1:2 * R + 1], dev[2 * R + 1:3 * R + 1], dev[3 * R + 1:host.size], items.shape[0])
+        ctx.step_cache[key] = plan
+        return plan
+
+    def _expanded(self, q, ov, gate, plan, ctx, cache, table):
+        n_keys, start, first, key_row, work, n_work = plan
+        T, H, R = ctx.n_tokens, self.H, self.R
+        rows = ctx.buf("lat_rows", (n_keys, self.Dk), self.dtype)
+        kv = ctx.buf("lat_kv", (n_keys, H * (self.Dn + self.Dv)), self.dtype)
+        ops.latent_gather(cache.plane, cache.page_stride, cache.page_size, table, start, first, ctx.pos0, self.window, n_keys, self.Dk, rows, ctx.err)
+        linear(rows[:, :R], self.w_ukv, kv, STORE, ctx, M=n_keys)
+        ops.latent_q_rope_own(q, T, ctx.positions, self.rotary, H, self.Dn, self.Rr, ctx.err)
+        ops.attention_rows(q, kv, rows, R, n_keys, ov, key_row, ctx.q_start, ctx.pos0, work, n_work, H, self.scale, self.window, ctx.err,
+                           gate=gate, sink=self.w_sink, wide_weights=self.wide_weights)
