@@ -1186,6 +1186,10 @@ static int sm_count() {
 // Measured on a B200, us, 256 tokens a tile with the cut -> this choice: 391 x [5120, 3072] 24.5 -> 18.5, 391 x [3072, 3072]
 // 22.0 -> 15.5, 391 x [3072, 8192] 45 -> 28..38, 512 x [12288, 4096] 60 -> 45, 512 x [4096, 4096] 37 -> 19..26, 300 x 2 x [8192, 3072]
 // 47 -> 38, 1,024 x [6144, 4096] 74..81 -> 41..65, 2,048 x [3072, 8192] 90 -> 80; 2,048 x [4096, 4096] stays at 51..54.
+// From PAIR_MIN_TOKENS tokens on a product is the pair kernel's: up to 64 a single CTA's 64-token tile holds them all.  (With 65 to
+// 128 tokens the single-CTA kernel's last arriver adds up to eight 64 KB partials of a tile: a prompt step of four latent layers,
+// 100 tokens, 1485 us there and 836 here; 128 tokens of a hybrid of Mamba-2 and attention 1647 and 856.)
+constexpr int PAIR_MIN_TOKENS = 65;
 struct PairPlan {
   int bt, tiles_t;
   bool cut;
@@ -1227,6 +1231,7 @@ FERRUM_API int ferrum_gemm_tc_default_ctas() { return sm_count(); }
 
 // The single-CTA kernel's counters: one per 128-row tile (rounded up to pairs of them).
 static long long single_cta_tiles(int M, int N, int bt) { return 2LL * ((N + 2 * TILE_N - 1) / (2 * TILE_N)) * ((M + bt - 1) / bt); }
+static long long single_cta_floats(int bt, int dual, int n_ctas) { return 2LL * n_ctas * (long long)(bt * (dual ? 2 : 1)) * TILE_N; }
 
 // Workspace floats and tile counters a launch needs.  Partial tiles arise where a CTA's
 // range of units begins or ends inside a tile, so every CTA has two partial slots.
@@ -1234,14 +1239,15 @@ FERRUM_API long long ferrum_gemm_tc_workspace(int M, int N, int K, int dual, int
   const int bt = ferrum_gemm_tc_token_tile(M, dual);
   if (n_ctas <= 0) n_ctas = sm_count();
   long long tiles = single_cta_tiles(M, N, bt);
-  if (M > 0 && n_ctas >= 2 && (dual ? M > TILE_N : bt == PAIR_BT)) {
+  const bool pair = M >= PAIR_MIN_TOKENS && n_ctas >= 2;
+  if (pair) {
     // may run on the pair kernel (gate and up as one product of 2 N interleaved rows): it numbers the counters by 256-row tile and half
     const long long rows = dual ? 2LL * N : N;
     const PairPlan plan = pair_plan(M, rows, K, n_ctas / 2);
     if (plan.cut) tiles = std::max(tiles, 2LL * ((rows + 2 * TILE_N - 1) / (2 * TILE_N)) * plan.tiles_t);
   }
   if (n_tiles) *n_tiles = (int)tiles;
-  return 2LL * n_ctas * (long long)(bt * (dual ? 2 : 1)) * TILE_N;
+  return std::max(single_cta_floats(bt, dual, n_ctas), pair ? 2LL * n_ctas * PAIR_BT * TILE_N : 0);
 }
 
 // x [M, K] (row stride ldx) and w [w_rows, K] (row stride ldw) of the 16-bit type `dtype`
@@ -1289,7 +1295,7 @@ FERRUM_API int ferrum_gemm_tc(const void* x, const void* w, void* out, int dtype
   p.glu_limit = glu_limit;
   p.store_act = store_act;
   CUtensorMap mw, mx;
-  if (dual && M > TILE_N && g_pair_kernel && n_ctas >= 2 && ((uintptr_t)out & 15) == 0 && ldo % 8 == 0) {
+  if (dual && M >= PAIR_MIN_TOKENS && g_pair_kernel && n_ctas >= 2 && ((uintptr_t)out & 15) == 0 && ldo % 8 == 0) {
     // Two products of many tokens: the pair kernel computes them as one product whose weight
     // rows alternate between gate and up (a three-dimensional tensor map interleaves them on
     // the way into shared memory), and its epilogue applies the activation.
@@ -1312,7 +1318,7 @@ FERRUM_API int ferrum_gemm_tc(const void* x, const void* w, void* out, int dtype
     return launch_tc_pair(mw, mx, mo, ms, p, 2 * pairs, stream);
   }
   if (int r = get_tensor_map(w, w_rows, K, ldw, TILE_N, &mw)) return r;
-  if (bt == PAIR_BT && !dual && g_pair_kernel && n_ctas >= 2) {
+  if (M >= PAIR_MIN_TOKENS && !dual && g_pair_kernel && n_ctas >= 2) {
     // many tokens: pairs of CTAs on 256 x 256 tiles; each CTA stages 128 tokens
     const PairPlan plan = pair_plan(M, N, K, asked_ctas / 2);
     p.bt = plan.bt;
@@ -1511,8 +1517,8 @@ FERRUM_API int ferrum_gemm_tc_noalloc(const void* x, const void* w, void* out, i
   int n_ctas = sm_count();
   const int bt = ferrum_gemm_tc_token_tile(M, dual);
   int tiles = 0;
-  const long long need_floats = ferrum_gemm_tc_workspace(M, N, K, dual, n_ctas, &tiles);
-  tiles = (int)single_cta_tiles(M, N, bt);       // (this entry never takes the pair kernel)
+  const long long need_floats = single_cta_floats(bt, dual, n_ctas);      // (this entry never takes the pair kernel)
+  tiles = (int)single_cta_tiles(M, N, bt);
   FERRUM_CHECK_ARG(need_floats * (long long)sizeof(float) <= (long long)FERRUM_NOALLOC_SCRATCH_BYTES,
                    "gemm_tc_noalloc: %d tokens%s need %lld bytes of scratch, the built-in array holds %u; use ferrum_gemm_tc "
                    "with a caller-provided workspace", M, dual ? " with the SwiGLU epilogue" : "",

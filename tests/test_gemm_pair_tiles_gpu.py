@@ -20,7 +20,9 @@ CASES = [(321, 256, 8192, 12, False, 64, False), (161, 256, 8192, 12, True, 64, 
          (321, 256, 8192, 16, False, 128, True), (257, 320, 64, 8, False, 160, False), (129, 320, 64, 8, True, 160, False),
          (289, 256, 8192, 16, False, 160, True), (129, 256, 8192, 14, True, 160, True), (321, 320, 64, 8, False, 192, False),
          (513, 320, 8192, 10, False, 192, True), (385, 320, 64, 8, False, 224, False), (193, 320, 64, 10, True, 224, False),
-         (193, 640, 8192, 8, True, 224, True), (449, 320, 64, 10, False, 256, False)]
+         (193, 640, 8192, 8, True, 224, True), (449, 320, 64, 10, False, 256, False),
+         (65, 320, 64, 8, False, 96, False), (65, 300, 200, 6, True, 96, False), (97, 640, 8192, 10, False, 160, False),
+         (128, 500, 8192, 14, True, 160, False), (128, 256, 64, 4, False, 96, False)]
 
 
 def test_plan_widths():
@@ -29,7 +31,7 @@ def test_plan_widths():
     for M, N, K, ctas, dual, bt, cut in CASES:
         got = plan(ops, M, 2 * N if dual else N, K, ctas // 2)
         assert got == (bt, -(-M // bt), int(cut)), (M, N, K, ctas, dual, got)
-    for M in (129, 257, 300, 512, 2048, 20000):
+    for M in (65, 129, 257, 300, 512, 2048, 20000):
         for rows in (128, 3072, 28672):
             for pairs in (1, 5, 74):
                 bt, tiles, _ = plan(ops, M, rows, 4096, pairs)
