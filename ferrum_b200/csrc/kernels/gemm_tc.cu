@@ -1178,8 +1178,8 @@ static int sm_count() {
 // tokens has too few such tiles for the pairs (12 tiles of [3072, K] on 74 pairs), or a last wave that is nearly empty.
 // The estimate behind the choice: a pair's time is its k-blocks times what one costs.  A k-block of 64 elements took, in
 // units of one at 128 tokens (0.26 us): 0.92 at 64 tokens, 0.96 at 96, 1.07 at 160, 1.16 at 192, 1.33 at 224, 1.50 at
-// 256 (single waves of K = 3,072 to 14,336 and 49 to 13 waves of 2,048 x [28672, 4096]): up to 160 tokens it is the copies of
-// the weight tiles, the same whatever the tile, above that the products and the token tiles.  Cutting costs the partials
+// 256 (single waves of K = 3,072 to 14,336 and 49 to 13 waves of 2,048 x [28672, 4096]): up to 160 tokens it is what
+// does not depend on the tile (the weight tiles' copies, the issue of four instructions), above that the products and the token tiles.  Cutting costs the partials
 // and the wait for them, some 15 k-blocks for every 32 tokens of a tile.  A narrower tile has to promise 5 %: on long steps
 // the power limit sets the clock, and the wider tile moves fewer bytes (192 tokens a tile for 2,048 x [28672, 4096]: 2 %
 // by the estimate, and a whole 2,048-token step 4 % slower).
