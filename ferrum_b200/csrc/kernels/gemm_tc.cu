@@ -1130,6 +1130,8 @@ FERRUM_API void ferrum_gemm_tc_test_hooks(long long wait_cycles, int drop_loads)
   g_drop_loads = drop_loads != 0;
 }
 
+FERRUM_API int ferrum_gemm_tc_can_defer(int M, int N, int K, int dual, int n_ctas);
+
 static bool g_pair_kernel = true;
 // The CTA-pair kernel can be switched off (every shape then runs on the single-CTA kernel).
 FERRUM_API void ferrum_set_gemm_pair_kernel(int on) { g_pair_kernel = on != 0; }
@@ -1294,8 +1296,12 @@ FERRUM_API int ferrum_gemm_tc(const void* x, const void* w, void* out, int dtype
   p.glu_act = glu_act;
   p.glu_limit = glu_limit;
   p.store_act = store_act;
+  // (The test hook's dropped loads are the single-CTA kernel's.  A residual sum of up to 128 tokens that could be left in partials
+  // stays there too: whether it is left or added here, it is the same bits.)
+  const bool use_pair = g_pair_kernel && !g_drop_loads &&
+                        !(epilogue == TC_RESIDUAL && M <= TILE_N && ferrum_gemm_tc_can_defer(M, N, K, 0, asked_ctas));
   CUtensorMap mw, mx;
-  if (dual && M >= PAIR_MIN_TOKENS && g_pair_kernel && n_ctas >= 2 && ((uintptr_t)out & 15) == 0 && ldo % 8 == 0) {
+  if (dual && M >= PAIR_MIN_TOKENS && use_pair && n_ctas >= 2 && ((uintptr_t)out & 15) == 0 && ldo % 8 == 0) {
     // Two products of many tokens: the pair kernel computes them as one product whose weight
     // rows alternate between gate and up (a three-dimensional tensor map interleaves them on
     // the way into shared memory), and its epilogue applies the activation.
@@ -1318,7 +1324,7 @@ FERRUM_API int ferrum_gemm_tc(const void* x, const void* w, void* out, int dtype
     return launch_tc_pair(mw, mx, mo, ms, p, 2 * pairs, stream);
   }
   if (int r = get_tensor_map(w, w_rows, K, ldw, TILE_N, &mw)) return r;
-  if (M >= PAIR_MIN_TOKENS && !dual && g_pair_kernel && n_ctas >= 2) {
+  if (M >= PAIR_MIN_TOKENS && !dual && use_pair && n_ctas >= 2) {
     // many tokens: pairs of CTAs on 256 x 256 tiles; each CTA stages 128 tokens
     const PairPlan plan = pair_plan(M, N, K, asked_ctas / 2);
     p.bt = plan.bt;
