@@ -74,7 +74,8 @@ struct AttnTcParams {
   int* err;
   int ldo, page_size, page_shift, table_width;
   int Hkv, G, tok, window;
-  float scale_log2;
+  float scale_log2;     // of the score scale's size: its sign is in the products (see set_scale)
+  uint32_t negate;      // 1: keys go into the products of the scores negated
   // keys and values that lie as rows (ROWS): see ferrum_attention_rows
   const int* key_row;   // [R] row of a request's key 0 (may lie before its first row: only the keys in use have rows)
   const float* gate;    // [tokens][Hkv] factor of a head's output, or null
@@ -337,7 +338,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     // ------------------------------------------------------------ MMA issuer of one row tile
     if (elect_one()) {
       const int t = warp - 1;
-      const uint32_t idesc_qk = umma_idesc_16bit(128, BN, HALF);
+      const uint32_t idesc_qk = umma_idesc_16bit(128, BN, HALF) | p.negate << UMMA_NEGATE_B_BIT;
       const uint32_t idesc_pv = umma_idesc_16bit(128, D, HALF) | (1u << 16);  // B (values) is MN-major
       const uint32_t q_addr = smem_base + Cfg::OFF_Q + t * Cfg::Q_TILE_BYTES;
       const uint32_t o_tmem = tmem_base + Cfg::O_COL + t * D;
@@ -786,7 +787,7 @@ attention_tc_pair_kernel(const __grid_constant__ CUtensorMap map_kv, const uint1
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (the leader's, for both CTAs)
     if (rank == 0 && elect_one()) {
-      const uint32_t idesc_qk = umma_idesc_16bit(256, BN, HALF);
+      const uint32_t idesc_qk = umma_idesc_16bit(256, BN, HALF) | p.negate << UMMA_NEGATE_B_BIT;
       const uint32_t idesc_pv = umma_idesc_16bit(256, D, HALF) | (1u << 16);  // B (values) is MN-major
       const uint32_t q_tmem = tmem_base + Cfg::Q_COL, o_tmem = tmem_base + Cfg::O_COL;
       const uint64_t k_desc0 = umma_desc_k_sw128(smem_base + Cfg::OFF_K);
@@ -1097,6 +1098,14 @@ void keep_map(const AttnMapKey& key, const CUtensorMap& m) {
   g_maps.emplace(key, m);
 }
 
+// The kernels mask raw scores with -inf, look for the largest and scale behind it, which holds for a positive factor only.
+// A negative scale therefore negates the keys inside the product (free, and exact) and scales by its size; for a scale of zero
+// the smallest normal number leaves -inf where it is and makes every finite score a zero.
+void set_scale(AttnTcParams& p, float scale) {
+  p.negate = scale < 0.f;
+  p.scale_log2 = scale == 0.f ? 1.17549435e-38f : fabsf(scale) * 1.4426950408889634f;
+}
+
 // Queries [rows, ld] bfloat16 seen as (D, Hq, rows); a box is 64 columns x G heads x tok tokens.
 int query_map(const void* q, long long rows, int ldq, int Hq, int D, int G, int tok, CUtensorMap* out) {
   AttnMapKey key{q, rows, (long long)ldq * 4096 + D, (long long)Hq * 65536 + G * 256 + tok, 0};
@@ -1236,7 +1245,7 @@ FERRUM_API int ferrum_attention_tc(const void* q, int ldq, long long q_rows, voi
   p.page_shift = 0;
   while ((1 << p.page_shift) < page_size) ++p.page_shift;
   p.Hkv = Hkv; p.G = G; p.tok = tok; p.window = window;
-  p.scale_log2 = scale * 1.4426950408889634f;
+  set_scale(p, scale);
   CUtensorMap mq, mkv;
   if (int r = cache_map(kv_plane, n_pages, Hkv, page_size, D, &mkv)) return r;
   if (D == 128 && g_attention_pair && !wide) {
@@ -1335,7 +1344,7 @@ FERRUM_API int ferrum_attention_rows(const void* q, int ldq, long long q_rows, c
   AttnTcParams p = {};
   p.out = (uint16_t*)out; p.q_start = q_start; p.pos0 = pos0; p.work = work; p.err = err_flag;
   p.ldo = ldo; p.Hkv = H; p.G = 1; p.tok = 128; p.window = window; p.page_size = TC_BN;
-  p.scale_log2 = scale * 1.4426950408889634f;
+  set_scale(p, scale);
   p.key_row = key_row; p.gate = gate; p.sink = sink;
   p.k_cols = 0; p.v_cols = H * 128; p.rot_col = rot_col;
   CUtensorMap mq, mkv, mrot;

@@ -147,6 +147,7 @@ __device__ __forceinline__ uint32_t umma_idesc_16bit(int M, int N, bool half) {
   d |= (uint32_t)(M >> 4) << 24;    // M / 16
   return d;
 }
+constexpr int UMMA_NEGATE_B_BIT = 14;    // of an instruction descriptor: the product takes -B
 __device__ __forceinline__ uint32_t umma_idesc_bf16(int M, int N) { return umma_idesc_16bit(M, N, false); }
 __device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, bool accumulate) {
   asm volatile(

@@ -25,28 +25,36 @@ def test_rows_plan():
         assert [h - l for _, _, l, h, *_ in items.tolist()] == sorted((h - l for _, _, l, h, *_ in items.tolist()), reverse=True)
 
 
-class OneMixer:
-    def __init__(self, mixer):
+class Mixers:
+    """A mixer that caches its rows and, if there is a second, a reader of them."""
+
+    def __init__(self, mixers):
         from ferrum_b200.models import Run
-        self.mixer, self.schedule = mixer, [Run(0)]
+        self.mixers, self.schedule = mixers, [Run(0)] + [Run(k, cache_of=0) for k in range(1, len(mixers))]
 
     def cache_needs(self):
-        return [self.mixer.cache_need()]
+        return [m.cache_need() for m in self.mixers]
 
 
-def exact(w, x, H, R, scale, window, rot, sink, eps):
-    """float64, one sequence from position 0."""
+def exact(w, writer, x, H, R, scale, window, rot, sink, eps):
+    """float64, one sequence from position 0; the latent and the shared key part by the weights of `writer`."""
     T = x.shape[0]
     rms = lambda v: v * torch.rsqrt((v * v).mean(-1, keepdim=True) + eps)
     pos = torch.arange(T, device="cuda")
 
-    def turn(v):          # [T, n, 64], halves paired
+    def turn(v):          # [T, n, 64]: the table's leading dimensions turn, paired as it says
+        if rot is None:
+            return v
+        n = rot.rope_dim
         a = rot.cos_sin[:T].double()
         c, s = a[:, None, :, 0], a[:, None, :, 1]
-        p, q = v[..., :32], v[..., 32:]
-        return torch.cat([p * c - q * s, q * c + p * s], -1)
-    d = x @ w["dkv.weight"].T
-    c = rms(d[:, :R]) * w["dkv_norm.weight"]
+        head = v[..., :n]
+        p, q = (head[..., :n // 2], head[..., n // 2:]) if rot.pairing else (head[..., ::2], head[..., 1::2])
+        p, q = p * c - q * s, q * c + p * s
+        head = torch.cat([p, q], -1) if rot.pairing else torch.stack([p, q], -1).flatten(-2)
+        return torch.cat([head, v[..., n:]], -1)
+    d = x @ writer["dkv.weight"].T
+    c = rms(d[:, :R]) * writer["dkv_norm.weight"]
     kr = turn(d[:, None, R:]).expand(T, H, 64)
     q = ((rms(x @ w["dq.weight"].T) * w["dq_norm.weight"]) @ w["uq.weight"].T).view(T, H, 192)
     q = torch.cat([q[..., :128], turn(q[..., 128:])], -1)
@@ -62,31 +70,49 @@ def exact(w, x, H, R, scale, window, rot, sink, eps):
     return o.reshape(T, H * 128) @ w["o.weight"].T
 
 
+# The plain case, sinks, windows and ranks; then scales that are not positive (which turn or level the scores), the other
+# pairing, a table of half of the shared part, none, and a layer that reads the rows another one cached, which has a window of its own.
+CASES = {"plain": dict(H=2, R=512), "sink-wide": dict(H=5, R=72, sink=True, wide=True), "window": dict(H=3, R=128, window=100),
+         "window-sink": dict(H=1, R=64, window=300, sink=True),
+         "negative": dict(H=2, R=512, scale=-0.07), "negative-window-sink-wide": dict(H=2, R=64, scale=-0.07, window=100, sink=True, wide=True),
+         "zero": dict(H=2, R=64, scale=0.0, sink=True), "adjacent": dict(H=2, R=128, rot=(64, "adjacent")),
+         "half-turned": dict(H=2, R=128, rot=(32, "half")), "half-turned-adjacent": dict(H=3, R=64, rot=(32, "adjacent")),
+         "unturned": dict(H=2, R=128, rot=None), "reader": dict(H=2, R=128, reader=True), "reader-window": dict(H=3, R=64, reader=True, window=200)}
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("td", [torch.bfloat16, torch.float16])
-@pytest.mark.parametrize("H,R,window,sink,wide", [(2, 512, 0, False, False), (5, 72, 0, True, True), (3, 128, 100, False, False), (1, 64, 300, True, False)])
-def test_latent_rows(td, H, R, window, sink, wide, monkeypatch):
+@pytest.mark.parametrize("case", list(CASES))
+def test_latent_rows(td, case, monkeypatch):
     from ferrum_b200.cache import CacheStorage
     from ferrum_b200.engine.batch import StepContext, StepEntry
     from ferrum_b200.ops import lib as ops
     from ferrum_b200.parts import LatentAttention, RotaryEmbedding, latent_attention
     ops.require_cuda()
-    E, Rq, eps, scale = 256, 96, 1e-5, 192 ** -0.5
-    rot = RotaryEmbedding(64, 64, 10000.0, None, "half", 1024, "cuda")
-    mixer = LatentAttention(E, H, 128, 64, 128, R, Rq, eps, scale, td, rotary=rot, window=window, sink=sink, wide_weights=wide)
+    spec = dict(window=0, sink=False, wide=False, scale=192 ** -0.5, rot=(64, "half"), reader=False)
+    spec.update(CASES[case])
+    H, R, window, sink, scale = (spec[k] for k in ("H", "R", "window", "sink", "scale"))
+    E, Rq, eps = 256, 96, 1e-5
+    rot = RotaryEmbedding(64, spec["rot"][0], 10000.0, None, spec["rot"][1], 1024, "cuda") if spec["rot"] else None
     g = torch.Generator(device="cuda").manual_seed(H + R)
-    w = {}
-    for name, spec in mixer.param_specs().items():
-        t = torch.randn(spec.shape, device="cuda", generator=g)
-        t = t * spec.shape[-1] ** -0.5 if spec.kind == "matrix" else (1.0 + 0.1 * t if "norm" in name else t)
-        t = t.to(td) if spec.kind == "matrix" else t
-        mixer.assign(name, t.contiguous())
-        w[name] = t.double()
-    mixer.finalize()
-    cache = CacheStorage(OneMixer(mixer), td, "cuda", page_size=16, max_tokens=4096, max_requests=4, max_model_len=1024)
+    mixers, ws = [], []
+    for k in range(1 + spec["reader"]):
+        mixer = LatentAttention(E, H, 128, 64, 128, R, Rq, eps, scale, td, rotary=rot, own_latent=k == 0, sink=sink, wide_weights=spec["wide"],
+                                window=window if k == spec["reader"] else 0)
+        w = {}
+        for name, p in mixer.param_specs().items():
+            t = torch.randn(p.shape, device="cuda", generator=g)
+            t = t * p.shape[-1] ** -0.5 if p.kind == "matrix" else (1.0 + 0.1 * t if "norm" in name else t)
+            t = t.to(td) if p.kind == "matrix" else t
+            mixer.assign(name, t.contiguous())
+            w[name] = t.double()
+        mixer.finalize()
+        mixers.append(mixer)
+        ws.append(w)
+    cache = CacheStorage(Mixers(mixers), td, "cuda", page_size=16, max_tokens=4096, max_requests=4, max_model_len=1024)
     ctx = StepContext("cuda", 1024, 4, [cache.table_width])
     xs = [torch.randn(n, E, device="cuda", generator=g).to(td) for n in (700, 257, 300)]
-    refs = [exact(w, x.double(), H, R, scale, window, rot, w.get("sink"), eps) for x in xs]
+    refs = [exact(ws[-1], ws[0], x.double(), H, R, scale, window, rot, ws[-1].get("sink"), eps) for x in xs]
     calls = []
     real = ops.attention_rows
     monkeypatch.setattr(ops, "attention_rows", lambda *a, **k: (calls.append(1), real(*a, **k))[1])
@@ -103,8 +129,9 @@ def test_latent_rows(td, H, R, window, sink, wide, monkeypatch):
                     cache.manager.grow(slots[r], at[r] + n)
                 ctx.fill([StepEntry(slots[r], at[r], [0] * n) for r, n in rows], cache.manager)
                 x = torch.cat([xs[r][at[r]:at[r] + n] for r, n in rows])
-                y = torch.full((x.shape[0], E), float("nan"), device="cuda")
-                mixer.forward(x, ctx, cache.layer_cache(0), y, accumulate=False)
+                for k, mixer in enumerate(mixers):
+                    y = torch.full((x.shape[0], E), float("nan"), device="cuda")
+                    mixer.forward(x, ctx, cache.layer_cache(k), y, accumulate=False)
                 assert ctx.err.item() == 0
                 t = 0
                 for r, n in rows:
