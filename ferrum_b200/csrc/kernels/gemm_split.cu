@@ -1,15 +1,16 @@
 // out[t, n] (=, +=) sum_k x[t, k] * w[n, k] for float32 operands on the tcgen05 tensor cores.
 //
 // The tensor cores have no float32 input type, but a float32 is exactly the sum of three bfloat16 values:
-// h = the upper 16 bits of v, m = the upper 16 bits of v - h, l = v - h - m (both differences are exact, and
-// the 24 bits of the significand are 8 + 8 + 8).  Of the nine products of two such sums six are formed,
-// hh, hm, mh, mm, hl and lh; what is left out (ml, lm, ll) is below 2^-23 of a product of the two values and
-// 1.5e-8 of it on average.  A product of two bfloat16 values is exact in float32; what a sum loses, it loses when
+// h = v rounded to bfloat16, m = v - h rounded, l = v - h - m (both differences are exact, and l has at most seven
+// bits left).  Of the nine products of two such sums six are formed, hh, hm, mh, mm, hl and lh; what is left out (ml, lm,
+// ll) is below 2^-24 of a product of the two values, 3.5e-9 of it on average, and of either sign (parts that are cut off instead of
+// rounded all have the value's sign: what is left out is then up to 2^-21, 4e-8 on average, and always makes the product smaller).
+// A product of two bfloat16 values is exact in float32; what a sum loses, it loses when
 // it is added up.  The matrix unit cuts off where it adds, so its accumulator is never the whole sum: it takes
 // 64 elements of K at a time, the small terms first (24 instructions, of which only the last four add at
 // full size), and the epilogue's warps add each such piece to the sum of the pieces before it in registers,
 // rounded to nearest.  (Error of 300 rows of standard normal elements against float64, 2-norm over 2-norm: K = 3,072
-// 1.4e-7, K = 8,192 1.6e-7; the CUDA cores' tiled kernel, one FFMA accumulator over K, 9.9e-7 and 1.6e-6.)
+// 1.1e-7, K = 8,192 1.2e-7; the CUDA cores' tiled kernel, one FFMA accumulator over K, 9.9e-7 and 1.6e-6.)
 //
 // The order of an output's sum is a function of N and K alone: pieces of 64 in K order within a range of K, and the
 // ranges (their number depends on N and K) in K order.  A token's result does not depend on the other tokens.
@@ -25,7 +26,7 @@
 // `split_sum_kernel`: the last CTA of a tile adding them itself was a serial tail of some 25 us.
 // Measured on a B200, us, FFMA tiles -> this: 300 tokens x [5120, 3072] 332 -> 70, x [3072, 3072] 332 -> 47, x [16384, 3072]
 // 898 -> 173, x [3072, 8192] 909 -> 92; 1,024 tokens x [16384, 3072] 2,090 -> 453 (228 TFLOP/s: 1.37 PFLOP/s of bfloat16
-// products, 0.82 of the measured burst peak). 
+// products, 0.84 of the measured burst peak).
 //
 // Roles (320 threads): warp 0 = TMA producer, warp 1 = TMEM owner and MMA issuer, warps 2..5 = sums and
 // epilogue, warps 6..9 = conversion of the weights.  Every wait is bounded; on a timeout the kernel raises the
@@ -88,18 +89,18 @@ __device__ __forceinline__ void gs_tmem_st8(uint32_t taddr, const uint32_t (&r)[
                : "memory");
 }
 
-// The upper halves of two words side by side, the first in the low half.
-__device__ __forceinline__ uint32_t upper_halves(uint32_t a, uint32_t b) { return __byte_perm(a, b, 0x7632); }
-
+// Two float32 values rounded to bfloat16, the first in the low half.
+__device__ __forceinline__ uint32_t round2(float a, float b) {
+  uint32_t r;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(b), "f"(a));
+  return r;
+}
 // Two float32 values as the sums of three bfloat16 values each, packed pairwise.
 __device__ __forceinline__ void split2(float a, float b, uint32_t& h, uint32_t& m, uint32_t& l) {
-  const uint32_t ua = __float_as_uint(a), ub = __float_as_uint(b);
-  const float ra = a - __uint_as_float(ua & 0xffff0000u), rb = b - __uint_as_float(ub & 0xffff0000u);
-  const uint32_t va = __float_as_uint(ra), vb = __float_as_uint(rb);
-  const float sa = ra - __uint_as_float(va & 0xffff0000u), sb = rb - __uint_as_float(vb & 0xffff0000u);
-  h = upper_halves(ua, ub);
-  m = upper_halves(va, vb);
-  l = upper_halves(__float_as_uint(sa), __float_as_uint(sb));
+  h = round2(a, b);
+  const float ra = a - __uint_as_float(h << 16), rb = b - __uint_as_float(h & 0xffff0000u);
+  m = round2(ra, rb);
+  l = round2(ra - __uint_as_float(m << 16), rb - __uint_as_float(m & 0xffff0000u));
 }
 
 // x [M, K] float32 -> planes [3, M, K] bfloat16 (h, m, l).  K a multiple of 8, rows 16-byte aligned.

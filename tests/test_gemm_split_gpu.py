@@ -32,9 +32,9 @@ def test_gemm_split(ops, M, N, K):
     x = torch.randn(M, K, device="cuda", generator=g)
     w = torch.randn(N, K, device="cuda", generator=g)
     ref = x.double() @ w.double().T
-    # Of |x| |w|: 2^-23 for the products left out, 2^-22 for the matrix unit's cut-offs within a piece, half an ulp for
+    # Of |x| |w|: 2^-24 for the products left out, 2^-22 for the matrix unit's cut-offs within a piece, half an ulp for
     # every piece and range that is added.
-    bound = (x.double().abs() @ w.double().abs().T) * (2.0 ** -23 + 2.0 ** -22 + (K // 64 + 9) * 2.0 ** -24)
+    bound = (x.double().abs() @ w.double().abs().T) * (2.0 ** -24 + 2.0 ** -22 + (K // 64 + 9) * 2.0 ** -24)
     out = run(ops, x, w)
     assert ((out.double() - ref).abs() <= bound).all()
     res = torch.randn(M, N, device="cuda", generator=g)
@@ -49,6 +49,21 @@ def test_gemm_split(ops, M, N, K):
     wide = torch.randn(len(pick), K + 12, device="cuda", generator=g)
     wide[:, :K] = x[pick]
     assert torch.equal(run(ops, wide[:, :K], w), out[pick])
+
+
+@pytest.mark.parametrize("K", [512, 3072])
+@pytest.mark.parametrize("kind", ["any", "long"])
+def test_gemm_split_one_sign(ops, K, kind):
+    """Where all products are positive nothing that is left out or cut off cancels: the error stays near half an ulp (2^-24) of the
+    result and as much for the matrix unit's cut-offs.  "long": all lower bits of a significand set but for the last few, which makes
+    the parts that are left out as large as they get."""
+    g = torch.Generator(device="cuda").manual_seed(K)
+    x, w = (torch.randn(n, K, device="cuda", generator=g).abs() for n in (300, 1024))
+    if kind == "long":
+        draw = lambda t, n: torch.randint(0, n, t.shape, device="cuda", generator=g)
+        x, w = ((0x3F80FF00 + draw(t, 256) + (draw(t, 128) << 16)).to(torch.int32).view(torch.float32) for t in (x, w))
+    ref = x.double() @ w.double().T
+    assert ((run(ops, x, w).double() - ref).norm() / ref.norm()).item() <= 2.0 ** -23
 
 
 def test_gemm_split_values(ops):
