@@ -5,6 +5,9 @@
 // bits left).  Of the nine products of two such sums six are formed, hh, hm, mh, mm, hl and lh; what is left out (ml, lm,
 // ll) is below 2^-24 of a product of the two values, 3.5e-9 of it on average, and of either sign (parts that are cut off instead of
 // rounded all have the value's sign: what is left out is then up to 2^-21, 4e-8 on average, and always makes the product smaller).
+// bfloat16's exponents end where float32's do, so the low part of a value below some 2^-102 would be cut off: the parts are
+// those of 2^24 v, which are zero or normal for every v, subnormal ones too, and an output is 2^-48 of its sum.  (Values from 2^103 and
+// sums from 2^80 on overflow there; see the last paragraph.)
 // A product of two bfloat16 values is exact in float32; what a sum loses, it loses when
 // it is added up.  The matrix unit cuts off where it adds, so its accumulator is never the whole sum: it takes
 // 64 elements of K at a time, the small terms first (24 instructions, of which only the last four add at
@@ -32,9 +35,9 @@
 // epilogue, warps 6..9 = conversion of the weights.  Every wait is bounded; on a timeout the kernel raises the
 // error flag, lets the copies in flight land, frees its tensor memory and returns.
 //
-// Infinities and NaN: the parts of an infinite value are not finite either, and inf * 0 among them may give NaN
+// Infinities, NaN and overflow: the parts of an infinite value are not finite either, and inf * 0 among them may give NaN
 // where the plain sum gives an infinity.  An output that is not finite is therefore summed again, plainly, in K
-// order: it comes out as the CUDA cores' kernel gives it.
+// order, of the values as they are: it comes out as the CUDA cores' kernel gives it.
 #include <algorithm>
 
 #include <cuda.h>
@@ -57,6 +60,7 @@ constexpr int GS_SMEM_BYTES = GS_RAW_STAGES * GS_RAW_BYTES + GS_X_STAGES * GS_X_
 constexpr int GS_A_COL = 2 * GS_TILE_T;     // tensor-memory columns: two accumulators, then two sets of weight parts
 constexpr int GS_A_COLS = 3 * GS_KC / 2;
 constexpr int GS_MAX_SPLITS = 8;
+constexpr float GS_UP = 16777216.f, GS_DOWN = 1.f / GS_UP / GS_UP;   // 2^24 for each operand, 2^-48 for a sum
 
 struct SplitParams {
   const float* x;
@@ -89,21 +93,34 @@ __device__ __forceinline__ void gs_tmem_st8(uint32_t taddr, const uint32_t (&r)[
                : "memory");
 }
 
-// Two float32 values rounded to bfloat16, the first in the low half.
-__device__ __forceinline__ uint32_t round2(float a, float b) {
+// Two float32 values of a pair rounded to bfloat16, the first in the low half.
+__device__ __forceinline__ uint32_t round2(float2 v) {
   uint32_t r;
-  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(b), "f"(a));
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(v.y), "f"(v.x));
   return r;
 }
-// Two float32 values as the sums of three bfloat16 values each, packed pairwise.
+// v - (the two bfloat16 values of h), in one instruction for both: exact where h is v rounded.
+__device__ __forceinline__ float2 minus2(float2 v, uint32_t h) {
+  float2 r;
+  asm("{\n\t.reg .b64 a, b, c;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %4};\n\tmov.b64 c, {%5, %6};\n\t"
+      "fma.rn.f32x2 a, a, b, c;\n\tmov.b64 {%0, %1}, a;\n\t}"
+      : "=f"(r.x), "=f"(r.y)
+      : "f"(__uint_as_float(h << 16)), "f"(__uint_as_float(h & 0xffff0000u)), "f"(-1.f), "f"(v.x), "f"(v.y));
+  return r;
+}
+// Two float32 values, times GS_UP, as the sums of three bfloat16 values each, packed pairwise.
 __device__ __forceinline__ void split2(float a, float b, uint32_t& h, uint32_t& m, uint32_t& l) {
-  h = round2(a, b);
-  const float ra = a - __uint_as_float(h << 16), rb = b - __uint_as_float(h & 0xffff0000u);
-  m = round2(ra, rb);
-  l = round2(ra - __uint_as_float(m << 16), rb - __uint_as_float(m & 0xffff0000u));
+  float2 v;
+  asm("{\n\t.reg .b64 a, b;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %4};\n\tmul.rn.f32x2 a, a, b;\n\tmov.b64 {%0, %1}, a;\n\t}"
+      : "=f"(v.x), "=f"(v.y)
+      : "f"(a), "f"(b), "f"(GS_UP));
+  h = round2(v);
+  v = minus2(v, h);
+  m = round2(v);
+  l = round2(minus2(v, m));
 }
 
-// x [M, K] float32 -> planes [3, M, K] bfloat16 (h, m, l).  K a multiple of 8, rows 16-byte aligned.
+// x [M, K] float32 -> planes [3, M, K] bfloat16 (h, m, l of GS_UP x).  K a multiple of 8, rows 16-byte aligned.
 __global__ void __launch_bounds__(256)
 split_rows_kernel(const float* __restrict__ x, int M, int K, int ldx, uint16_t* __restrict__ planes) {
   pdl_launch();
@@ -127,9 +144,9 @@ split_rows_kernel(const float* __restrict__ x, int M, int K, int ldx, uint16_t* 
   }
 }
 
-// An output that did not come out finite, once more and plainly.
+// The output of a sum of products of the scaled parts; one that is not finite, once more and plainly.
 __device__ __noinline__ float finite_or_plain(const SplitParams& p, int t, int n, float v) {
-  if (isfinite(v)) return v;
+  if (isfinite(v)) return v * GS_DOWN;
   const float* xr = p.x + (size_t)t * p.ldx;
   const float* wr = p.w + (size_t)n * p.ldw;
   float sum = 0.f;
@@ -143,10 +160,10 @@ __device__ __forceinline__ void finish16(const SplitParams& p, int t, int n, int
   bool fine = true;
 #pragma unroll
   for (int j = 0; j < 16; ++j) fine = fine && (j >= count || isfinite(v[j]));
-  if (!fine) {
 #pragma unroll
-    for (int j = 0; j < 16; ++j)
-      if (j < count) v[j] = finite_or_plain(p, t + j, n, v[j]);
+  for (int j = 0; j < 16; ++j) {
+    if (fine) v[j] *= GS_DOWN;
+    else if (j < count) v[j] = finite_or_plain(p, t + j, n, v[j]);
   }
   float r[16];
 #pragma unroll
@@ -184,7 +201,9 @@ split_sum_kernel(const SplitParams p) {
           v.w += part[q].w;
         }
       }
-      if (!(isfinite(v.x) && isfinite(v.y) && isfinite(v.z) && isfinite(v.w))) {
+      if (isfinite(v.x) && isfinite(v.y) && isfinite(v.z) && isfinite(v.w)) {
+        v = make_float4(v.x * GS_DOWN, v.y * GS_DOWN, v.z * GS_DOWN, v.w * GS_DOWN);
+      } else {
         v.x = finite_or_plain(p, t, n, v.x);
         v.y = finite_or_plain(p, t, n + 1, v.y);
         v.z = finite_or_plain(p, t, n + 2, v.z);

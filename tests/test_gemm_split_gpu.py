@@ -73,6 +73,12 @@ def test_gemm_split_values(ops):
     w = torch.randn(256, 1024, device="cuda", generator=g) * 1e-22
     ref = x.double() @ w.double().T
     assert ((run(ops, x, w).double() - ref).abs() <= (x.double().abs() @ w.double().abs().T) * 2.0 ** -20).all()
+    # at the lower end of float32, subnormal operands among them, the three parts are still exact (an output may be subnormal itself:
+    # half of its last place, 2^-150, comes on top); at the upper end the outputs are summed again plainly
+    for up, down in ((1.0, 1e-36), (1e-33, 1e2), (1.0, 1e-38), (3e-39, 1e3), (1e30, 1e-37), (1e32, 1.0), (1e-3, 1e33), (1e13, 1e13)):
+        a, b = (x.double() * (up * 1e-18)).float(), (w.double() * (down * 1e22)).float()
+        ref = a.double() @ b.double().T
+        assert ((run(ops, a, b).double() - ref).abs() <= (a.double().abs() @ b.double().abs().T) * 2.0 ** -18 + 2.0 ** -150).all(), (up, down)
     x = torch.randn(70, 1024, device="cuda", generator=g)
     w = torch.randn(256, 1024, device="cuda", generator=g)
     x[3, 17], x[9, 1000], x[20, 5], x[20, 6] = float("inf"), float("-inf"), float("nan"), 2.0
