@@ -36,8 +36,11 @@
 // error flag, lets the copies in flight land, frees its tensor memory and returns.
 //
 // Infinities, NaN and overflow: the parts of an infinite value are not finite either, and inf * 0 among them may give NaN
-// where the plain sum gives an infinity.  An output that is not finite is therefore summed again, plainly, in K
-// order, of the values as they are: it comes out as the CUDA cores' kernel gives it.
+// where the plain sum gives an infinity.  An output that is not finite is therefore summed again, plainly, of the values as
+// they are, by a whole warp (`plain16`, `plain_quads`): NaN, an infinity or a finite sum, as the CUDA cores' kernel gives it.
+// (Only where finite terms overflow beside an infinity of the other sign does the order of the terms decide between the two.)
+// Cost, B200, 300 tokens, one token with a NaN / all: x [3072, 3072] 52 -> 160 / 286 us, x [16384, 3072] 183 -> 183 / 292; the FFMA tiles
+// take 334 and 908 whatever the values.
 #include <algorithm>
 
 #include <cuda.h>
@@ -144,27 +147,64 @@ split_rows_kernel(const float* __restrict__ x, int M, int K, int ldx, uint16_t* 
   }
 }
 
-// The output of a sum of products of the scaled parts; one that is not finite, once more and plainly.
-__device__ __noinline__ float finite_or_plain(const SplitParams& p, int t, int n, float v) {
-  if (isfinite(v)) return v * GS_DOWN;
+// The outputs that are not finite among feature n of tokens t .. t + 15, summed again plainly in K order, and the others' scale: a
+// whole warp, a lane per feature.  The lanes share the tokens' elements; once every such sum is a NaN the rest cannot change it.
+__device__ __noinline__ void plain16(const SplitParams& p, int t, int n, float (&v)[16]) {
+  unsigned own = 0;
+#pragma unroll
+  for (int j = 0; j < 16; ++j) own |= (unsigned)(n < p.N && t + j < p.M && !isfinite(v[j])) << j;
+  const unsigned rows = __reduce_or_sync(0xffffffffu, own);
   const float* xr = p.x + (size_t)t * p.ldx;
-  const float* wr = p.w + (size_t)n * p.ldw;
-  float sum = 0.f;
-  for (int k = 0; k < p.K; ++k) sum = fmaf(xr[k], wr[k], sum);
-  return sum;
+  const float* wr = p.w + (size_t)min(n, p.N - 1) * p.ldw;
+  float sum[16];
+#pragma unroll
+  for (int j = 0; j < 16; ++j) sum[j] = 0.f;
+  for (int k = 0; k < p.K; k += 8) {
+    const float4 a = *reinterpret_cast<const float4*>(wr + k), b = *reinterpret_cast<const float4*>(wr + k + 4);
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      if (rows >> j & 1) {
+        const float4 c = *reinterpret_cast<const float4*>(xr + (size_t)j * p.ldx + k), d = *reinterpret_cast<const float4*>(xr + (size_t)j * p.ldx + k + 4);
+        sum[j] = fmaf(c.x, a.x, sum[j]);
+        sum[j] = fmaf(c.y, a.y, sum[j]);
+        sum[j] = fmaf(c.z, a.z, sum[j]);
+        sum[j] = fmaf(c.w, a.w, sum[j]);
+        sum[j] = fmaf(d.x, b.x, sum[j]);
+        sum[j] = fmaf(d.y, b.y, sum[j]);
+        sum[j] = fmaf(d.z, b.z, sum[j]);
+        sum[j] = fmaf(d.w, b.w, sum[j]);
+      }
+    }
+    if ((k & 56) == 0) {
+      bool lost = true;
+#pragma unroll
+      for (int j = 0; j < 16; ++j) lost = lost && (!(own >> j & 1) || isnan(sum[j]));
+      if (__all_sync(0xffffffffu, lost)) break;
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 16; ++j) v[j] = own >> j & 1 ? sum[j] : v[j] * GS_DOWN;
 }
 
-// Feature n of tokens t .. t + count - 1 (at most 16) goes to `out`: the loads first, so that they overlap.
+// A whole warp, feature n in every lane: tokens t .. t + count - 1 (at most 16) go to `out`, the loads first, so that they overlap.
 __device__ __forceinline__ void finish16(const SplitParams& p, int t, int n, int count, float* v) {
+  const bool mine = n < p.N;
   float* o = p.out + (size_t)t * p.ldo + n;
   bool fine = true;
 #pragma unroll
   for (int j = 0; j < 16; ++j) fine = fine && (j >= count || isfinite(v[j]));
+  if (__all_sync(0xffffffffu, fine || !mine)) {
 #pragma unroll
-  for (int j = 0; j < 16; ++j) {
-    if (fine) v[j] *= GS_DOWN;
-    else if (j < count) v[j] = finite_or_plain(p, t + j, n, v[j]);
+    for (int j = 0; j < 16; ++j) v[j] *= GS_DOWN;
+  } else {
+    float copy[16];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) copy[j] = v[j];
+    plain16(p, t, n, copy);
+#pragma unroll
+    for (int j = 0; j < 16; ++j) v[j] = copy[j];
   }
+  if (!mine) return;
   float r[16];
 #pragma unroll
   for (int j = 0; j < 16; ++j) r[j] = p.add && j < count ? o[(size_t)j * p.ldo] : 0.f;
@@ -173,25 +213,71 @@ __device__ __forceinline__ void finish16(const SplitParams& p, int t, int n, int
     if (j < count) o[(size_t)j * p.ldo] = p.add ? r[j] + v[j] : v[j];
 }
 
-// out[t, n] (=, +=) the sum of the ranges' partial sums, in K order; a thread takes four neighbouring features.
+// Features n .. n + count - 1 of token t in every lane, at most four, of which the bits of `bad` are to be summed again (none: v is
+// handed back): a whole warp takes one lane's quad after the other, lane l the elements 4 l .. 4 l + 3 of every 128, and the lanes' sums
+// meet at the end.  (A thread on its own walked K in 7 ms where one token of a 3072 x 3072 product had a NaN.)
+__device__ __noinline__ float4 plain_quads(const SplitParams& p, int t, int n, int count, unsigned bad, float4 v) {
+  const int lane = threadIdx.x & 31;
+  for (unsigned todo = __ballot_sync(0xffffffffu, bad != 0); todo; todo &= todo - 1) {
+    const int from = __ffs(todo) - 1;
+    const int ft = __shfl_sync(0xffffffffu, t, from), fn = __shfl_sync(0xffffffffu, n, from), fc = __shfl_sync(0xffffffffu, count, from);
+    const unsigned fbad = __shfl_sync(0xffffffffu, bad, from);
+    const float* xr = p.x + (size_t)ft * p.ldx;
+    const float* wr = p.w + (size_t)fn * p.ldw;
+    float sum[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int k0 = 0; k0 < p.K; k0 += 256) {
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int k = k0 + u * 128 + lane * 4;
+        if (k < p.K) {
+          const float4 a = *reinterpret_cast<const float4*>(xr + k);
+#pragma unroll
+          for (int f = 0; f < 4; ++f) {
+            if (f < fc) {
+              const float4 b = *reinterpret_cast<const float4*>(wr + (size_t)f * p.ldw + k);
+              sum[f] = fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, sum[f]))));
+            }
+          }
+        }
+      }
+      bool lost = true;      // a NaN in every sum that is asked for: the rest cannot change it
+#pragma unroll
+      for (int f = 0; f < 4; ++f) lost = lost && (!(fbad >> f & 1) || isnan(sum[f]));
+      if (__any_sync(0xffffffffu, lost)) break;
+    }
+#pragma unroll
+    for (int f = 0; f < 4; ++f)
+#pragma unroll
+      for (int d = 16; d > 0; d >>= 1) sum[f] += __shfl_xor_sync(0xffffffffu, sum[f], d);
+    if (lane == from) v = make_float4(bad & 1 ? sum[0] : v.x, bad & 2 ? sum[1] : v.y, bad & 4 ? sum[2] : v.z, bad & 8 ? sum[3] : v.w);
+  }
+  return v;
+}
+
+// out[t, n] (=, +=) the sum of the ranges' partial sums, in K order; a thread takes four neighbouring features, and a warp
+// stays together for the outputs that are summed again.
 __global__ void __launch_bounds__(256)
 split_sum_kernel(const SplitParams p) {
   pdl_launch();
   pdl_wait();
-  const int groups = (p.N + 3) / 4;
+  const int lane = threadIdx.x & 31, groups = (p.N + 3) / 4;
   const size_t plane = (size_t)p.M * p.N;
+  const long long quads = (long long)p.M * groups;
   const bool vec = p.N % 4 == 0 && p.ldo % 4 == 0 && ((uintptr_t)p.out & 15) == 0;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < (long long)p.M * groups; i += (long long)gridDim.x * blockDim.x) {
-    const int t = (int)(i / groups), n = (int)(i - (long long)t * groups) * 4;
+  for (long long i0 = (long long)blockIdx.x * blockDim.x + threadIdx.x - lane; i0 < quads; i0 += (long long)gridDim.x * blockDim.x) {
+    const long long i = min(i0 + lane, quads - 1);      // (lanes past the end go along with the last quad and write nothing)
+    const int t = (int)(i / groups), n = (int)(i - (long long)t * groups) * 4, count = min(4, p.N - n);
+    const bool mine = i0 + lane < quads;
     const float* src = p.partials + (size_t)t * p.N + n;
     float* o = p.out + (size_t)t * p.ldo + n;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f), r = v;
     if (vec) {
-      float4 part[GS_MAX_SPLITS], r = make_float4(0.f, 0.f, 0.f, 0.f);
+      float4 part[GS_MAX_SPLITS];
 #pragma unroll
       for (int q = 0; q < GS_MAX_SPLITS; ++q)
         if (q < p.splits) part[q] = __ldcg(reinterpret_cast<const float4*>(src + q * plane));
-      if (p.add) r = *reinterpret_cast<const float4*>(o);
-      float4 v = part[0];
+      if (p.add && mine) r = *reinterpret_cast<const float4*>(o);
+      v = part[0];
 #pragma unroll
       for (int q = 1; q < GS_MAX_SPLITS; ++q) {
         if (q < p.splits) {
@@ -201,24 +287,33 @@ split_sum_kernel(const SplitParams p) {
           v.w += part[q].w;
         }
       }
-      if (isfinite(v.x) && isfinite(v.y) && isfinite(v.z) && isfinite(v.w)) {
-        v = make_float4(v.x * GS_DOWN, v.y * GS_DOWN, v.z * GS_DOWN, v.w * GS_DOWN);
-      } else {
-        v.x = finite_or_plain(p, t, n, v.x);
-        v.y = finite_or_plain(p, t, n + 1, v.y);
-        v.z = finite_or_plain(p, t, n + 2, v.z);
-        v.w = finite_or_plain(p, t, n + 3, v.w);
+    } else {
+      for (int q = 0; q < p.splits; ++q) {
+        v.x += __ldcg(src + q * plane);
+        if (count > 1) v.y += __ldcg(src + q * plane + 1);
+        if (count > 2) v.z += __ldcg(src + q * plane + 2);
+        if (count > 3) v.w += __ldcg(src + q * plane + 3);
       }
-      if (p.add) v = make_float4(r.x + v.x, r.y + v.y, r.z + v.z, r.w + v.w);
+      if (p.add && mine) {
+        r.x = o[0];
+        if (count > 1) r.y = o[1];
+        if (count > 2) r.z = o[2];
+        if (count > 3) r.w = o[3];
+      }
+    }
+    const unsigned bad = !mine ? 0u : (unsigned)!isfinite(v.x) | (unsigned)!isfinite(v.y) << 1 | (unsigned)!isfinite(v.z) << 2 | (unsigned)!isfinite(v.w) << 3;
+    v = make_float4(v.x * GS_DOWN, v.y * GS_DOWN, v.z * GS_DOWN, v.w * GS_DOWN);
+    if (__any_sync(0xffffffffu, bad != 0)) v = plain_quads(p, t, n, count, bad, v);
+    if (!mine) continue;
+    if (p.add) v = make_float4(r.x + v.x, r.y + v.y, r.z + v.z, r.w + v.w);
+    if (vec) {
       *reinterpret_cast<float4*>(o) = v;
       continue;
     }
-    for (int c = 0; c < 4 && n + c < p.N; ++c) {
-      float v = __ldcg(src + c);
-      for (int q = 1; q < p.splits; ++q) v += __ldcg(src + q * plane + c);
-      v = finite_or_plain(p, t, n + c, v);
-      o[c] = p.add ? o[c] + v : v;
-    }
+    o[0] = v.x;
+    if (count > 1) o[1] = v.y;
+    if (count > 2) o[2] = v.z;
+    if (count > 3) o[3] = v.w;
   }
 }
 
@@ -433,11 +528,9 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
       asm volatile("bar.sync 1, 128;" ::: "memory");      // the four warps agree on going on
       if (ep_stop) break;
       if (p.splits == 1) {
-        if (n < p.N) {
 #pragma unroll
-          for (int c0 = 0; c0 < GS_TILE_T; c0 += 16)
-            if (c0 < valid) finish16(p, t0 + c0, n, min(16, valid - c0), &sum[c0]);
-        }
+        for (int c0 = 0; c0 < GS_TILE_T; c0 += 16)
+          if (c0 < valid) finish16(p, t0 + c0, n, min(16, valid - c0), &sum[c0]);
         continue;
       }
       // a range of K of the tile: to the workspace [range][token][feature], for split_sum_kernel

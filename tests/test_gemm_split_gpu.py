@@ -67,7 +67,7 @@ def test_gemm_split_one_sign(ops, K, kind):
 
 
 def test_gemm_split_values(ops):
-    """Large and small magnitudes keep their relative error; what is not finite comes out as the CUDA cores' kernel gives it."""
+    """Large and small magnitudes keep their relative error."""
     g = torch.Generator(device="cuda").manual_seed(5)
     x = torch.randn(70, 1024, device="cuda", generator=g) * 1e18
     w = torch.randn(256, 1024, device="cuda", generator=g) * 1e-22
@@ -79,22 +79,37 @@ def test_gemm_split_values(ops):
         a, b = (x.double() * (up * 1e-18)).float(), (w.double() * (down * 1e22)).float()
         ref = a.double() @ b.double().T
         assert ((run(ops, a, b).double() - ref).abs() <= (a.double().abs() @ b.double().abs().T) * 2.0 ** -18 + 2.0 ** -150).all(), (up, down)
-    x = torch.randn(70, 1024, device="cuda", generator=g)
-    w = torch.randn(256, 1024, device="cuda", generator=g)
-    x[3, 17], x[9, 1000], x[20, 5], x[20, 6] = float("inf"), float("-inf"), float("nan"), 2.0
-    w[100, 40], w[7, 900] = float("inf"), torch.tensor(0x7F800001, dtype=torch.int32).view(torch.float32).item()
+
+
+# One range of K and several; features that end inside a quad, a warp's eight and a tile; more tokens than a tile.
+@pytest.mark.parametrize("M,N,K", [(70, 256, 1024), (70, 250, 1032), (70, 1001, 512), (140, 9500, 1024), (65, 128, 8)])
+@pytest.mark.parametrize("add", [False, True])
+def test_gemm_split_not_finite(ops, M, N, K, add):
+    """What is not finite comes out as the CUDA cores' kernel gives it: single elements, whole rows of tokens and of weights, sums that
+    overflow."""
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    x, w = torch.randn(M, K, device="cuda", generator=g), torch.randn(N, K, device="cuda", generator=g)
+    inf, nan = float("inf"), float("nan")
+    x[3, K // 3], x[9, K - 1], x[20, 5], x[20, 6] = inf, -inf, nan, 2.0
+    w[100, K // 2], w[7, K - 4], w[N - 1, 0] = inf, torch.tensor(0x7F800001, dtype=torch.int32).view(torch.float32).item(), -inf
     w[50, 3] = 3.4e38
     x[30] = 0.0
     x[31, 3] = 3.4e38
     w[60] = 0.0
-    got, want = run(ops, x, w), torch.empty(70, 256, device="cuda")
-    ops.gemm_generic(x, w, want, ops.EPI_STORE_F32)
+    x[40], x[41], x[42], w[70], w[71] = nan, inf, -inf, nan, inf
+    x[43, ::2], x[43, 1::2] = inf, 1.0
+    x[44] = x[44].abs() * 1e36      # (overflows with w[72] only, in whatever order the terms are added)
+    w[72] = w[72].abs() * 1e4
+    x[M - 1, 0] = nan
+    start = torch.randn(M, N, device="cuda", generator=g) if add else None
+    got, want = run(ops, x, w, add=start), start.clone() if add else torch.empty(M, N, device="cuda")
+    ops.gemm_generic(x, w, want, ops.EPI_RESIDUAL if add else ops.EPI_STORE_F32)
     assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.isinf())
     inf = want.isinf()
     assert torch.equal(got[inf], want[inf])
     fine = want.isfinite()
     scale = x.nan_to_num(0, 0, 0).double().abs() @ w.nan_to_num(0, 0, 0).double().abs().T
-    assert ((got - want).abs()[fine].double() <= 2.0 ** -14 * scale[fine]).all()
+    assert ((got - want).abs()[fine].double() <= 2.0 ** -14 * scale[fine] + 2.0 ** -22).all()
 
 
 def test_gemm_split_linear(ops):
