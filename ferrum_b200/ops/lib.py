@@ -8,6 +8,7 @@ from __future__ import annotations
 
 import ctypes
 import functools
+import operator
 import os
 import threading
 from ctypes import c_float, c_int, c_longlong, c_void_p
@@ -29,6 +30,19 @@ _lock = threading.Lock()
 ABI = 23
 
 
+class _Entry(ctypes._CFuncPtr):
+    """An entry point.  The wrappers below hand sizes over as they come, which ctypes takes for plain integers only; a call with
+    another kind of integer (a numpy scalar, say) is made again with plain ones.  (Nothing has run before: ctypes converts first.)"""
+    _flags_ = ctypes._FUNCFLAG_CDECL
+    _restype_ = c_int
+
+    def __call__(self, *args):
+        try:
+            return super().__call__(*args)
+        except ctypes.ArgumentError:
+            return super().__call__(*[a if a is None or isinstance(a, (ctypes._SimpleCData, ctypes.Array)) else operator.index(a) for a in args])
+
+
 def lib():
     global _lib
     if _lib is None:
@@ -37,6 +51,7 @@ def lib():
                 path = build.build_kernels()
                 try:
                     handle = ctypes.CDLL(path)
+                    handle._FuncPtr = _Entry
                 except OSError as e:
                     raise KernelError(f"cannot load the kernel library {path}: {e}") from None
                 handle.ferrum_last_error.restype = ctypes.c_char_p
