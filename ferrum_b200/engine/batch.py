@@ -45,18 +45,21 @@ class Scratch:
         self._bufs: Dict[str, torch.Tensor] = {}
         self._views: Dict[str, tuple] = {}     # name -> (shape, dtype, view): the last view handed out (a step asks for the same one in every layer)
         self._guards: Dict[str, torch.Tensor] = {}
-        self.generation = 0      # bumped whenever a buffer is (re)allocated and so may have moved
+        self.generation = 0      # bumped whenever a buffer that a captured step may read is (re)allocated and so may have moved
         self.guard = int(os.environ.get("FERRUM_CANARY", "0") == "1") * 64 if guard is None else int(guard)
 
-    def get(self, name, shape, dtype):
+    def get(self, name, shape, dtype, limit=0, captured=True):
+        """A buffer of this shape.  limit: the elements that it may come to have; given, a buffer that has to grow grows to twice
+        its size, up to the limit (for sizes that follow a prompt portion by portion).  captured=False: no captured step reads it,
+        so that its moves leave `generation` alone."""
         last = self._views.get(name)
         if last is not None and last[0] == shape and last[1] is dtype:
             return last[2]
-        view = self._get(name, shape, dtype)
+        view = self._get(name, shape, dtype, limit, captured)
         self._views[name] = (shape, dtype, view)
         return view
 
-    def _get(self, name, shape, dtype):
+    def _get(self, name, shape, dtype, limit, captured):
         n = 1
         for s in shape:
             n *= int(s)
@@ -70,12 +73,13 @@ class Scratch:
                 words.fill_(CANARY)
                 t = raw[:max(n, 1) * esize].view(dtype)
                 self._bufs[name], self._guards[name] = t, words
-                self.generation += 1
+                self.generation += captured
             return t[:n].view(*shape)
         if t is None or t.dtype != dtype or t.numel() < n:
-            t = torch.empty(max(n, 1), dtype=dtype, device=self.device)
+            spare = min(2 * t.numel(), limit) if t is not None and t.dtype == dtype else 0
+            t = torch.empty(max(n, spare, 1), dtype=dtype, device=self.device)
             self._bufs[name] = t
-            self.generation += 1
+            self.generation += captured
         return t[:n].view(*shape)
 
     def check(self):
@@ -122,14 +126,14 @@ class PlanStore:
         self._bufs = {}
         self.generation = 0
 
-    def buffers(self, key, n):
-        """(PinnedRing, int32 device buffer) of at least n elements for `key`."""
+    def buffers(self, key, n, captured=True):
+        """(PinnedRing, int32 device buffer) of at least n elements for `key`; captured as in `Scratch.get`."""
         b = self._bufs.get(key)
         if b is None or b[1].numel() < n:
             cap = max(1024, 2 * n)
             b = (PinnedRing(cap, torch.int32, self.device), torch.empty(cap, dtype=torch.int32, device=self.device))
             self._bufs[key] = b
-            self.generation += 1
+            self.generation += captured
         return b
 
 
@@ -347,8 +351,8 @@ class StepContext:
         self.pending_experts = None
 
     # ------------------------------------------------------------------ scratch
-    def buf(self, name, shape, dtype):
-        return self.scratch.get(name, shape, dtype)
+    def buf(self, name, shape, dtype, limit=0, captured=True):
+        return self.scratch.get(name, shape, dtype, limit, captured)
 
     def gemm_scratch(self, M, N, K, dual):
         """(float32 workspace, zeroed int32 tile counters) for the tensor-core product."""
@@ -360,11 +364,11 @@ class StepContext:
         return self.scratch.get("gemm_partials_side" if self.lane else "gemm_partials", (floats,), torch.float32), getattr(self, name)
 
     def gemm_split_scratch(self, M, N, K):
-        """(tokens' parts, partial sums) for the float32 product on the tensor cores."""
-        parts, partials = ops.gemm_split_workspace(M, N, K)
+        """(tokens' parts, partial sums) for the float32 product on the tensor cores; both grow with the step's tokens."""
+        (parts, partials), (all_parts, all_partials) = ops.gemm_split_workspace(M, N, K), ops.gemm_split_workspace(self.max_tokens, N, K)
         lane = "_side" if self.lane else ""
-        return (self.scratch.get("gemm_split_parts" + lane, (parts,), torch.float32),
-                self.scratch.get("gemm_split_partials" + lane, (partials,), torch.float32))
+        return (self.scratch.get("gemm_split_parts" + lane, (parts,), torch.float32, all_parts),
+                self.scratch.get("gemm_split_partials" + lane, (partials,), torch.float32, all_partials))
 
     def side_stream(self):
         """A second CUDA stream with a fork and a join event, made at first use: (stream, fork, join)."""

@@ -35,12 +35,15 @@ SPLIT_BELOW = 4
 MAX_SPLITS = 1024       # what the merge kernel folds per (token, head)
 
 # Prompt portions write their requests' keys and values out (a product of the cached rows with U_k and U_v) and attend to
-# those on the tcgen05 kernel: (128 + 64 + 128) products a (query, key) pair and head instead of the (512 + 64 + 512) on the
-# cached rows, for 2 * 256 * 512 a key and head.  That pays where a key meets EXPAND_MIN_QUERIES queries of the step or
-# more on average (B200, a prompt step of four layers of 16 heads, us, cached rows -> written out: 256 tokens 975 -> 984, 400
-# 1001 -> 993, 700 1331 -> 1019, 1500 2691 -> 1373, 2048 3903 -> 1684).  The rows of EXPAND_MAX_KEYS keys are as much scratch as
-# a step may take (306 MB with 16 heads).
-EXPAND_MIN_QUERIES, EXPAND_MAX_KEYS = 192, 32768
+# those on the tcgen05 kernel: (128 + 64 + 128) products a (query, key) pair and head instead of the (kv_rank + 64 + kv_rank) on
+# the cached rows, for 2 * 256 * kv_rank a key and head.  That pays where a key meets EXPAND_MIN_QUERIES queries of the step or
+# more on average (B200, a prompt step of four layers of 16 heads, rank 512, us, cached rows -> written out: 256 tokens 975 -> 984, 400
+# 1001 -> 993, 700 1331 -> 1019, 1500 2691 -> 1373, 2048 3903 -> 1684: below it is the launches that count).  The tcgen05 kernel is so
+# much the quicker that kv_rank has no say: a layer's time on the GPU, 16 heads, 400 tokens, rank 64 / 128 / 256 / 512: 85 -> 64, 92 ->
+# 64, 95 -> 66, 119 -> 68; 1,024 tokens after 4,096: 574 -> 172, 648 -> 173, 962 -> 177, 1346 -> 181; 4 heads, 400 tokens, rank 64 75 -> 57;
+# 128 heads 216 -> 159; a window of 128 keys 71 -> 63.  What limits it is scratch: EXPAND_MAX_KEYS keys (306 MB with 16 heads of rank
+# 512) and EXPAND_MAX_BYTES (16,101 keys with 128 of them).
+EXPAND_MIN_QUERIES, EXPAND_MAX_KEYS, EXPAND_MAX_BYTES = 192, 32768, 1 << 30
 
 
 def rows_plan(q_len, pos0, window):
@@ -176,12 +179,17 @@ class LatentAttention(Mixer):
         linear(ov, self.w_o_weight, residual, RESIDUAL if accumulate else STORE_F32, ctx, M=ctx.n_tokens)
         return None
 
+    def _row_elements(self):
+        """Scratch of one key that is written out."""
+        return self.Dk + self.H * (self.Dn + self.Dv)
+
     def _expand_plan(self, ctx):
-        """Where this step's keys and values are written out: (keys, start, first, key_row, work, items), the same for every layer
-        with this window; None where attention runs on the cached rows."""
+        """Where this step's keys and values are written out: (keys, keys at most, start, first, key_row, work, items), the same for every
+        layer with this window and size; None where attention runs on the cached rows."""
         if self.w_ukv is None or ctx.max_q_len < EXPAND_MIN_QUERIES or ctx.fixed_shapes:
             return None
-        key = ("latent rows", self.window)
+        max_keys = min(EXPAND_MAX_KEYS, EXPAND_MAX_BYTES // (2 * self._row_elements()))
+        key = ("latent rows", self.window, max_keys)
         if key in ctx.step_cache:
             return ctx.step_cache[key]
         import numpy as np
@@ -189,24 +197,25 @@ class LatentAttention(Mixer):
         n_keys = int(start[-1])
         seen = sum(n * min(p + (n + 1) // 2, self.window if self.window > 0 else p + n) for p, n in zip(ctx.h_pos0, ctx.h_q_len))
         plan = None
-        if n_keys <= EXPAND_MAX_KEYS and seen >= EXPAND_MIN_QUERIES * n_keys:
+        if n_keys <= max_keys and seen >= EXPAND_MIN_QUERIES * n_keys:
             R = len(ctx.h_q_len)
             items = attention_plan.whole_items(ctx.h_q_len, ctx.h_pos0, self.window, 256)
             host = np.concatenate([start, first, start[:-1] - first, items.reshape(-1)]).astype(np.int32)
-            ring, dev = ctx.plan_store.buffers(key, host.size)
+            ring, dev = ctx.plan_store.buffers(key, host.size, captured=False)
             ring.next().numpy()[:host.size] = host
             dev[:host.size].copy_(ring.bufs[ring.i][:host.size], non_blocking=True)
             ring.sent()
             ctx.h2d_bytes += host.size * 4
-            plan = (n_keys, dev[:R + 1], dev[R + 1:2 * R + 1], dev[2 * R + 1:3 * R + 1], dev[3 * R + 1:host.size], items.shape[0])
+            plan = (n_keys, max_keys, dev[:R + 1], dev[R + 1:2 * R + 1], dev[2 * R + 1:3 * R + 1], dev[3 * R + 1:host.size], items.shape[0])
         ctx.step_cache[key] = plan
         return plan
 
     def _expanded(self, q, ov, gate, plan, ctx, cache, table):
-        n_keys, start, first, key_row, work, n_work = plan
+        n_keys, max_keys, start, first, key_row, work, n_work = plan
         T, H, R = ctx.n_tokens, self.H, self.R
-        rows = ctx.buf("lat_rows", (n_keys, self.Dk), self.dtype)
-        kv = ctx.buf("lat_kv", (n_keys, H * (self.Dn + self.Dv)), self.dtype)
+        # (the keys grow with every portion of a prompt, and no captured step comes here)
+        rows = ctx.buf("lat_rows", (n_keys, self.Dk), self.dtype, limit=max_keys * self.Dk, captured=False)
+        kv = ctx.buf("lat_kv", (n_keys, H * (self.Dn + self.Dv)), self.dtype, limit=max_keys * H * (self.Dn + self.Dv), captured=False)
         ops.latent_gather(cache.plane, cache.page_stride, cache.page_size, table, start, first, ctx.pos0, self.window, n_keys, self.Dk, rows, ctx.err)
         linear(rows[:, :R], self.w_ukv, kv, STORE, ctx, M=n_keys)
         ops.latent_q_rope_own(q, T, ctx.positions, self.rotary, H, self.Dn, self.Rr, ctx.err)

@@ -148,3 +148,44 @@ def test_latent_rows(td, case, monkeypatch):
                 error.setdefault(limit, []).append(((out - ref).norm() / ref.norm()).item())
         assert (len(calls) > before) == (limit == 8)
     assert sum(error[8]) <= 1.1 * sum(error[1 << 30])          # no less precise than on the cached rows
+
+
+@pytest.mark.gpu
+def test_portions_leave_captured_steps_alone(monkeypatch):
+    """The keys that are written out grow with every portion of a prompt; no buffer that a captured step reads moves with them.
+    And where the scratch of the keys would be too much, attention runs on the cached rows."""
+    from ferrum_b200.cache import CacheStorage
+    from ferrum_b200.engine.batch import StepContext, StepEntry
+    from ferrum_b200.ops import lib as ops
+    from ferrum_b200.parts import LatentAttention, latent_attention
+    ops.require_cuda()
+    td, E, H, R = torch.bfloat16, 256, 2, 64
+    mixer = LatentAttention(E, H, 128, 64, 128, R, 96, 1e-5, 192 ** -0.5, td)
+    g = torch.Generator(device="cuda").manual_seed(1)
+    for name, p in mixer.param_specs().items():
+        mixer.assign(name, torch.randn(p.shape, device="cuda", generator=g).mul_(p.shape[-1] ** -0.5).to(td if p.kind == "matrix" else torch.float32))
+    mixer.finalize()
+    cache = CacheStorage(Mixers([mixer]), td, "cuda", page_size=16, max_tokens=4096, max_requests=4, max_model_len=4096)
+    calls = []
+    real = ops.attention_rows
+    monkeypatch.setattr(ops, "attention_rows", lambda *a, **k: (calls.append(a[4]), real(*a, **k))[1])
+
+    def prompt(ctx):
+        slot, seen = cache.open(), []
+        x, y = torch.randn(256, E, device="cuda", generator=g).to(td), torch.empty(256, E, device="cuda")
+        for at in range(0, 2048, 256):
+            cache.manager.grow(slot, at + 256)
+            ctx.fill([StepEntry(slot, at, [0] * 256)], cache.manager)
+            mixer.forward(x, ctx, cache.layer_cache(0), y, accumulate=False)
+            cache.manager.commit(slot, at + 256)
+            seen.append(ctx.buffers_generation())
+        assert ctx.err.item() == 0
+        cache.close(slot)
+        return seen
+    monkeypatch.setattr(latent_attention, "EXPAND_MIN_QUERIES", 64)
+    seen = prompt(StepContext("cuda", 256, 4, [cache.table_width]))
+    assert calls == list(range(256, 2049, 256)) and len(set(seen)) == 1
+    calls.clear()
+    monkeypatch.setattr(latent_attention, "EXPAND_MAX_BYTES", 1100 * 2 * (R + 64 + H * 256))
+    prompt(StepContext("cuda", 256, 4, [cache.table_width]))
+    assert calls == [256, 512, 768, 1024]
