@@ -71,4 +71,10 @@ def test_pair_tiles(M, N, K, ctas, dual, bt, cut, h16):
         acc = res.clone()
         ops.gemm_tc(x, w, acc, ops.TC_RESIDUAL, err, ws, cnt, n_ctas=ctas)
         assert ((acc.double() - res.double() - ref).abs() <= absref + 2.0 ** -23 * acc.double().abs()).all()
+        # float32 results, through the tensor map where rows are 16-byte multiples and by the threads where not: the same bits
+        plain = [torch.full((M, N + pad), float("nan"), device="cuda") for pad in (4, 1)]
+        for out in plain:
+            ops.gemm_tc(x, w, out, ops.TC_STORE_F32, err, ws, cnt, n_ctas=ctas)
+            assert out[:, N:].isnan().all()
+        assert ((plain[0][:, :N].double() - ref).abs() <= absref).all() and torch.equal(plain[0][:, :N], plain[1][:, :N])
     assert err.item() == 0 and cnt.abs().sum().item() == 0
