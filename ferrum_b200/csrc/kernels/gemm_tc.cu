@@ -1217,6 +1217,17 @@ static PairPlan pair_plan(int M, long long rows, int K, int pairs) {
   return best;
 }
 
+// The plan and the pairs that run it: no more than there are units (tile, k-block).
+struct PairLaunch {
+  PairPlan plan;
+  int pairs;
+};
+static PairLaunch pair_launch(int M, long long rows, int K, int pairs) {
+  const PairPlan plan = pair_plan(M, rows, K, pairs);
+  const long long units = (rows + 2 * TILE_N - 1) / (2 * TILE_N) * plan.tiles_t * ((K + TILE_K - 1) / TILE_K);
+  return PairLaunch{plan, (int)std::min<long long>(pairs, units)};
+}
+
 // The token-tile width the kernel uses for M tokens.
 FERRUM_API int ferrum_gemm_tc_token_tile(int M, int dual) {
   if (M <= 16) return 16;
@@ -1306,12 +1317,10 @@ FERRUM_API int ferrum_gemm_tc(const void* x, const void* w, void* out, int dtype
     p.N = 2 * N;
     p.gated = 1;
     p.stream_weights = 0;
-    const PairPlan plan = pair_plan(M, p.N, K, asked_ctas / 2);
+    const PairLaunch run = pair_launch(M, p.N, K, asked_ctas / 2);
+    const PairPlan& plan = run.plan;
     p.bt = plan.bt;
     p.cut = plan.cut;
-    const long long units = (long long)((p.N + 2 * TILE_N - 1) / (2 * TILE_N)) * plan.tiles_t * ((K + TILE_K - 1) / TILE_K);
-    int pairs = asked_ctas / 2;
-    if (pairs > units) pairs = (int)units;
     CUtensorMap mo, ms;
     if (int r = get_tensor_map(w, N, K, ldw, dual_offset, &mw, 4)) return r;
     if (int r = get_tensor_map(x, M, K, ldx, plan.bt / 2, &mx)) return r;
@@ -1319,17 +1328,15 @@ FERRUM_API int ferrum_gemm_tc(const void* x, const void* w, void* out, int dtype
     FERRUM_CHECK_ARG(((uintptr_t)workspace & 15) == 0, "gemm_tc: the workspace must be 16-byte aligned");
     if (int r = get_tensor_map(workspace, workspace_floats / TILE_N, TILE_N, TILE_N, PAIR_OUT_ROWS, &ms, 1)) return r;
     p.out_tma = 1;
-    return launch_tc_pair(mw, mx, mo, ms, p, 2 * pairs, stream);
+    return launch_tc_pair(mw, mx, mo, ms, p, 2 * run.pairs, stream);
   }
   if (int r = get_tensor_map(w, w_rows, K, ldw, TILE_N, &mw)) return r;
   if (M >= PAIR_MIN_TOKENS && !dual && use_pair && n_ctas >= 2) {
-    // many tokens: pairs of CTAs on 256 x 256 tiles; each CTA stages 128 tokens
-    const PairPlan plan = pair_plan(M, N, K, asked_ctas / 2);
+    // many tokens: pairs of CTAs on tiles of 256 rows x 64 to 256 tokens (`pair_plan`); each CTA stages half of both
+    const PairLaunch run = pair_launch(M, N, K, asked_ctas / 2);
+    const PairPlan& plan = run.plan;
     p.bt = plan.bt;
     p.cut = plan.cut;
-    const long long units = (long long)((N + 2 * TILE_N - 1) / (2 * TILE_N)) * plan.tiles_t * ((K + TILE_K - 1) / TILE_K);
-    int pairs = asked_ctas / 2;
-    if (pairs > units) pairs = (int)units;
     if (int r = get_tensor_map(x, M, K, ldx, plan.bt / 2, &mx)) return r;
     // the output through a tensor map where its rows are 16-byte multiples; else by the threads
     CUtensorMap mo = mw;
@@ -1344,7 +1351,7 @@ FERRUM_API int ferrum_gemm_tc(const void* x, const void* w, void* out, int dtype
       FERRUM_CHECK_ARG(((uintptr_t)workspace & 15) == 0, "gemm_tc: the workspace must be 16-byte aligned");
       if (int r = get_tensor_map(workspace, workspace_floats / TILE_N, TILE_N, TILE_N, PAIR_OUT_ROWS, &ms, 1)) return r;
     }
-    return launch_tc_pair(mw, mx, mo, ms, p, 2 * pairs, stream);
+    return launch_tc_pair(mw, mx, mo, ms, p, 2 * run.pairs, stream);
   }
   if (int r = get_tensor_map(x, M, K, ldx, bt, &mx)) return r;
 #define TC_CASE(BT_)                                                         \
@@ -1370,6 +1377,23 @@ FERRUM_API void ferrum_gemm_pair_plan(int M, long long rows, int K, int pairs, i
   out[2] = plan.cut;
 }
 
+static int schedule_segment(const PairSchedule& sched, int cluster, int s, long long* out) {
+  long long tile;
+  int kb0, kb1, n_idx, t_idx;
+  if (!sched.segment(s, tile, kb0, kb1)) return 0;
+  sched.coords(tile, n_idx, t_idx);
+  const bool whole = kb0 == 0 && kb1 == sched.nkb;
+  out[0] = tile;
+  out[1] = kb0;
+  out[2] = kb1;
+  out[3] = n_idx;
+  out[4] = t_idx;
+  out[5] = whole ? -1 : sched.first_owner(tile);
+  out[6] = whole ? -1 : sched.last_owner(tile);
+  out[7] = whole ? -1 : sched.slot_of(cluster, tile);
+  return 1;
+}
+
 // For tests of the schedule on the host: pair `cluster`'s s-th segment when `pairs` pairs
 // compute M tokens x `rows` weight rows (for gate and up as one product: both) over K in tiles of 256 tokens.
 // out[0..7] = tile, first k-block, one past the last, weight tile index, token tile index, and
@@ -1380,21 +1404,18 @@ FERRUM_API int ferrum_gemm_pair_schedule(int M, long long rows, int K, int pairs
   const int tiles_n = (int)((rows + 2 * TILE_N - 1) / (2 * TILE_N)), tiles_t = (M + PAIR_BT - 1) / PAIR_BT;
   bool cut;
   pair_cost((long long)tiles_n * tiles_t, nkb, pairs, PAIR_BT, &cut);
-  const PairSchedule sched(tiles_n, tiles_t, nkb, pairs, cluster, cut);
-  long long tile;
-  int kb0, kb1, n_idx, t_idx;
-  if (!sched.segment(s, tile, kb0, kb1)) return 0;
-  sched.coords(tile, n_idx, t_idx);
-  const bool whole = kb0 == 0 && kb1 == nkb;
-  out[0] = tile;
-  out[1] = kb0;
-  out[2] = kb1;
-  out[3] = n_idx;
-  out[4] = t_idx;
-  out[5] = whole ? -1 : sched.first_owner(tile);
-  out[6] = whole ? -1 : sched.last_owner(tile);
-  out[7] = whole ? -1 : sched.slot_of(cluster, tile);
-  return 1;
+  return schedule_segment(PairSchedule(tiles_n, tiles_t, nkb, pairs, cluster, cut), cluster, s, out);
+}
+
+// The same as a launch for `pairs` pairs runs it: with the widths, the cut and the number of pairs of `pair_launch`.
+// out[8..10] = tokens per tile, token tiles, pairs that run (also where the pair has no such segment).
+FERRUM_API int ferrum_gemm_pair_launch_schedule(int M, long long rows, int K, int pairs, int cluster, int s, long long* out) {
+  const PairLaunch run = pair_launch(M, rows, K, pairs);
+  out[8] = run.plan.bt;
+  out[9] = run.plan.tiles_t;
+  out[10] = run.pairs;
+  const int tiles_n = (int)((rows + 2 * TILE_N - 1) / (2 * TILE_N));
+  return schedule_segment(PairSchedule(tiles_n, run.plan.tiles_t, (K + TILE_K - 1) / TILE_K, run.pairs, cluster, run.plan.cut), cluster, s, out);
 }
 
 // ------------------------------------------------------------------ deferred reduction

@@ -34,9 +34,30 @@ def schedule():
     return segments
 
 
-def check(schedule, M, rows, K, pairs):
+@pytest.fixture(scope="module")
+def launch():
+    """(tokens per tile, token tiles, pairs that run, their segments) of a launch for so many pairs."""
+    from ferrum_b200.ops import lib as ops
+    fn = ops.lib().ferrum_gemm_pair_launch_schedule
+    out = (ctypes.c_longlong * 11)()
+
+    def run(M, rows, K, pairs):
+        args = ctypes.c_int(M), ctypes.c_longlong(rows), ctypes.c_int(K), ctypes.c_int(pairs)
+        fn(*args, ctypes.c_int(0), ctypes.c_int(0), out)
+        bt, tiles_t, runs = out[8:]
+        segs = {}
+        for c in range(runs):
+            segs[c] = []
+            while fn(*args, ctypes.c_int(c), ctypes.c_int(len(segs[c])), out):
+                segs[c].append(tuple(out[:8]))
+                assert len(segs[c]) < 100000
+        return bt, tiles_t, runs, segs
+    return run
+
+
+def check(schedule, M, rows, K, pairs, tiles_t=None):
     nkb = (K + 63) // 64
-    tiles_n, tiles_t = (rows + 255) // 256, (M + 255) // 256
+    tiles_n, tiles_t = (rows + 255) // 256, tiles_t or (M + 255) // 256
     done = {}
     coords = {}
     sharers = {}
@@ -91,3 +112,38 @@ def test_random_shapes(schedule):
         rows = rng.randint(1, 40) * rng.choice((64, 200, 256))
         K = rng.choice((64, 320, 4096, 8192, 14336, 20000))
         check(schedule, M, rows, K, rng.randint(1, 74))
+
+
+def check_launch(launch, M, rows, K, pairs):
+    from ferrum_b200.ops import lib as ops
+    bt, tiles_t, runs, segs = launch(M, rows, K, pairs)
+    assert 64 <= bt <= 256 and bt % 32 == 0 and (tiles_t - 1) * bt < M <= tiles_t * bt
+    assert runs == min(pairs, (rows + 255) // 256 * tiles_t * ((K + 63) // 64))
+    shared = check(lambda M, rows, K, pairs, c: segs[c], M, rows, K, runs, tiles_t)
+    if shared:      # the shared tiles' counters, two each, are there
+        n = ctypes.c_int()
+        ops.lib().ferrum_gemm_tc_workspace(ctypes.c_int(M), ctypes.c_int(rows), ctypes.c_int(K), ctypes.c_int(0), ctypes.c_int(2 * pairs), ctypes.byref(n))
+        assert 2 * max(tile for s in segs.values() for tile, *_, slot in s if slot >= 0) + 1 < n.value
+    return bt, shared > 0
+
+
+def test_launches(launch):
+    """What runs: the width of the token tiles and the cut as the launch chooses them, fewer units than pairs among them."""
+    rng = random.Random(11)
+    seen = set()
+    for i in range(700):
+        M = rng.randint(65, 512) if i % 2 else rng.randint(65, 3000)
+        rows = rng.randint(1, 40) * rng.choice((64, 200, 256))
+        K = rng.choice((64, 320, 4096, 8192, 14336, 20000))
+        seen.add(check_launch(launch, M, rows, K, rng.randint(1, 74)))
+    assert {bt for bt, _ in seen} == set(range(64, 257, 32))
+    assert {bt for bt, cut in seen if cut} == set(range(64, 257, 32))       # every width also with shared tiles
+    check_launch(launch, 65, 200, 64, 74)                                     # one unit
+    check_launch(launch, 100, 256, 64 * 30, 74)                               # fewer k-blocks than pairs
+
+
+def test_launches_of_models(launch):
+    """A Llama-3.1-8B layer's products at the sizes a server meets."""
+    for rows, K in ((6144, 4096), (4096, 4096), (28672, 4096), (4096, 14336)):
+        for M in (65, 80, 128, 129, 256, 300, 391, 512, 2048):
+            check_launch(launch, M, rows, K, 74)
