@@ -1128,7 +1128,7 @@ FERRUM_API void ferrum_gemm_tc_test_hooks(long long wait_cycles, int drop_loads)
   g_drop_loads = drop_loads != 0;
 }
 
-FERRUM_API int ferrum_gemm_tc_can_defer(int M, int N, int K, int dual, int n_ctas);
+FERRUM_API int ferrum_gemm_tc_should_defer(int M, int N, int K, int dual, int n_ctas);
 
 static bool g_pair_kernel = true;
 // The CTA-pair kernel can be switched off (every shape then runs on the single-CTA kernel).
@@ -1305,10 +1305,9 @@ FERRUM_API int ferrum_gemm_tc(const void* x, const void* w, void* out, int dtype
   p.glu_act = glu_act;
   p.glu_limit = glu_limit;
   p.store_act = store_act;
-  // (The test hook's dropped loads are the single-CTA kernel's.  A residual sum of up to 128 tokens that could be left in partials
+  // (The test hook's dropped loads are the single-CTA kernel's.  A residual sum that the layers would leave in partials
   // stays there too: whether it is left or added here, it is the same bits.)
-  const bool use_pair = g_pair_kernel && !g_drop_loads &&
-                        !(epilogue == TC_RESIDUAL && M <= TILE_N && ferrum_gemm_tc_can_defer(M, N, K, 0, asked_ctas));
+  const bool use_pair = g_pair_kernel && !g_drop_loads && !(epilogue == TC_RESIDUAL && ferrum_gemm_tc_should_defer(M, N, K, 0, asked_ctas));
   CUtensorMap mw, mx;
   if (dual && M >= PAIR_MIN_TOKENS && use_pair && n_ctas >= 2 && ((uintptr_t)out & 15) == 0 && ldo % 8 == 0) {
     // Two products of many tokens: the pair kernel computes them as one product whose weight
@@ -1425,8 +1424,6 @@ FERRUM_API int ferrum_gemm_pair_launch_schedule(int M, long long rows, int K, in
 // product (RMSNorm, the rotary kernel, ...) adds them while it reads, in K order, with
 // partial_sum() of partials.cuh.  Requirements: one token tile (M <= 256, or 128 for two
 // products) and at most one output tile per CTA, so that a CTA writes at most two partials.
-// With 65 to 256 tokens the in-kernel reduction is worse still: the last arriver of a tile
-// reads several 64 to 128 KB partials and read-modify-writes the output on its own.
 FERRUM_API int ferrum_gemm_tc_can_defer(int M, int N, int K, int dual, int n_ctas) {
   if (n_ctas <= 0) n_ctas = sm_count();
   const int bt = ferrum_gemm_tc_token_tile(M, dual);
@@ -1436,6 +1433,14 @@ FERRUM_API int ferrum_gemm_tc_can_defer(int M, int N, int K, int dual, int n_cta
   // at most 8 CTAs may share a tile (the consumers keep that many loads in flight per element)
   const long long per = units / n_ctas;
   return M > 0 && M <= bt && tiles <= n_ctas && per > 0 && ((K + TILE_K - 1) / TILE_K) / per + 2 <= 8;
+}
+
+// Whether the layers do: up to this many tokens the next kernel sums the partials for less than they save.  With more the
+// CTA-pair kernel, which writes whole tiles, is the quicker (B200, prompt steps of 160 and 256 tokens, Llama-3.2-3B 3.66 -> 3.26 ms and
+// 4.11 -> 3.62, Llama-2-7B 5.93 -> 5.26 and 6.77 -> 5.66; at 80 and 128 tokens 3.00 against 3.21 and 3.00 against 3.12 the other way).
+constexpr int DEFER_MAX_TOKENS = 128;
+FERRUM_API int ferrum_gemm_tc_should_defer(int M, int N, int K, int dual, int n_ctas) {
+  return M <= DEFER_MAX_TOKENS && ferrum_gemm_tc_can_defer(M, N, K, dual, n_ctas);
 }
 
 // layout[0..3] = k-blocks per tile, tiles, CTAs, columns per partial: what partial_sum() needs.

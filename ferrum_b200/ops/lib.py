@@ -27,7 +27,7 @@ TC_STORE_BF16, TC_STORE_F32, TC_RESIDUAL, TC_SWIGLU, TC_GEGLU, TC_SWISH_CLAMP, T
 
 _lib = None
 _lock = threading.Lock()
-ABI = 23
+ABI = 24
 
 
 class _Entry(ctypes._CFuncPtr):
@@ -413,6 +413,12 @@ def swiglu_reduce(act, n_tokens, F, partials):
 def gemm_tc_can_defer(M, N, K, dual):
     """(A pure function of the shape, asked for every product of every step: remembered.)"""
     return bool(lib().ferrum_gemm_tc_can_defer(c_int(M), c_int(N), c_int(K), c_int(1 if dual else 0), c_int(0)))
+
+
+@functools.lru_cache(maxsize=4096)
+def gemm_tc_should_defer(M, N, K, dual):
+    """Whether the layers leave such a product in partials: it can be, and the next kernel sums them for less than they save."""
+    return bool(lib().ferrum_gemm_tc_should_defer(c_int(M), c_int(N), c_int(K), c_int(1 if dual else 0), c_int(0)))
 
 
 def gemm_tc_deferred(x, w, err, workspace, M=None, N=None, dual_offset=0, n_ctas=0):

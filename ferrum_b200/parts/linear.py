@@ -15,11 +15,6 @@ STORE, STORE_F32, RESIDUAL = "store", "store_f32", "residual"
 _GENERIC = {STORE: ops.EPI_STORE, STORE_F32: ops.EPI_STORE_F32, RESIDUAL: ops.EPI_RESIDUAL}
 _TC = {STORE: ops.TC_STORE_BF16, STORE_F32: ops.TC_STORE_F32, RESIDUAL: ops.TC_RESIDUAL}
 
-# Products of up to this many tokens may stay in partials for the next kernel.  With more the CTA-pair kernel is quicker, its
-# tiles written out whole: B200, prompt steps of 160 and 256 tokens, Llama-3.2-3B 3.66 -> 3.26 ms and 4.11 -> 3.62, Llama-2-7B
-# 5.93 -> 5.26 and 6.77 -> 5.66; at 80 and 128 tokens 3.00 against 3.21 and 3.00 against 3.12 the other way.
-DEFER_MAX_TOKENS = 128
-
 
 def linear_deferred(x, w, ctx, M, N=None, dual_offset=0):
     """The product as float32 partials for the next kernel to sum (`ops.Partials`), or None
@@ -28,7 +23,7 @@ def linear_deferred(x, w, ctx, M, N=None, dual_offset=0):
     thin = N is None and not dual_offset
     N = (w.shape[0] - dual_offset) if N is None else N
     K = w.shape[1]
-    if M == 0 or M > DEFER_MAX_TOKENS or not ops.gemm_tc_can_defer(M, N, K, dual_offset > 0) or not ops.gemm_tc_supported(x, w) or (thin and ops.thin_linear_supported(x, w, M)):
+    if M == 0 or not ops.gemm_tc_should_defer(M, N, K, dual_offset > 0) or not ops.gemm_tc_supported(x, w) or (thin and ops.thin_linear_supported(x, w, M)):
         return None
     ctx.flush_residual()
     ws, _ = ctx.gemm_scratch(M, N, K, dual_offset > 0)

@@ -78,3 +78,24 @@ def test_pair_tiles(M, N, K, ctas, dual, bt, cut, h16):
             assert out[:, N:].isnan().all()
         assert ((plain[0][:, :N].double() - ref).abs() <= absref).all() and torch.equal(plain[0][:, :N], plain[1][:, :N])
     assert err.item() == 0 and cnt.abs().sum().item() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("h16", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M", [64, 65, 128, 129])
+@pytest.mark.parametrize("N,K", [(4096, 4096), (5000, 520), (3072, 8192)])
+def test_residual_left_or_added(M, N, K, h16):
+    """A residual sum that the layers leave in partials for the next kernel is the same bits where the product adds it itself."""
+    from ferrum_b200.ops import lib as ops
+    ops.require_cuda()
+    assert ops.gemm_tc_should_defer(M, N, K, False) == (M <= 128)
+    if M > 128:
+        return
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    x, w, h = torch.randn(M, K, device="cuda", generator=g).to(h16), torch.randn(N, K, device="cuda", generator=g).to(h16), torch.randn(M, N, device="cuda", generator=g)
+    floats, tiles = ops.gemm_tc_workspace(M, N, K, False)
+    ws, cnt, err = torch.empty(floats, device="cuda"), torch.zeros(tiles, dtype=torch.int32, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    left, added = h.clone(), h.clone()
+    ops.residual_reduce(left, M, ops.gemm_tc_deferred(x, w, err, ws))
+    ops.gemm_tc(x, w, added, ops.TC_RESIDUAL, err, ws, cnt)
+    assert err.item() == 0 and torch.equal(left, added)
