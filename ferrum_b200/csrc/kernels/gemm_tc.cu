@@ -666,10 +666,13 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             break;
           }
           tc_fence_after();
-          const uint32_t a_lo = (uint32_t)desc0 + (uint32_t)(s * (stage_bytes >> 4)), hi = (uint32_t)(desc0 >> 32);
+          const uint64_t a_desc = desc0 + (uint64_t)(s * (stage_bytes >> 4));
+          const uint64_t b_desc = a_desc + (A_BYTES >> 4);
 #pragma unroll
-          for (int kk = 0; kk < TILE_K / UMMA_K; ++kk)
-            umma_bf16_pair_lo(d0, a_lo + kk * 2, a_lo + (A_BYTES >> 4) + kk * 2, hi, idesc, !first || kk > 0);
+          for (int kk = 0; kk < TILE_K / UMMA_K; ++kk) {
+            const uint64_t adv = (uint64_t)(kk * UMMA_K * 2 >> 4);
+            umma_bf16_pair(d0, a_desc + adv, b_desc + adv, idesc, !first || kk > 0);
+          }
           first = false;
           umma_commit_pair(empty_bar(s), 3);  // both CTAs may refill the stage
           if (++s == STAGES) {

@@ -260,14 +260,6 @@ __device__ __forceinline__ void umma_bf16_pair(uint32_t d_tmem, uint64_t a_desc,
       "l"(a_desc), "l"(b_desc), "r"(idesc), "r"((uint32_t)accumulate)
       : "memory");
 }
-// The same with the descriptors' low words apart: their high words are the same for every stage.
-__device__ __forceinline__ void umma_bf16_pair_lo(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t hi, uint32_t idesc, bool accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\tsetp.ne.b32 p, %5, 0;\n\tmov.b64 a, {%1, %3};\n\tmov.b64 b, {%2, %3};\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], a, b, %4, p;\n\t}\n" ::"r"(d_tmem),
-      "r"(a_lo), "r"(b_lo), "r"(hi), "r"(idesc), "r"((uint32_t)accumulate)
-      : "memory");
-}
 // The same with the A operand in tensor memory: rows 0..127 of A in the leader's tensor memory,
 // rows 128..255 in its peer's, at the same column address in both.
 __device__ __forceinline__ void umma_16bit_pair_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, bool accumulate) {
