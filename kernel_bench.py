@@ -5,9 +5,10 @@ peaks.  This is the small case that `ncu` captures are taken on.
 
     python kernel_bench.py attn_decode [--batch 8] [--context 8192] [--layers 4]
     python kernel_bench.py attn_prefill [--tokens 2048]
-    python kernel_bench.py gemm --tokens 8 --n 6144 --k 4096 [--epilogue store|residual|swiglu|relu2] [--copies 8]
-    python kernel_bench.py gemm|attn_decode|attn_prefill ... --dtype fp32    (the CUDA-core kernels of the 32-bit path)
+    python kernel_bench.py gemm --tokens 8 --n 6144 --k 4096 [--epilogue store|float32|residual|swiglu|relu2] [--copies 8]
+    python kernel_bench.py gemm|attn_decode|attn_prefill ... --dtype fp32    (the 32-bit path; gemm: the kernel that a layer takes, or with --cuda-cores the CUDA cores' one)
     python kernel_bench.py latent_decode|latent_prefill [--hq 16] [--kv-rank 512] [--rot-dim 64] [--window W] [--cuda-cores]
+    python kernel_bench.py latent_rows --tokens 1500 [--hq 16] [--kv-rank 512] [--window W]   (keys and values written out: rows, product and attention)
     python kernel_bench.py head_linear --tokens 8 --hq 16 --n 512 --k 128
     python kernel_bench.py attn_decode|attn_prefill --exact [--window W] [--penalty]   (float32 weights and sums on 16-bit storage)
     python kernel_bench.py ssm --tokens 2048 [--batch 1] [--hq 64] [--head-dim 64] [--state 128]   (the state-space mixer's kernels)
@@ -41,7 +42,7 @@ sys.path.insert(0, ROOT)
 
 def main():
     ap = argparse.ArgumentParser()
-    ap.add_argument("kernel", choices=["attn_decode", "attn_prefill", "latent_decode", "latent_prefill", "head_linear", "gemm", "moe", "streams", "rmsnorm", "dyn_tanh",
+    ap.add_argument("kernel", choices=["attn_decode", "attn_prefill", "latent_decode", "latent_prefill", "latent_rows", "head_linear", "gemm", "moe", "streams", "rmsnorm", "dyn_tanh",
                                        "rope", "ssm", "delta", "memory", "cdecay", "step", "timeline"])
     ap.add_argument("--bonus", action="store_true", help="cdecay: the read-out before the write, with a bonus for the current token")
     ap.add_argument("--segment", type=int, default=-1, help="cdecay: tokens per segment (0: one piece; -1: the library's choice)")
@@ -49,7 +50,7 @@ def main():
     ap.add_argument("--rot-dim", type=int, default=64, help="latent_*: rotated key elements behind the latent")
     ap.add_argument("--window", type=int, default=0, help="latent_*: keys a query looks back over (0: all)")
     ap.add_argument("--stage", type=int, default=0, choices=[0, 32, 64], help="latent_*: force the tensor-core kernel's stage size")
-    ap.add_argument("--cuda-cores", action="store_true", help="latent_*: the CUDA-core kernel also where the tensor-core one applies")
+    ap.add_argument("--cuda-cores", action="store_true", help="latent_*, gemm --dtype fp32: the CUDA-core kernel also where the tensor-core one applies")
     ap.add_argument("--exact", action="store_true", help="attn_*: the CUDA-core kernel with float32 results, as the shaped attention runs it")
     ap.add_argument("--penalty", action="store_true", help="attn_* --exact: with a distance penalty per head")
     ap.add_argument("--streams", type=int, default=4, help="streams: copies of the residual stream")
@@ -61,7 +62,7 @@ def main():
     ap.add_argument("--tokens", type=int, default=8)
     ap.add_argument("--n", type=int, default=6144)
     ap.add_argument("--k", type=int, default=4096)
-    ap.add_argument("--epilogue", default="store", choices=["store", "residual", "swiglu", "relu2"])
+    ap.add_argument("--epilogue", default="store", choices=["store", "float32", "residual", "swiglu", "relu2"])
     ap.add_argument("--wide", action="store_true", help="attn_*, latent_*: softmax weights kept to float32 precision on the tensor cores")
     ap.add_argument("--top", type=int, default=0, help="dyn_tanh: expert rows per token whose sum is made on the way")
     ap.add_argument("--ctas", type=int, default=0, help="gemm: CTAs of the grid (0 = one per SM)")
@@ -75,7 +76,7 @@ def main():
     ap.add_argument("--page-size", type=int, default=16)
     ap.add_argument("--deferred", action="store_true", help="gemm: leave the partials to the consumer (as decoding does)")
     ap.add_argument("--dtype", default="bf16", choices=["bf16", "fp16", "fp32"],
-                    help="fp32 times the CUDA-core kernels of the true 32-bit path (its fraction is of the FFMA peak)")
+                    help="fp32 times the kernels of the true 32-bit path (their fraction is of the FFMA peak, or of a sixth of the bf16 rate)")
     ap.add_argument("--attention-pair", choices=["on", "off"], default=None,
                     help="attn_prefill at head size 128: the kernel of two CTAs on one tile (on) or of one CTA (off)")
     ap.add_argument("--no-graph", action="store_true", help="launch from the host instead of replaying a CUDA graph")
@@ -231,6 +232,35 @@ def main():
         keys, pairs = ops.visible_keys(ctx, args.window)
         work = {"bytes": keys * Dk * esize + T * Hq * (Dk + Rk) * esize, "flops": 2.0 * pairs * Hq * (Dk + Rk),
                 "bound": "hbm" if decode else "tensor"}
+    elif args.kernel == "latent_rows":
+        # a prompt of --tokens tokens from position 0, --hq heads of 128 + 64 / 128 over rows of kv_rank + 64: the gathered rows, their
+        # product with U_k and U_v, the turned queries and the attention, as a layer runs them
+        from ferrum_b200.parts import LatentAttention, RotaryEmbedding, latent_attention
+        H, Rk, T = Hq, args.kv_rank, args.tokens
+        width = (T + ps - 1) // ps
+        rot = RotaryEmbedding(64, 64, 10000.0, None, "half", T, dev)
+        mixer = LatentAttention(64, H, 128, 64, 128, Rk, 64, 1e-6, 192 ** -0.5, td, rotary=rot, window=args.window, wide_weights=args.wide)
+        for name, spec in mixer.param_specs().items():
+            w = torch.randn(*spec.shape, device=dev, generator=gen)
+            mixer.assign(name, w.mul_(spec.shape[-1] ** -0.5).to(td) if spec.kind == "matrix" else w)
+        mixer.finalize()
+        ctx = StepContext(dev, max(16, T), 1, [width])
+        ctx.fill([StepEntry(0, 0, [1] * T)], [torch.randperm(width).view(1, width).tolist()])
+        table = ctx.block_tables[0]
+        q, ov = torch.randn(T, H * 192, device=dev, generator=gen).to(td), torch.empty(T, H * 128, device=dev, dtype=td)
+        gate = torch.rand(T, H, device=dev, generator=gen)
+        latent_attention.EXPAND_MIN_QUERIES = 0      # (written out at any length)
+        plan = mixer._expand_plan(ctx)
+
+        class Cache:
+            pass
+        for _ in range(args.layers):
+            c = Cache()
+            c.plane = torch.randn(width, ps, Rk + 64, device=dev, generator=gen).to(td)
+            c.page_stride, c.page_size = c.plane.stride(0), ps
+            runs.append(lambda c=c: mixer._expanded(q, ov, gate, plan, ctx, c, table))
+        pairs = ops.visible_keys(ctx, args.window)[1]
+        work = {"bytes": T * (Rk + 64) * 2 + H * 256 * Rk * 2 + T * H * 320 * 2, "flops": 2.0 * T * H * 256 * Rk + 2.0 * pairs * H * 320, "bound": "tensor"}
     elif args.kernel == "head_linear":
         # one small product per head: [tokens, n] = [tokens, k] x [n, k]^T for each of --hq heads
         M, N, K = args.tokens, args.n, args.k
@@ -248,13 +278,18 @@ def main():
         err = torch.zeros(1, dtype=torch.int32, device=dev)
         x = torch.randn(M, K, device=dev, generator=gen).to(td)
         weights = [torch.randn(N * (2 if dual else 1), K, device=dev, generator=gen).mul_(0.02).to(td) for _ in range(args.copies)]
-        if args.epilogue == "residual":
+        if args.epilogue in ("residual", "float32"):
             o = torch.zeros(M, N, device=dev)
-            epi = ops.TC_RESIDUAL
+            epi = ops.TC_RESIDUAL if args.epilogue == "residual" else ops.TC_STORE_F32
         else:
             o = torch.empty(M, N * (2 if dual and args.dtype == "fp32" else 1), device=dev, dtype=td)
             epi = ops.TC_SWIGLU if dual else (ops.TC_RELU2 if args.epilogue == "relu2" else ops.TC_STORE_BF16)
-        if args.dtype == "fp32":     # the CUDA-core product (gate and up as one product of 2N rows; the activation is a kernel of its own)
+        split = args.dtype == "fp32" and not args.cuda_cores and ops.gemm_split_supported(x, weights[0], M)
+        if split:                    # (gate and up as one product of 2N rows; the activation is a kernel of its own)
+            rows = weights[0].shape[0]
+            parts, partials = (torch.empty(n, device=dev) for n in ops.gemm_split_workspace(M, rows, K))
+            runs = [lambda w=w: ops.gemm_split(x, w, o, err, parts, partials, add=args.epilogue == "residual") for w in weights]
+        elif args.dtype == "fp32":
             gepi = ops.EPI_RESIDUAL if args.epilogue == "residual" else ops.EPI_STORE
             runs = [lambda w=w: ops.gemm_generic(x, w, o, gepi) for w in weights]
         else:
@@ -264,8 +299,8 @@ def main():
                 sys.exit("this shape cannot defer its reduction")
             runs = [lambda w=w: ops.gemm_tc_deferred(x, w, err, ws, N=N, dual_offset=N if dual else 0) for w in weights]
         wb = N * K * esize * (2 if dual else 1)
-        work = {"bytes": wb + M * K * esize + M * N * (4 if args.epilogue == "residual" else esize),
-                "flops": 2.0 * M * N * K * (2 if dual else 1), "bound": "hbm" if M <= 128 else "tensor"}
+        work = {"bytes": wb + M * K * esize + M * N * (4 if o.dtype == torch.float32 else esize),
+                "flops": 2.0 * M * N * K * (2 if dual else 1), "bound": "six tensor products" if split else ("hbm" if M <= 128 else "tensor")}
     elif args.kernel == "moe":
         # --tokens sorted rows spread evenly over the experts (the last takes the remainder); swiglu: gate and up rows and the activation
         R, N, K, X = args.tokens, args.n, args.k, args.experts
@@ -351,6 +386,8 @@ def main():
     tf = work["flops"] / (us * 1e-6) / 1e12
     if work["bound"] == "hbm":
         frac = gbs / pk["hbm_gbs"]
+    elif work["bound"] == "six tensor products":
+        frac = tf / (pk["bf16_tflops"] / 6)
     elif args.dtype == "fp32" or work["bound"] == "ffma" or args.exact:       # the CUDA cores' own peak: SMs x 128 lanes x 2 flops x the maximum clock
         frac = tf / (ops.sm_count() * 128 * 2 * 1.965e9 / 1e12)
         work["bound"] = "ffma"
