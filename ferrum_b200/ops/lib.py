@@ -30,17 +30,27 @@ _lock = threading.Lock()
 ABI = 24
 
 
-class _Entry(ctypes._CFuncPtr):
-    """An entry point.  The wrappers below hand sizes over as they come, which ctypes takes for plain integers only; a call with
-    another kind of integer (a numpy scalar, say) is made again with plain ones.  (Nothing has run before: ctypes converts first.)"""
-    _flags_ = ctypes._FUNCFLAG_CDECL
-    _restype_ = c_int
+_CTYPES = (ctypes._SimpleCData, ctypes.Array, type(ctypes.byref(c_int())))
 
-    def __call__(self, *args):
-        try:
-            return super().__call__(*args)
-        except ctypes.ArgumentError:
-            return super().__call__(*[a if a is None or isinstance(a, (ctypes._SimpleCData, ctypes.Array)) else operator.index(a) for a in args])
+
+class _Library:
+    """The library's entry points.  The wrappers below hand sizes over as they come, which ctypes takes for plain integers only: a
+    call with another kind of integer (a numpy scalar, say) is made again with plain ones.  (Nothing has run before: ctypes converts
+    first.  A closure costs a call next to nothing, a Python method of ctypes' function class 0.3 us.)"""
+
+    def __init__(self, handle):
+        self._handle = handle
+
+    def __getattr__(self, name):
+        fn = getattr(self._handle, name)
+
+        def entry(*args):
+            try:
+                return fn(*args)
+            except ctypes.ArgumentError:
+                return fn(*[a if a is None or isinstance(a, _CTYPES) else operator.index(a) for a in args])
+        setattr(self, name, entry)
+        return entry
 
 
 def lib():
@@ -51,7 +61,6 @@ def lib():
                 path = build.build_kernels()
                 try:
                     handle = ctypes.CDLL(path)
-                    handle._FuncPtr = _Entry
                 except OSError as e:
                     raise KernelError(f"cannot load the kernel library {path}: {e}") from None
                 handle.ferrum_last_error.restype = ctypes.c_char_p
@@ -61,7 +70,7 @@ def lib():
                     raise KernelError(f"{path} is a stale build; delete it and call again")
                 if os.environ.get("FERRUM_DEPENDENT_LAUNCH", "1") == "0":
                     handle.ferrum_set_dependent_launch(c_int(0))
-                _lib = handle
+                _lib = _Library(handle)
     return _lib
 
 

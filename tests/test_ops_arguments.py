@@ -1,5 +1,7 @@
 """Sizes that are integers but no Python ints (numpy scalars, as plans and tables hand them out) are taken by the wrappers and the
 library's entry points."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -10,8 +12,12 @@ def test_entry_point_sizes():
     can = ops.lib().ferrum_gemm_tc_can_defer
     for M, N, K in ((8, 4096, 4096), (300, 4096, 4096)):
         assert can(np.int64(M), np.int32(N), K, np.int8(0), np.uint16(148)) == can(M, N, K, 0, 148) == int(M == 8)
+    assert ops.gemm_tc_workspace(np.int64(8), np.int64(4096), 4096, False) == ops.gemm_tc_workspace(8, 4096, 4096, False)
     with pytest.raises(TypeError):
         can(8.0, 4096, 4096, 0, 148)
+    n = ctypes.c_int()
+    ops.lib().ferrum_gemm_tc_workspace(np.int64(8), 4096, 4096, 0, 148, ctypes.byref(n))
+    assert n.value == 32
 
 
 @pytest.mark.gpu
