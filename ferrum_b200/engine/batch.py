@@ -351,8 +351,8 @@ class StepContext:
         self.pending_experts = None
 
     # ------------------------------------------------------------------ scratch
-    def buf(self, name, shape, dtype, limit=0, captured=True):
-        return self.scratch.get(name, shape, dtype, limit, captured)
+    def buf(self, name, shape, dtype):
+        return self.scratch.get(name, shape, dtype)
 
     def gemm_scratch(self, M, N, K, dual):
         """(float32 workspace, zeroed int32 tile counters) for the tensor-core product."""

@@ -206,7 +206,7 @@ def _bytes_work(*tensors_rows):
 
 
 def _ptr(t):
-    return c_void_p(t.data_ptr()) if t is not None else c_void_p(0)
+    return c_void_p(t.data_ptr()) if t is not None else None      # (which ctypes passes as a null pointer)
 
 
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)

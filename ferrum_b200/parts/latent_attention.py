@@ -214,8 +214,8 @@ class LatentAttention(Mixer):
         n_keys, max_keys, start, first, key_row, work, n_work = plan
         T, H, R = ctx.n_tokens, self.H, self.R
         # (the keys grow with every portion of a prompt, and no captured step comes here)
-        rows = ctx.buf("lat_rows", (n_keys, self.Dk), self.dtype, limit=max_keys * self.Dk, captured=False)
-        kv = ctx.buf("lat_kv", (n_keys, H * (self.Dn + self.Dv)), self.dtype, limit=max_keys * H * (self.Dn + self.Dv), captured=False)
+        rows = ctx.scratch.get("lat_rows", (n_keys, self.Dk), self.dtype, limit=max_keys * self.Dk, captured=False)
+        kv = ctx.scratch.get("lat_kv", (n_keys, H * (self.Dn + self.Dv)), self.dtype, limit=max_keys * H * (self.Dn + self.Dv), captured=False)
         ops.latent_gather(cache.plane, cache.page_stride, cache.page_size, table, start, first, ctx.pos0, self.window, n_keys, self.Dk, rows, ctx.err)
         linear(rows[:, :R], self.w_ukv, kv, STORE, ctx, M=n_keys)
         ops.latent_q_rope_own(q, T, ctx.positions, self.rotary, H, self.Dn, self.Rr, ctx.err)
