@@ -728,8 +728,8 @@ def attention_tc_tokens(D, G, page_size, kv_plane=None, page_stride=0):
 
 
 def set_attention_pair_kernel(on: bool):
-    """Head size 128 runs the tcgen05 attention on CTA pairs (on by default); off: the single-CTA
-    kernel takes the same work items (for comparisons)."""
+    """Head size 128 runs the tcgen05 attention on CTA pairs (off by default; for comparisons): the
+    single-CTA kernel, which takes the same work items, is the quicker."""
     lib().ferrum_set_attention_pair_kernel(c_int(1 if on else 0))
 
 

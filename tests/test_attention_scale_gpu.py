@@ -40,7 +40,7 @@ def test_scales(ops, Hq, Hkv, D, window, kernel, scale, h16):
                 ops.attention_combine(out, part_o, part_ml, dev(qs), dev(req), dev(h["req_tile0"]), dev(h["tile_info"]),
                                       dev(h["comb"]), int(h["comb"].size), Hq, Hkv, D, h["bm"], 1)
     finally:
-        ops.set_attention_pair_kernel(True)
+        ops.set_attention_pair_kernel(False)
     assert e.item() == 0
     for r, (n, ql) in enumerate(zip(lens, qlens)):
         qr = q[qs[r]:qs[r + 1]].double().view(ql, Hkv, Hq // Hkv, D)
