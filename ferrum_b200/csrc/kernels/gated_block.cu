@@ -14,11 +14,32 @@
 // portion, in the request's state row.  A portion's last a goes to a staging row first and is
 // copied into the state by the block's last kernel: the state is read and written by different
 // launches, never by blocks of one grid.
+#include <initializer_list>
+
 #include "common.cuh"
 #include "partials.cuh"
 
 constexpr int GB_THREADS = 256;
 constexpr int GB_MAX_GROUPS = 512;
+
+// Four neighbouring values: loads of 16 bytes (zeros where there is no vector) and one store in the output type.
+// The three kernels of a prompt portion move every element once and are bound by memory; with a 4-byte access per element
+// and thread too few bytes were on their way (B200, 1,500 tokens x 2,048 / 5,632, us a launch within a step, before -> after:
+// norm_pair_shift 21 -> 11, bias_glu 36 -> 21, gated_residual 36 -> 20).
+template <typename T> __device__ __forceinline__ void gb_store4(T* p, float a, float b, float c, float d) {
+  *reinterpret_cast<uint2*>(p) = make_uint2(pack2<T>(a, b), pack2<T>(c, d));
+}
+template <> __device__ __forceinline__ void gb_store4<float>(float* p, float a, float b, float c, float d) {
+  *reinterpret_cast<float4*>(p) = make_float4(a, b, c, d);
+}
+__device__ __forceinline__ float4 gb_load4(const float* p, int i) { return *reinterpret_cast<const float4*>(p + i); }
+__device__ __forceinline__ float4 gb_load4_or_zero(const float* p, int i) { return p ? gb_load4(p, i) : make_float4(0.f, 0.f, 0.f, 0.f); }
+// Whether all of these (null ones aside) lie on 16-byte boundaries.
+static bool gb_aligned(std::initializer_list<const void*> ps) {
+  for (const void* p : ps)
+    if ((uintptr_t)p & 15) return false;
+  return true;
+}
 
 // 1 / sqrt(mean(part^2) + eps) of every group of row xr into inv[0 .. groups): warp w takes groups
 // w, w + warps, ...; a lane walks its group with stride 32, then the lanes meet in a butterfly.
@@ -29,7 +50,13 @@ __device__ __forceinline__ void group_inverse_rms(const float* __restrict__ xr, 
   for (int g = warp; g < groups; g += nw) {
     const float* p = xr + (size_t)g * Eg;
     float ss = 0.f;
-    for (int i = lane; i < Eg; i += 32) ss = fmaf(p[i], p[i], ss);
+    for (int i0 = lane; i0 < Eg; i0 += 32 * 8) {     // (eight loads on their way at a time; a zero changes no sum)
+      float v[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[k] = i0 + 32 * k < Eg ? p[i0 + 32 * k] : 0.f;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) ss = fmaf(v[k], v[k], ss);
+    }
     ss = warp_sum(ss);
     if (lane == 0) inv[g] = 1.0f / sqrtf(ss / (float)Eg + eps);
   }
@@ -110,7 +137,8 @@ FERRUM_API int ferrum_group_norm(const float* x, const float* w, void* out, int 
 // One block per token.  a, m, b: [T, E] in the compute dtype (b and w2 may be null: a layer without
 // a second sublayer).  shift null: m = a.  state: [slots, E] float32, the a of every request's last
 // token; stage: [requests of the batch, E] float32, receives the a of every portion's last token.
-template <typename TOut>
+// VEC: four elements a thread at a time (E / groups a multiple of 4, everything on 16-byte boundaries).
+template <typename TOut, bool VEC>
 __global__ void __launch_bounds__(GB_THREADS)
 norm_pair_shift_kernel(const float* __restrict__ x, const float* __restrict__ w1, const float* __restrict__ w2,
                        const float* __restrict__ shift, TOut* __restrict__ a_out, TOut* __restrict__ m_out, TOut* __restrict__ b_out,
@@ -132,6 +160,34 @@ norm_pair_shift_kernel(const float* __restrict__ x, const float* __restrict__ w1
   if (prev == 1) group_inverse_rms(xp, E, groups, eps, inv_prev);
   const float* sp = prev == 2 ? state + (size_t)slots[r] * E : nullptr;
   const int Eg = E / groups;
+  if constexpr (VEC) {
+    for (int i = threadIdx.x * 4; i < E; i += GB_THREADS * 4) {
+      const int g = i / Eg;
+      const float4 xv = gb_load4(xr, i), wv = gb_load4(w1, i);
+      const float4 pv = gb_load4_or_zero(prev == 1 ? xp : (prev == 2 ? sp : nullptr), i);
+      const float4 sv = gb_load4_or_zero(shift, i), w2v = gb_load4_or_zero(w2, i);
+      const float xs[4] = {xv.x, xv.y, xv.z, xv.w}, ws[4] = {wv.x, wv.y, wv.z, wv.w}, ps[4] = {pv.x, pv.y, pv.z, pv.w};
+      const float ss[4] = {sv.x, sv.y, sv.z, sv.w}, w2s[4] = {w2v.x, w2v.y, w2v.z, w2v.w};
+      const float in = inv[g], ip = prev == 1 ? inv_prev[g] : 0.f;
+      float a[4], m[4], b[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const float n = xs[k] * in;
+        a[k] = n * ws[k];
+        m[k] = a[k];
+        if (shift != nullptr) {
+          const float ap = prev == 1 ? ps[k] * ip * ws[k] : ps[k];
+          m[k] = a[k] + (ap - a[k]) * ss[k];
+        }
+        b[k] = n * w2s[k];
+      }
+      const size_t o = (size_t)t * E + i;
+      gb_store4<TOut>(a_out + o, a[0], a[1], a[2], a[3]);
+      gb_store4<TOut>(m_out + o, m[0], m[1], m[2], m[3]);
+      if (b_out != nullptr) gb_store4<TOut>(b_out + o, b[0], b[1], b[2], b[3]);
+      if (last && stage != nullptr) gb_store4<float>(stage + (size_t)r * E + i, a[0], a[1], a[2], a[3]);
+    }
+  } else
   for (int i = threadIdx.x; i < E; i += blockDim.x) {
     const int g = i / Eg;
     const float n = xr[i] * inv[g];
@@ -160,8 +216,10 @@ FERRUM_API int ferrum_norm_pair_shift(const float* x, const float* w1, const flo
   FERRUM_CHECK_ARG((b_out == nullptr) == (w2 == nullptr), "norm pair: second weight and second output go together");
   FERRUM_CHECK_ARG(shift == nullptr || (state != nullptr && stage != nullptr && slots != nullptr), "norm pair: a token shift needs its state");
   if (n_tokens == 0) return 0;
-  FERRUM_DISPATCH_DTYPE(out_dtype, T, launch_kernel(norm_pair_shift_kernel<T>, n_tokens, GB_THREADS, 0, stream, x, w1, w2, shift, (T*)a_out,
-                                                    (T*)m_out, (T*)b_out, positions, req_of_token, q_start, slots, state, stage, E, groups, eps));
+  const bool vec = E / groups % 4 == 0 && gb_aligned({x, w1, w2, shift, a_out, m_out, b_out, state, stage});
+  FERRUM_DISPATCH_DTYPE(out_dtype, T, launch_kernel(vec ? norm_pair_shift_kernel<T, true> : norm_pair_shift_kernel<T, false>, n_tokens, GB_THREADS, 0,
+                                                    stream, x, w1, w2, shift, (T*)a_out, (T*)m_out, (T*)b_out, positions, req_of_token, q_start,
+                                                    slots, state, stage, E, groups, eps));
   FERRUM_CHECK_LAUNCH("norm_pair_shift");
   return 0;
 }
@@ -193,12 +251,34 @@ bias_glu_kernel(const float* __restrict__ gu, int ld, const float* __restrict__ 
   }
 }
 
+// The same, four features a thread (F and both strides multiples of 4, 16-byte boundaries).
+constexpr int GLU_VEC_THREADS = 128;
+template <typename TOut>
+__global__ void __launch_bounds__(GLU_VEC_THREADS)
+bias_glu_vec_kernel(const float* __restrict__ gu, int ld, const float* __restrict__ bg, const float* __restrict__ bu, TOut* __restrict__ act,
+                    int ld_out, int F, int kind, float limit) {
+  pdl_launch();
+  pdl_wait();
+  const int f = (blockIdx.x * GLU_VEC_THREADS + threadIdx.x) * 4;
+  if (f >= F) return;
+  const float* row = gu + (size_t)blockIdx.y * ld;
+  const float4 g = gb_load4(row, f), u = gb_load4(row + F, f), cg = gb_load4_or_zero(bg, f), cu = gb_load4_or_zero(bu, f);
+  gb_store4<TOut>(act + (size_t)blockIdx.y * ld_out + f, glu_of(g.x + cg.x, u.x + cu.x, kind, limit), glu_of(g.y + cg.y, u.y + cu.y, kind, limit),
+                  glu_of(g.z + cg.z, u.z + cu.z, kind, limit), glu_of(g.w + cg.w, u.w + cu.w, kind, limit));
+}
+
 FERRUM_API int ferrum_bias_glu(const float* gu, int ld, const float* bias_gate, const float* bias_up, void* act, int act_dtype,
                                int ld_out, int n_tokens, int F, int kind, float limit, cudaStream_t stream) {
   FERRUM_CHECK_ARG(n_tokens >= 0 && n_tokens <= 65535 * 32 && F > 0 && ld >= 2 * F && ld_out >= F, "bias glu: bad sizes T=%d F=%d", n_tokens, F);
   FERRUM_CHECK_ARG(kind >= 0 && kind <= GLU_SWISH_CLAMP, "bias glu: unknown activation %d", kind);
   if (n_tokens == 0) return 0;
   FERRUM_CHECK_ARG(n_tokens <= 65535, "bias glu: too many tokens");
+  if (F % 4 == 0 && ld % 4 == 0 && ld_out % 4 == 0 && gb_aligned({gu, bias_gate, bias_up, act})) {
+    const dim3 vgrid((F / 4 + GLU_VEC_THREADS - 1) / GLU_VEC_THREADS, n_tokens);
+    FERRUM_DISPATCH_DTYPE(act_dtype, T, launch_kernel(bias_glu_vec_kernel<T>, vgrid, dim3(GLU_VEC_THREADS), 0, stream, gu, ld, bias_gate, bias_up, (T*)act, ld_out, F, kind, limit));
+    FERRUM_CHECK_LAUNCH("bias_glu");
+    return 0;
+  }
   const dim3 grid(min((F + 255) / 256, 64), n_tokens);
   FERRUM_DISPATCH_DTYPE(act_dtype, T, launch_kernel(bias_glu_kernel<T>, grid, dim3(256), 0, stream, gu, ld, bias_gate, bias_up, (T*)act, ld_out, F, kind, limit));
   FERRUM_CHECK_LAUNCH("bias_glu");
@@ -287,6 +367,45 @@ gated_residual_kernel(float* __restrict__ x, int E, const float* __restrict__ y1
   }
 }
 
+// The same over whole rows, four elements a thread (no partials; E and the strides multiples of 4, 16-byte boundaries).
+__global__ void __launch_bounds__(GB_THREADS)
+gated_residual_vec_kernel(float* __restrict__ x, int E, const float* __restrict__ y1, int ld_y1, const float* __restrict__ g1, int ld_g1,
+                          const float* __restrict__ c1, const float* __restrict__ y2, int ld_y2, const float* __restrict__ c2,
+                          const float* __restrict__ g2, int ld_g2, const float* __restrict__ c3, const int* __restrict__ req_of_token,
+                          const int* __restrict__ q_start, const int* __restrict__ slots, const float* __restrict__ stage,
+                          float* __restrict__ state) {
+  pdl_launch();
+  pdl_wait();
+  const int t = blockIdx.x;
+  float* xr = x + (size_t)t * E;
+  const float *y1r = y1 + (size_t)t * ld_y1, *g1r = g1 + (size_t)t * ld_g1;
+  const float *y2r = y2 ? y2 + (size_t)t * ld_y2 : nullptr, *g2r = y2 ? g2 + (size_t)t * ld_g2 : nullptr;
+#pragma unroll 2
+  for (int i = threadIdx.x * 4; i < E; i += GB_THREADS * 4) {
+    const float4 xv = gb_load4(xr, i), v1 = gb_load4(y1r, i), z1 = gb_load4(g1r, i), b1 = gb_load4_or_zero(c1, i);
+    const float4 v2 = gb_load4_or_zero(y2r, i), z2 = gb_load4_or_zero(g2r, i), b2 = gb_load4_or_zero(c2, i), b3 = gb_load4_or_zero(c3, i);
+    const float xs[4] = {xv.x, xv.y, xv.z, xv.w}, v1s[4] = {v1.x, v1.y, v1.z, v1.w}, z1s[4] = {z1.x, z1.y, z1.z, z1.w};
+    const float b1s[4] = {b1.x, b1.y, b1.z, b1.w}, v2s[4] = {v2.x, v2.y, v2.z, v2.w}, z2s[4] = {z2.x, z2.y, z2.z, z2.w};
+    const float b2s[4] = {b2.x, b2.y, b2.z, b2.w}, b3s[4] = {b3.x, b3.y, b3.z, b3.w};
+    float o[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      float add = v1s[k] * gb_sigmoid(z1s[k] + b1s[k]);
+      if (y2r != nullptr) add += (v2s[k] + b2s[k]) * gb_sigmoid(z2s[k] + b3s[k]);
+      o[k] = xs[k] + add;
+    }
+    gb_store4<float>(xr + i, o[0], o[1], o[2], o[3]);
+  }
+  if (state != nullptr) {
+    const int r = req_of_token[t];
+    if (t == q_start[r + 1] - 1) {
+      float* dst = state + (size_t)slots[r] * E;
+      const float* src = stage + (size_t)r * E;
+      for (int i = threadIdx.x * 4; i < E; i += GB_THREADS * 4) *reinterpret_cast<float4*>(dst + i) = gb_load4(src, i);
+    }
+  }
+}
+
 FERRUM_API int ferrum_gated_residual(float* x, int n_tokens, int E, const float* y1, int ld_y1, const float* g1, int ld_g1,
                                      const float* c1, const float* y2, int ld_y2, const float* c2, const float* g2, int ld_g2,
                                      const float* c3, const int* req_of_token, const int* q_start, const int* slots,
@@ -306,6 +425,13 @@ FERRUM_API int ferrum_gated_residual(float* x, int n_tokens, int E, const float*
   FERRUM_CHECK_ARG(state == nullptr || (stage != nullptr && slots != nullptr && q_start != nullptr && req_of_token != nullptr),
                    "gated residual: the state copy needs the batch description");
   if (n_tokens == 0) return 0;
+  if (n_tokens > 64 && L1.ws == nullptr && L2.ws == nullptr && (E | ld_y1 | ld_g1 | (y2 ? ld_y2 | ld_g2 : 0)) % 4 == 0 &&
+      gb_aligned({x, y1, g1, c1, y2, c2, y2 ? g2 : nullptr, c3, stage, state})) {
+    launch_kernel(gated_residual_vec_kernel, dim3(n_tokens), dim3(GB_THREADS), 0, stream, x, E, y1, ld_y1, g1, ld_g1, c1, y2, ld_y2, c2, g2, ld_g2, c3,
+                  req_of_token, q_start, slots, stage, state);
+    FERRUM_CHECK_LAUNCH("gated_residual");
+    return 0;
+  }
   const int slices = n_tokens <= 64 ? max(1, min(16, E / 256)) : 1;
   launch_kernel(gated_residual_kernel, dim3(n_tokens, slices), dim3(GB_THREADS), 0, stream, x, E, y1, ld_y1, g1, ld_g1, c1, y2, ld_y2, c2, g2, ld_g2, c3,
                 req_of_token, q_start, slots, stage, state, L1, L2);
