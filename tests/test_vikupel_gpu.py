@@ -268,6 +268,12 @@ def test_state_space_mixer_alone(cuda, dtype, heads, P_, N, G, ng, taps):
         assert (got - ref).abs().max() < (2e-4 if dtype == "float32" else 4e-2) * ref.abs().max(), cuts
 
 
+@pytest.mark.parametrize("heads,P_,ng", [(51, 5, 1), (64, 64, 1), (66, 64, 1), (66, 64, 2)])
+def test_state_space_mixer_norm_widths(cuda, heads, P_, ng):
+    """Gated norms of 255, 4096 (what a block's threads keep between their two passes), 4224 and 2112 elements."""
+    test_state_space_mixer_alone(cuda, "float32", heads, P_, 8, 1, ng, 3)
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("kind,H,G,Dk,Dv", [("window", 3, 1, 10, 14), ("window", 6, 2, 80, 80), ("rotary", 4, 2, 64, 64), ("rotary", 2, 2, 12, 10),
                                             ("rotary", 4, 1, 8, 24)])
