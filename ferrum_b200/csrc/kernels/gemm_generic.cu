@@ -18,7 +18,7 @@
 // Llama-3.1-8B shapes with 8 tokens: 43 to 60 % of the copy bandwidth, 65 % with one token; four
 // features per CTA with the next block's weights requested ahead was no faster.)
 //
-// Stream (float32 with 16-byte aligned rows, up to 64 tokens in passes of 8: the decode steps of
+// Stream (float32 with 16-byte aligned rows, up to four tokens in a kernel of their own, up to 64 in passes of 8: the decode steps of
 // the 32-bit path; the skinny kernel remains for 16-bit types and unaligned rows):
 // the skinny kernel keeps too few bytes on their way (its loads wait in registers for the
 // multiplications before them: 22 % of the warp slots busy, 46 % of the copy bandwidth at 8
@@ -33,6 +33,8 @@
 // result does not depend on how many other tokens are in the call or where it stands among
 // them.  (Between the kernels the orders differ: a token decoded alone and the same token
 // inside a larger batch agree to rounding, not bitwise.)
+#include <algorithm>
+
 #include "common.cuh"
 
 enum GemmEpilogue : int {
@@ -341,6 +343,162 @@ gemm_stream_kernel(const float* __restrict__ x, const float* __restrict__ w, voi
   }
 }
 
+// ------------------------------------------------------------------ stream kernel for up to four tokens
+// With up to four tokens a thread can carry all of a group's sums, so that nothing but their meeting at the group's end crosses
+// threads: a thread owns the elements 4 tid .. + 3 of every 512-element slice of K, brings them into its own places of a ring of
+// six slices with cp.async, and needs no barrier until then.  A CTA owns an even share of the features and walks it in groups of up
+// to 8; the ring runs on across slices and groups, so that no group begins with an empty one.  The tokens (which the L2
+// holds) come through registers one slice ahead.  Same sums in the same order as the kernel above: over slices in a thread, over a
+// warp's lanes in a butterfly, over the four warps in order.
+// B200, weights from memory, us, the kernel above -> this one, 4 tokens: 3072 x 3072 12.2 -> 10.5, 5120 x 3072 18.2 -> 14.8,
+// 16384 x 3072 45.4 -> 34.6, 3072 x 8192 25.9 -> 21.8, 128256 x 3072 333 -> 244 (6.5 TB/s); one token the same, 64 x 64 2.6 -> 2.0.
+// From five tokens on it loses (8 tokens, two sets of threads or eight sums a feature: 12.4 -> 14.6..15.8, 26.2 -> 30.8..33.6): every group
+// reads the tokens again, and a group of five or six features has then as many of their bytes as of the weights'.
+constexpr int S4_FEAT = 8;       // features of a group at most
+constexpr int S4_TOK = 4;        // tokens at most
+constexpr int S4_THREADS = 128;
+constexpr int S4_CTAS_PER_SM = 2;
+constexpr int S4_STAGES = 6;
+constexpr int S4_SMEM_BYTES = S4_STAGES * S4_FEAT * ST_KT * 4;
+
+__global__ void __launch_bounds__(S4_THREADS, S4_CTAS_PER_SM)
+gemm_stream4_kernel(const float* __restrict__ x, const float* __restrict__ w, void* __restrict__ out, int M, int N, int K,
+                    int ldx, int ldw, int ldo, int epi) {
+  constexpr int ROW = ST_KT * 4, STAGE = S4_FEAT * ROW;
+  extern __shared__ __align__(16) float st_smem[];
+  __shared__ float red[2][S4_THREADS / 32][32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int f_begin = (int)((long long)N * blockIdx.x / gridDim.x), f_end = (int)((long long)N * (blockIdx.x + 1) / gridDim.x);
+  const int n_groups = (f_end - f_begin + S4_FEAT - 1) / S4_FEAT, n_slices = (K + ST_KT - 1) / ST_KT;
+  float* const ring = st_smem + tid * 4;
+
+  // a step of the walk: slice s of the nf features from n0 on (group g)
+  struct Step {
+    int g, s, n0, nf;
+  };
+  auto enter_group = [&](Step& q) {
+    q.n0 = f_begin + (int)((long long)(f_end - f_begin) * q.g / n_groups);
+    q.nf = f_begin + (int)((long long)(f_end - f_begin) * (q.g + 1) / n_groups) - q.n0;
+  };
+  auto advance = [&](Step& q) {
+    if (++q.s < n_slices) return;
+    q.s = 0;
+    if (++q.g < n_groups) enter_group(q);
+  };
+  // rows past the group's features are not brought (what the ring holds there only reaches sums that are not stored),
+  // elements past K arrive as zeros
+  auto load_weights = [&](const Step& q, int stage) {
+    const int k = q.s * ST_KT + tid * 4, bytes = k < K ? 16 : 0;
+    const float* p = w + (size_t)q.n0 * ldw + (k < K ? k : 0);
+#pragma unroll
+    for (int f = 0; f < S4_FEAT; ++f)
+      if (f < q.nf) st_cp_async16(ring + (stage * STAGE + f * ROW) / 4, p + (size_t)f * ldw, bytes);
+  };
+  auto load_tokens = [&](const Step& q, float4 (&v)[S4_TOK]) {
+    const int k = q.s * ST_KT + tid * 4;
+#pragma unroll
+    for (int m = 0; m < S4_TOK; ++m)
+      v[m] = k < K && m < M ? __ldcg(reinterpret_cast<const float4*>(x + (size_t)m * ldx + k)) : make_float4(0.f, 0.f, 0.f, 0.f);
+  };
+
+  Step ahead{0, 0, f_begin, 0};
+  enter_group(ahead);
+  Step now = ahead, next = ahead;
+  // The first weights start for the L2 before the kernel ahead of this one has ended.
+  {
+    Step q = ahead;
+    for (int i = 0; i < S4_STAGES && q.g < n_groups; ++i) {
+      const int k = q.s * ST_KT + tid * 4;
+      if ((tid & 7) == 0 && k < K)
+        for (int f = 0; f < q.nf; ++f) asm volatile("prefetch.global.L2 [%0];" ::"l"(w + (size_t)(q.n0 + f) * ldw + k));
+      advance(q);
+    }
+  }
+  pdl_wait();
+  pdl_launch();
+#pragma unroll
+  for (int i = 0; i < S4_STAGES - 1; ++i) {
+    if (ahead.g < n_groups) {
+      load_weights(ahead, i);
+      advance(ahead);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  float4 xn[S4_TOK];
+  load_tokens(next, xn);
+  advance(next);
+  float acc[S4_FEAT * S4_TOK];
+#pragma unroll
+  for (int i = 0; i < S4_FEAT * S4_TOK; ++i) acc[i] = 0.f;
+  int stage = 0;
+  while (now.g < n_groups) {
+    float4 xv[S4_TOK];
+#pragma unroll
+    for (int m = 0; m < S4_TOK; ++m) xv[m] = xn[m];
+    if (next.g < n_groups) {
+      load_tokens(next, xn);
+      advance(next);
+    }
+    asm volatile("cp.async.wait_group %0;" ::"n"(S4_STAGES - 2) : "memory");   // this thread's weights of the step are there
+    // (the place this fills was read by this thread in the step before)
+    if (ahead.g < n_groups) {
+      load_weights(ahead, stage == 0 ? S4_STAGES - 1 : stage - 1);
+      advance(ahead);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    const float* const st = ring + stage * (STAGE / 4);
+#pragma unroll
+    for (int f = 0; f < S4_FEAT; ++f) {
+      const float4 wv = *reinterpret_cast<const float4*>(st + f * ST_KT);
+#pragma unroll
+      for (int m = 0; m < S4_TOK; ++m) {
+        float& a = acc[f * S4_TOK + m];
+        a = fmaf(wv.x, xv[m].x, a);
+        a = fmaf(wv.y, xv[m].y, a);
+        a = fmaf(wv.z, xv[m].z, a);
+        a = fmaf(wv.w, xv[m].w, a);
+      }
+    }
+    if (++stage == S4_STAGES) stage = 0;
+
+    if (now.s == n_slices - 1) {
+      // the 32 lanes meet: after five steps lane i holds the warp's sum of value i = f * 4 + m
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) {
+        const bool upper = (lane & off) != 0;
+#pragma unroll
+        for (int i = 0; i < off; ++i) {
+          const float mine = upper ? acc[i + off] : acc[i];
+          const float theirs = upper ? acc[i] : acc[i + off];
+          acc[i] = mine + __shfl_xor_sync(0xffffffffu, theirs, off);
+        }
+      }
+      float (*const place)[32] = red[now.g & 1];     // (two places: one is written again only after the barrier of the group between)
+      place[warp][lane] = acc[0];
+      __syncthreads();
+      if (tid < 32) {
+        float sum = 0.f;
+#pragma unroll
+        for (int wi = 0; wi < S4_THREADS / 32; ++wi) sum += place[wi][tid];
+        const int f = tid / S4_TOK, m = tid % S4_TOK;
+        if (f < now.nf && m < M) epilogue_store<float>(out, (size_t)m * ldo + now.n0 + f, sum, epi);
+      }
+#pragma unroll
+      for (int i = 0; i < S4_FEAT * S4_TOK; ++i) acc[i] = 0.f;
+    }
+    advance(now);
+  }
+}
+
+static int stream_sm_count() {
+  static const int n = [] {
+    int dev = 0, v = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v <= 0) v = 148;
+    return v;
+  }();
+  return n;
+}
+
 template <typename T>
 static int launch_generic(const void* x, const void* w, void* out, int M, int N, int K, int ldx, int ldw, int ldo,
                           int epilogue, cudaStream_t stream) {
@@ -349,6 +507,15 @@ static int launch_generic(const void* x, const void* w, void* out, int M, int N,
   const T* xp = (const T*)x;
   const T* wp = (const T*)w;
   if constexpr (sizeof(T) == 4) {
+    if (vec && M <= S4_TOK) {
+      static const cudaError_t e4 = cudaFuncSetAttribute(gemm_stream4_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S4_SMEM_BYTES);
+      FERRUM_CHECK_ARG(e4 == cudaSuccess, "gemm: cannot reserve %d bytes of shared memory: %s", S4_SMEM_BYTES, cudaGetErrorString(e4));
+      const int ctas = std::min((N + 3) / 4, S4_CTAS_PER_SM * stream_sm_count());      // (every CTA has a feature)
+      launch_kernel(gemm_stream4_kernel, dim3(ctas), dim3(S4_THREADS), S4_SMEM_BYTES, stream, (const float*)x, (const float*)w, out, M, N, K,
+                    ldx, ldw, ldo, epilogue);
+      FERRUM_CHECK_LAUNCH("gemm_generic");
+      return 0;
+    }
     if (vec && M <= SK_MAX_TOKENS) {
       static bool configured = false;
       if (!configured) {
