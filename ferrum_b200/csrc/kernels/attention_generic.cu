@@ -143,6 +143,7 @@ attention_generic_kernel(const T* __restrict__ q, int ldq, T* __restrict__ out, 
                          int* __restrict__ err, float* __restrict__ part, int split_slots, int vec,
                          const float* __restrict__ bias1, const float* __restrict__ bias2, int out_f32, int chunked,
                          float softcap, int sink, int keep_first, float out_scale) {
+  pdl_wait();
   using Tile = AgTile<DI>;
   constexpr int TK = Tile::TK, DP = Tile::DP, KS = Tile::KS;
   extern __shared__ __align__(16) float ag_smem[];
@@ -405,6 +406,7 @@ attention_generic_tokens_kernel(const T* __restrict__ q, int ldq, T* __restrict_
                                 int* __restrict__ err, int vec, const float* __restrict__ bias1,
                                 const float* __restrict__ bias2, int out_f32, int chunked, float softcap, int sink, int keep_first,
                                 float out_scale) {
+  pdl_wait();
   using Tile = AgTile<DI>;
   using TT = AgTokenTile<DI>;
   constexpr int TK = Tile::TK, DP = Tile::DP, KS = Tile::KS;
@@ -628,6 +630,8 @@ __global__ void __launch_bounds__(32)
 attention_generic_combine_kernel(T* __restrict__ out, int ldo, const float* __restrict__ part, const int* __restrict__ positions,
                                  int Hq, int D, int window, int split_slots, int out_f32, int chunked, int sink, int keep_first,
                                  float out_scale) {
+  pdl_launch();
+  pdl_wait();
   const int t = blockIdx.x, h = blockIdx.y, lane = threadIdx.x;
   const int pos = positions[t];
   const int lo = ag_first_key(pos, window, chunked);
@@ -720,7 +724,7 @@ FERRUM_API int ferrum_attention_generic(const void* q, int ldq, void* out, int l
                        AgTokenTile<DI_>::SMEM_BYTES, cudaGetErrorString(e));                                            \
       configured = true;                                                                                                \
     }                                                                                                                   \
-    attention_generic_tokens_kernel<T, DI_><<<(unsigned)ctas, AG_TWARPS * 32, AgTokenTile<DI_>::SMEM_BYTES, stream>>>(   \
+    launch_kernel(attention_generic_tokens_kernel<T, DI_>, dim3((unsigned)ctas), dim3(AG_TWARPS * 32), AgTokenTile<DI_>::SMEM_BYTES, stream, \
       (const T*)q, ldq, (T*)out, ldo, positions, q_start, n_reqs, block_table, table_width, (const T*)kv_plane,         \
       page_stride, page_size, Hq, Hkv, D, scale, window, err_flag, vec, bias1, bias2, out_f32, chunked, softcap, sink, keep_first, out_scale);                \
   })
@@ -743,7 +747,7 @@ FERRUM_API int ferrum_attention_generic(const void* q, int ldq, void* out, int l
                        cudaGetErrorString(e));                                                                          \
       configured = true;                                                                                                \
     }                                                                                                                   \
-    attention_generic_kernel<T, DI_><<<grid, AG_WARPS * 32, AgTile<DI_>::SMEM_BYTES, stream>>>(                        \
+    launch_kernel(attention_generic_kernel<T, DI_>, grid, dim3(AG_WARPS * 32), AgTile<DI_>::SMEM_BYTES, stream,            \
       (const T*)q, ldq, (T*)out, ldo, positions, req_of_token, block_table, table_width, (const T*)kv_plane, page_stride, \
       page_size, Hq, Hkv, D, scale, window, err_flag, part, split_slots, vec, bias1, bias2, out_f32, chunked, softcap, sink, keep_first, out_scale);          \
   })
@@ -756,7 +760,7 @@ FERRUM_API int ferrum_attention_generic(const void* q, int ldq, void* out, int l
   if (part != nullptr) {
     const dim3 cgrid(n_tokens, Hq);
     FERRUM_CHECK_ARG(cgrid.y <= 65535, "attention: too many heads");
-    FERRUM_DISPATCH_DTYPE(dtype, T, (attention_generic_combine_kernel<T><<<cgrid, 32, 0, stream>>>(
+    FERRUM_DISPATCH_DTYPE(dtype, T, (launch_kernel(attention_generic_combine_kernel<T>, cgrid, dim3(32), 0, stream,
         (T*)out, ldo, part, positions, Hq, D, window, split_slots, out_f32, chunked, sink, keep_first, out_scale)));
     FERRUM_CHECK_LAUNCH("attention_generic_combine");
   }

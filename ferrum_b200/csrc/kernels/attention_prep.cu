@@ -49,6 +49,8 @@ qkv_shape_kernel(const float* __restrict__ proj, int ldp, int n_tokens, const in
                  const float* __restrict__ cs_v, int v_pairing, int n_pos_v, int unit_norm, float eps,
                  T* __restrict__ q_out, int ldq, T* __restrict__ plane, long long page_stride, int page_size,
                  int Hq, int Hkv, int Dk, int Dv, int Dp, int writes, int* __restrict__ err, const HeadExtras x) {
+  pdl_launch();
+  pdl_wait();
   __shared__ float rows[AP_WARPS][AP_MAX_D];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int slots = Hq + (writes ? 2 * Hkv : 0);
@@ -147,6 +149,7 @@ attention_finish_kernel(const float* __restrict__ o, int ldo, int n_tokens, cons
                         const float* __restrict__ cs_v, int v_pairing, int n_pos_v, const float* __restrict__ gate,
                         int ldg, T* __restrict__ out, int ldout, int Hq, int Dv, int Dp, int* __restrict__ err, float out_scale) {
   pdl_launch();      // the product that follows may fetch its weights meanwhile
+  pdl_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long long item = (long long)blockIdx.x * AP_WARPS + warp;
   if (item >= (long long)n_tokens * Hq) return;
@@ -205,7 +208,7 @@ FERRUM_API int ferrum_qkv_shape(const float* proj, int ldp, int n_tokens, const 
   const long long items = (long long)n_tokens * (Hq + (writes ? 2 * Hkv : 0));
   const long long blocks = (items + AP_WARPS - 1) / AP_WARPS;
   FERRUM_CHECK_ARG(blocks < (1LL << 31), "qkv_shape: too many rows");
-  FERRUM_DISPATCH_DTYPE(dtype, T, (qkv_shape_kernel<T><<<(unsigned)blocks, AP_WARPS * 32, 0, stream>>>(
+  FERRUM_DISPATCH_DTYPE(dtype, T, (launch_kernel(qkv_shape_kernel<T>, dim3((unsigned)blocks), dim3(AP_WARPS * 32), 0, stream,
       proj, ldp, n_tokens, positions, req_of_token, block_table, table_width, cs_qk, rope_dim, qk_pairing, n_pos_qk, cs_v,
       v_pairing, n_pos_v, unit_norm, eps, (T*)q_out, ldq, (T*)plane, page_stride, page_size, Hq, Hkv, Dk, Dv, Dp, writes,
       err, extras)));
@@ -221,7 +224,7 @@ FERRUM_API int ferrum_attention_finish(const float* o, int ldo, int n_tokens, co
   if (n_tokens == 0) return 0;
   const long long blocks = ((long long)n_tokens * Hq + AP_WARPS - 1) / AP_WARPS;
   FERRUM_CHECK_ARG(blocks < (1LL << 31), "attention_finish: too many rows");
-  FERRUM_DISPATCH_DTYPE(dtype, T, (attention_finish_kernel<T><<<(unsigned)blocks, AP_WARPS * 32, 0, stream>>>(
+  FERRUM_DISPATCH_DTYPE(dtype, T, (launch_kernel(attention_finish_kernel<T>, dim3((unsigned)blocks), dim3(AP_WARPS * 32), 0, stream,
       o, ldo, n_tokens, positions, cs_v, v_pairing, n_pos_v, gate, ldg, (T*)out, ldout, Hq, Dv, Dp, err, out_scale)));
   FERRUM_CHECK_LAUNCH("attention_finish");
   return 0;

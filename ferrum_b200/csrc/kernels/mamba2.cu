@@ -29,6 +29,8 @@ mamba_conv_kernel(const float* __restrict__ proj, int ldp, int off_xbc, int C, i
                   const float* __restrict__ bias, const float* __restrict__ state, long long state_stride,
                   long long conv_off, const int* __restrict__ req_of_token, const int* __restrict__ q_start,
                   const int* __restrict__ slots, float* __restrict__ out, int n_tokens) {
+  pdl_launch();
+  pdl_wait();
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (long long)n_tokens * C) return;
   const int t = (int)(idx / C), c = (int)(idx % C);
@@ -49,6 +51,8 @@ __global__ void __launch_bounds__(256)
 mamba_conv_state_kernel(const float* __restrict__ proj, int ldp, int off_xbc, int C, int taps, float* __restrict__ state,
                         long long state_stride, long long conv_off, const int* __restrict__ q_start,
                         const int* __restrict__ slots, int n_reqs) {
+  pdl_launch();
+  pdl_wait();
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (long long)n_reqs * C) return;
   const int r = (int)(idx / C), c = (int)(idx % C);
@@ -102,6 +106,7 @@ mamba_scan_kernel(const float* __restrict__ xbc, int C, const float* __restrict_
                   const float* __restrict__ dt_bias, const float* __restrict__ a_log, const float* __restrict__ d_skip,
                   float* __restrict__ state, long long state_stride, const int* __restrict__ q_start,
                   const int* __restrict__ slots, float* __restrict__ y, int heads, int P, int N, int groups, int vec) {
+  pdl_wait();
   using Tile = MsTile<NQ, TC>;
   constexpr int W = Tile::W, NT = MS_WARPS * 32;
   extern __shared__ __align__(16) float ms_smem[];
@@ -235,6 +240,12 @@ mamba_gate_norm_kernel(const float* __restrict__ y, int inner, const float* __re
   const float* zr = proj + (size_t)t * ldp + off_z + (size_t)grp * width;
   const float* wr = w + (size_t)grp * width;
   float keep[GN_KEEP], wk[GN_KEEP];
+#pragma unroll
+  for (int k = 0; k < GN_KEEP; ++k) {      // (the weights never change: they come while the kernel ahead of this one ends)
+    const int i = threadIdx.x + k * 256;
+    wk[k] = i < width ? wr[i] : 0.f;
+  }
+  pdl_wait();
   float ss = 0.f;
   {
     float yv[GN_KEEP], zv[GN_KEEP];
@@ -243,7 +254,6 @@ mamba_gate_norm_kernel(const float* __restrict__ y, int inner, const float* __re
       const int i = threadIdx.x + k * 256;
       yv[k] = i < width ? yr[i] : 0.f;
       zv[k] = i < width ? zr[i] : 0.f;
-      wk[k] = i < width ? wr[i] : 0.f;
     }
 #pragma unroll
     for (int k = 0; k < GN_KEEP; ++k) {
@@ -287,14 +297,14 @@ FERRUM_API int ferrum_mamba2_mix(const float* proj, int ldp, int n_tokens, int n
   const long long conv_off = (long long)inner * N;
   {
     const long long n = (long long)n_tokens * C;
-    mamba_conv_kernel<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(proj, ldp, off_xbc, C, taps, conv_w, conv_b, state,
+    launch_kernel(mamba_conv_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, stream, proj, ldp, off_xbc, C, taps, conv_w, conv_b, state,
                                                                       state_stride, conv_off, req_of_token, q_start, slots,
                                                                       xbc, n_tokens);
     FERRUM_CHECK_LAUNCH("mamba_conv");
   }
   if (taps > 1) {
     const long long n = (long long)n_reqs * C;
-    mamba_conv_state_kernel<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(proj, ldp, off_xbc, C, taps, state, state_stride,
+    launch_kernel(mamba_conv_state_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, stream, proj, ldp, off_xbc, C, taps, state, state_stride,
                                                                             conv_off, q_start, slots, n_reqs);
     FERRUM_CHECK_LAUNCH("mamba_conv_state");
   }
@@ -312,7 +322,7 @@ FERRUM_API int ferrum_mamba2_mix(const float* proj, int ldp, int n_tokens, int n
                        MsTile<NQ_, TC_>::SMEM_BYTES, cudaGetErrorString(e));                                               \
       configured = true;                                                                                                   \
     }                                                                                                                      \
-    mamba_scan_kernel<NQ_, TC_><<<grid, MS_WARPS * 32, MsTile<NQ_, TC_>::SMEM_BYTES, stream>>>(                            \
+    launch_kernel(mamba_scan_kernel<NQ_, TC_>, grid, dim3(MS_WARPS * 32), MsTile<NQ_, TC_>::SMEM_BYTES, stream,           \
         xbc, C, proj, ldp, off_dt, dt_bias, a_log, d_skip, state, state_stride, q_start, slots, y, heads, P, N, groups, vec); \
   } while (0)
 #define MS_SCAN(NQ_)                  \
@@ -330,7 +340,7 @@ FERRUM_API int ferrum_mamba2_mix(const float* proj, int ldp, int n_tokens, int n
   }
   {
     const dim3 grid(n_tokens, norm_groups);
-    FERRUM_DISPATCH_DTYPE(dtype, T, (mamba_gate_norm_kernel<T><<<grid, 256, 0, stream>>>(y, inner, proj, ldp, 0, norm_w, (T*)out,
+    FERRUM_DISPATCH_DTYPE(dtype, T, (launch_kernel(mamba_gate_norm_kernel<T>, grid, dim3(256), 0, stream, y, inner, proj, ldp, 0, norm_w, (T*)out,
                                                                                          ldo, norm_groups, eps)));
     FERRUM_CHECK_LAUNCH("mamba_gate_norm");
   }

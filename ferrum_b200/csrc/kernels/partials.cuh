@@ -58,6 +58,30 @@ __device__ __forceinline__ float partial_sum(const PartialLayout& L, const Parti
   return acc;
 }
 
+// The same for four neighbouring features from n on (a multiple of 4: they share a tile), in 16-byte loads.
+__device__ __forceinline__ float4 partial_sum4(const PartialLayout& L, const PartialTable& tab, int col, int n) {
+  const int tile = n >> 7, nl = n & 127;
+  const int fc = tab.first_and_count[tile];
+  const int c_first = fc & 0xFFFF, count = fc >> 16;
+  const unsigned bits = tab.slot_bits[tile];
+  const float* base = L.ws + (size_t)col * 128 + nl;
+  const size_t slot_floats = (size_t)L.acc_cols * 128;
+  float4 v[PARTIAL_MAX_CONTRIB];
+#pragma unroll
+  for (int s = 0; s < PARTIAL_MAX_CONTRIB; ++s)
+    v[s] = s < count ? __ldcg(reinterpret_cast<const float4*>(base + (size_t)((c_first + s) * 2 + ((bits >> s) & 1)) * slot_floats))
+                     : make_float4(0.f, 0.f, 0.f, 0.f);
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+  for (int s = 0; s < PARTIAL_MAX_CONTRIB; ++s) {
+    acc.x += v[s].x;
+    acc.y += v[s].y;
+    acc.z += v[s].z;
+    acc.w += v[s].w;
+  }
+  return acc;
+}
+
 // The four numbers a product in deferred mode hands to its consumer (k-blocks per tile, tiles,
 // CTAs, columns per partial) as a PartialLayout; returns non-zero (and sets the error text) when
 // they cannot be what the product kernel writes.

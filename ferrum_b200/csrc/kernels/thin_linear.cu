@@ -45,6 +45,11 @@ thin_linear_kernel(const T* __restrict__ x, int ldx, const T* __restrict__ w, in
   for (int i = 0; i < TL_TOKENS; ++i) xr[i] = x + (size_t)(t0 + min(i, nt - 1)) * ldx;     // (rows past the last repeat it and are dropped)
 #pragma unroll
   for (int j = 0; j < NF; ++j) wr[j] = w + (size_t)min(n0 + j, N - 1) * K;
+  // The weights never change: they start for the L2 while the kernel ahead of this one ends.
+  for (int k = tid * 8; k < K; k += TL_THREADS * 8)
+#pragma unroll
+    for (int j = 0; j < NF; ++j) asm volatile("prefetch.global.L2 [%0];" ::"l"(wr[j] + k));
+  pdl_wait();
   for (int k = tid * 8; k < K; k += TL_THREADS * 8) {
     uint4 xraw[TL_TOKENS];
 #pragma unroll
@@ -135,10 +140,10 @@ FERRUM_API int ferrum_thin_linear(const void* x, int ldx, const void* w, int dty
   FERRUM_CHECK_ARG(chunks <= 65535, "thin_linear: too many tokens");
   // a few tokens: two features a block, so that the blocks cover the GPU; many: eight, so that the rows are read once or twice
   if (n_tokens <= 64) {
-    FERRUM_DISPATCH_16BIT(dtype, T, (thin_linear_kernel<T, 2><<<dim3((N + 1) / 2, chunks), TL_THREADS, 0, stream>>>((const T*)x, ldx, (const T*)w, K, N,
+    FERRUM_DISPATCH_16BIT(dtype, T, (launch_kernel(thin_linear_kernel<T, 2>, dim3((N + 1) / 2, chunks), dim3(TL_THREADS), 0, stream, (const T*)x, ldx, (const T*)w, K, N,
                                                                                                                   n_tokens, ep)));
   } else {
-    FERRUM_DISPATCH_16BIT(dtype, T, (thin_linear_kernel<T, 8><<<dim3((N + 7) / 8, chunks), TL_THREADS, 0, stream>>>((const T*)x, ldx, (const T*)w, K, N,
+    FERRUM_DISPATCH_16BIT(dtype, T, (launch_kernel(thin_linear_kernel<T, 8>, dim3((N + 7) / 8, chunks), dim3(TL_THREADS), 0, stream, (const T*)x, ldx, (const T*)w, K, N,
                                                                                                                   n_tokens, ep)));
   }
   FERRUM_CHECK_LAUNCH("thin_linear");
