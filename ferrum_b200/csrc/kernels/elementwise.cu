@@ -589,7 +589,10 @@ FERRUM_API int ferrum_rope_cache_write(void* qkv, int dtype, int n_tokens, int l
   const int threads = 256;
   // few tokens, or a product still in partials (several loads per element): several blocks per
   // token, four head slots each, so that a row is read by many SMs at once
-  const dim3 grid(n_tokens, (n_tokens <= 64 || partials != nullptr) ? (Hq + 2 * Hkv + 3) / 4 : 1);
+  // more: eight head slots each while a block a token would leave an SM fewer than eight (float32, 300 tokens of 40 slots of
+  // 128: 9.7 us with a block a token, 7.7 so)
+  const int slots = Hq + 2 * Hkv;
+  const dim3 grid(n_tokens, (n_tokens <= 64 || partials != nullptr) ? (slots + 3) / 4 : (n_tokens < 8 * 148 ? (slots + 7) / 8 : 1));
   FERRUM_DISPATCH_DTYPE(dtype, T, launch_kernel(rope_cache_kernel<T>, grid, threads, 0, stream, (T*)qkv, ld, positions, req_of_token,
                                                 block_table, table_width, cos_sin, n_pos, (T*)kv_plane, page_stride, page_size, Hq,
                                                 Hkv, D, R, pairing, write_kv, err_flag, L));
@@ -611,6 +614,20 @@ __global__ void swiglu_kernel(const T* __restrict__ gu, T* __restrict__ act, int
     const float gv = to_f32<T>(g[f]);
     o[f] = from_f32<T>(gv / (1.0f + expf(-gv)) * to_f32<T>(u[f]));
   }
+}
+
+// float32 rows of 16-byte multiples: four features a thread, the same formula.  (300 tokens x 8,192 on a B200: 11.7 us with an
+// element at a time, 5.8 so.)
+__global__ void __launch_bounds__(128)
+swiglu_f32x4_kernel(const float* __restrict__ gu, float* __restrict__ act, int F, int ld_in, int ld_out) {
+  pdl_launch();
+  pdl_wait();
+  const int f = (blockIdx.x * 128 + threadIdx.x) * 4;
+  if (f >= F) return;
+  const float* row = gu + (size_t)blockIdx.y * ld_in + f;
+  const float4 g = *reinterpret_cast<const float4*>(row), u = *reinterpret_cast<const float4*>(row + F);
+  *reinterpret_cast<float4*>(act + (size_t)blockIdx.y * ld_out + f) =
+      make_float4(g.x / (1.0f + expf(-g.x)) * u.x, g.y / (1.0f + expf(-g.y)) * u.y, g.z / (1.0f + expf(-g.z)) * u.z, g.w / (1.0f + expf(-g.w)) * u.w);
 }
 
 // 16-bit rows of 16-byte multiples: 16-byte loads and stores, SWIGLU_VEC groups of eight features
@@ -751,6 +768,11 @@ FERRUM_API int ferrum_swiglu(const void* gu, void* act, int dtype, int n_tokens,
       ((uintptr_t)act & 15) == 0) {
     dim3 vgrid((F / 8 + 256 * SWIGLU_VEC - 1) / (256 * SWIGLU_VEC), n_tokens);
     FERRUM_DISPATCH_16BIT(dtype, T, launch_kernel(swiglu_vec_kernel<T>, vgrid, dim3(256), 0, stream, (const T*)gu, (T*)act, F, ld_in, ld_out));
+    FERRUM_CHECK_LAUNCH("swiglu");
+    return 0;
+  }
+  if (dtype == FERRUM_F32 && F % 4 == 0 && ld_in % 4 == 0 && ld_out % 4 == 0 && ((uintptr_t)gu & 15) == 0 && ((uintptr_t)act & 15) == 0) {
+    launch_kernel(swiglu_f32x4_kernel, dim3((F / 4 + 127) / 128, n_tokens), dim3(128), 0, stream, (const float*)gu, (float*)act, F, ld_in, ld_out);
     FERRUM_CHECK_LAUNCH("swiglu");
     return 0;
   }
