@@ -105,11 +105,18 @@ __global__ void __launch_bounds__(512)
 rmsnorm_vec_kernel(const float* __restrict__ x, const float* __restrict__ w, TOut* __restrict__ out,
                    const int* __restrict__ rows, int E, float eps) {
   __shared__ float red[32];
+  const int n4 = E >> 2;
+  const float4* w4 = reinterpret_cast<const float4*>(w);
+  float4 g4[NORM_VEC_MAX];      // (the weights never change: they come while the kernel ahead of this one ends)
+#pragma unroll
+  for (int k = 0; k < NORM_VEC_MAX; ++k) {
+    const int i = threadIdx.x + k * blockDim.x;
+    g4[k] = i < n4 ? __ldg(w4 + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
   pdl_launch();
   pdl_wait();
   const int r = blockIdx.x;
   const float4* xr = reinterpret_cast<const float4*>(x + (size_t)(rows ? rows[r] : r) * E);
-  const int n4 = E >> 2;
   float4 v[NORM_VEC_MAX];
   float ss = 0.f;
 #pragma unroll
@@ -123,13 +130,12 @@ rmsnorm_vec_kernel(const float* __restrict__ x, const float* __restrict__ w, TOu
   }
   ss = block_sum(ss, red);
   const float inv = 1.0f / sqrtf(ss / (float)E + eps);
-  const float4* w4 = reinterpret_cast<const float4*>(w);
   TOut* o = out + (size_t)r * E;
 #pragma unroll
   for (int k = 0; k < NORM_VEC_MAX; ++k) {
     const int i = threadIdx.x + k * blockDim.x;
     if (i >= n4) continue;
-    const float4 g = w4[i];
+    const float4 g = g4[k];
     const float a = v[k].x * inv * g.x, b = v[k].y * inv * g.y, c = v[k].z * inv * g.z, d = v[k].w * inv * g.w;
     if (sizeof(TOut) == 4) {
       reinterpret_cast<float4*>(o)[i] = make_float4(a, b, c, d);
@@ -485,13 +491,20 @@ rope_cache_vec_kernel(T* __restrict__ qkv, int ld, const int* __restrict__ posit
   const int per_token = rot_items + (write_kv ? Hkv * (D >> 3) : 0);
   const int t = blockIdx.y, item = blockIdx.x * blockDim.x + threadIdx.x;   // the grid is (items, tokens)
   if (item >= per_token) return;
-  const int pos = positions[t];
   const int half = D >> 1;
+  T* row = qkv + (size_t)t * ld;
+  // What the thread turns or copies is asked for before its position and page are known: three latencies in a row otherwise.
+  const bool value = item >= rot_items;
+  const int h = value ? (item - rot_items) / (D >> 3) : item / chunks, c = value ? (item - rot_items) % (D >> 3) : item % chunks;
+  if (!value && h >= Hq && !write_kv) return;
+  const T* from = row + (size_t)(value ? Hq + Hkv + h : h) * D;
+  const int o0 = value || pairing != 0 ? c * 8 : c * 16, o1 = value ? o0 : (pairing == 0 ? c * 16 + 8 : half + c * 8);
+  const uint4 r0 = *reinterpret_cast<const uint4*>(from + o0), r1 = *reinterpret_cast<const uint4*>(from + o1);
+  const int pos = positions[t];
   if (pos < 0 || pos >= n_pos) {
     if (item == 0) atomicExch(err, 2);
     return;
   }
-  T* row = qkv + (size_t)t * ld;
   T* kdst = nullptr;
   if (write_kv) {
     const int lp = pos / page_size;
@@ -506,17 +519,10 @@ rope_cache_vec_kernel(T* __restrict__ qkv, int ld, const int* __restrict__ posit
     }
     kdst = kv_plane + (size_t)page * page_stride + (size_t)(pos % page_size) * D;
   }
-  if (item >= rot_items) {  // a value chunk
-    const int w = item - rot_items, h = w / (D >> 3), c = w % (D >> 3);
-    const uint4 v = *reinterpret_cast<const uint4*>(row + (size_t)(Hq + Hkv + h) * D + c * 8);
-    *reinterpret_cast<uint4*>(kdst + (size_t)(Hkv + h) * page_size * D + c * 8) = v;
+  if (value) {
+    *reinterpret_cast<uint4*>(kdst + (size_t)(Hkv + h) * page_size * D + o0) = r0;
     return;
   }
-  const int h = item / chunks, c = item % chunks;
-  if (h >= Hq && !write_kv) return;
-  T* src = row + (size_t)h * D;
-  const int o0 = pairing == 0 ? c * 16 : c * 8, o1 = pairing == 0 ? c * 16 + 8 : half + c * 8;
-  uint4 r0 = *reinterpret_cast<const uint4*>(src + o0), r1 = *reinterpret_cast<const uint4*>(src + o1);
   const T* e0 = reinterpret_cast<const T*>(&r0);
   const T* e1 = reinterpret_cast<const T*>(&r1);
   const float4* cs4 = reinterpret_cast<const float4*>(cos_sin + ((size_t)pos * half + c * 8) * 2);
@@ -553,7 +559,7 @@ rope_cache_vec_kernel(T* __restrict__ qkv, int ld, const int* __restrict__ posit
       }
     }
   }
-  T* dst = h < Hq ? src : kdst + (size_t)(h - Hq) * page_size * D;
+  T* dst = h < Hq ? row + (size_t)h * D : kdst + (size_t)(h - Hq) * page_size * D;
   *reinterpret_cast<uint4*>(dst + o0) = w0;
   *reinterpret_cast<uint4*>(dst + o1) = w1;
 }
