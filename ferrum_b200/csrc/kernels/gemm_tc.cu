@@ -537,10 +537,11 @@ constexpr int PAIR_MAX_STAGES = PAIR_RING_BYTES / (A_BYTES + 16 * TILE_K * 2);
 // 65 x [4096, 14336] 45.1 us, 36 staged; 200 x [4096, 11008] 47.3 and 35.4, 300 x [3072, 8192] 40.1 and 28.5, 391 x [5120, 3072] 18.9 and 17.3.)
 constexpr int PAIR_OUT_ROWS = 32;
 constexpr int PAIR_OUT_BYTES = PAIR_OUT_ROWS * TILE_N * 4;
+constexpr int PAIR_THREADS = 320;      // producer, issuer, eight epilogue warps
 constexpr int PAIR_SMEM_BYTES = PAIR_RING_BYTES + 1024 + 256 + 2 * PAIR_OUT_BYTES;
 static_assert((2 * PAIR_MAX_STAGES + 5) * 8 <= 256, "the barriers do not fit their place");
 
-__global__ void __launch_bounds__(192, 1)
+__global__ void __launch_bounds__(PAIR_THREADS, 1)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                     const __grid_constant__ CUtensorMap tmap_out, const __grid_constant__ CUtensorMap tmap_ws,
                     const TcParams p) {
@@ -586,7 +587,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(acc_full_bar(b), 1);
-      mbar_init(acc_empty_bar(b), 8);  // the leader's: four epilogue warps of each CTA
+      mbar_init(acc_empty_bar(b), 16);  // the leader's: eight epilogue warps of each CTA
     }
     mbar_init(fetch_bar, 1);
     fence_barrier_init();
@@ -684,28 +685,44 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
       }
     }
   } else {
-    // ------------------------------------------------------------ epilogue (warps 2..5, both CTAs)
+    // ------------------------------------------------------------ epilogue (warps 2..9, both CTAs)
     const int quarter = warp & 3;
     const int n_local = quarter * 32 + lane;
     const int ep_tid = threadIdx.x - 64;
     const uint32_t lane_addr = tmem_base + ((uint32_t)(quarter * 32) << 16);
     const size_t tile_floats = (size_t)ACC_COLS * TILE_N;
-    uint8_t* out_stage = smem + PAIR_RING_BYTES + 256;
     const bool staged = p.out_tma != 0, floats = p.epilogue == TC_RESIDUAL || p.epilogue == TC_STORE_F32;
+    // Two groups of four warps take the 32-column pieces of a tile of 16-bit results in turn, each with half of the staging (two
+    // buffers of 32 tokens x 128 features) and a barrier of its own: what follows a tile's last product is a chain of read,
+    // stage and send for every piece, up to eight of them, and with short K it is a good part of the kernel.  float32 results need
+    // twice the staging and keep one group with both buffers (two groups with one each: 512 x [4096, 4096] 20.0 -> 21.2 us).
+    // B200, us, one group -> two: 391 x 2 x [8192, 3072] 42.5 -> 38.3, 200 x the same 34.3 -> 30.3, 391 x [5120, 3072] 17.7 -> 16.9,
+    // 512 x 2 x [8192, 3072] 47.1 -> 42.4, 1,024 x the same 83 -> 76; 391 tokens of Llama-3.2-3B 3,984 -> 3,878..3,949 (2 to 3 %).
+    // (float32 results of tiles that are cut along K pay for the wider barriers: 200 x [3072, 8192] 24.1 -> 24.9, 391 x [4096, 14336]
+    // 55.8 -> 56.8, the others the same.)
+    const int group = ep_tid >> 7, g_tid = ep_tid & 127;
+    const int piece0 = floats ? (group ? PAIR_BT : 0) : group * 32, piece_step = floats ? 32 : 64;
+    uint8_t* out_stage = smem + PAIR_RING_BYTES + 256 + (floats ? 0 : group * PAIR_OUT_BYTES);
+    bool whole_stage = false;     // 16-bit results: the last store (of a partial) reads the group's whole staging, not a half of it
+    auto group_sync = [&]() { asm volatile("bar.sync %0, 128;" ::"r"(2 + group) : "memory"); };
     int emitted = 0;  // staged stores issued so far; buffer = emitted & 1
     pdl_wait();
     // A staging buffer, once the bulk store that last used it has read it; and its way out:
     // through a tensor map (which clips at the tensor's edges), as a store or a float32 add.
-    auto stage_acquire = [&]() {
-      const int b = emitted & 1;
-      if (ep_tid == 0) bulk_wait_read<1>();
-      asm volatile("bar.sync 1, 128;" ::: "memory");
-      return out_stage + b * PAIR_OUT_BYTES;
+    auto stage_acquire = [&](bool full) {
+      const int b = floats || !full ? emitted & 1 : 0;
+      if (g_tid == 0) {
+        if (!floats && (full || whole_stage)) bulk_wait_read<0>();
+        else bulk_wait_read<1>();
+      }
+      whole_stage = full;
+      group_sync();
+      return out_stage + b * (floats ? PAIR_OUT_BYTES : PAIR_OUT_BYTES / 2);
     };
     auto stage_send = [&](uint8_t* st, const CUtensorMap* map, bool add, int x, int y) {
       fence_proxy_async();
-      asm volatile("bar.sync 1, 128;" ::: "memory");
-      if (ep_tid == 0) {
+      group_sync();
+      if (g_tid == 0) {
         if (add) tma_reduce_add_2d(map, smem_u32(st), x, y);
         else tma_store_2d(map, smem_u32(st), x, y);
         bulk_commit();
@@ -716,7 +733,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
     // tensor map (which clips at M and N), or written by the thread itself.
     auto emit32 = [&](int t0, int c0, int n0_cta, const float (&v)[32]) {
       if (staged) {
-        uint8_t* stage = stage_acquire();
+        uint8_t* stage = stage_acquire(floats);
         if (floats) {
           float* st = (float*)stage;
 #pragma unroll
@@ -744,7 +761,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
     // values of 16 tokens, and the tile leaves as 32 tokens x 64 features of bfloat16.
     auto emit32_gated = [&](int t0, int c0, int n0_cta, const float (&v)[32]) {
       const int odd = lane & 1;
-      uint8_t* stage = stage_acquire();
+      uint8_t* stage = stage_acquire(false);
       uint16_t* st = (uint16_t*)stage + (odd * 16) * (TILE_N / 2) + (n_local >> 1);
       const bool half = p.half != 0;
 #pragma unroll
@@ -763,7 +780,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
       const int buf = seg & 1, use = seg >> 1;
       bool ok = mbar_wait(acc_full_bar(buf), use & 1, abort_p, wait_limit);
       if (!ok) abort_flag = 1;
-      asm volatile("bar.sync 1, 128;" ::: "memory");
+      asm volatile("bar.sync 1, 256;" ::: "memory");
       if (abort_flag) {
         if (ep_tid == 0) atomicExch(p.err, 12);
         break;
@@ -781,7 +798,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         float* out = (float*)p.out + (size_t)t0 * p.ldo + n;
         const size_t ld = (size_t)p.ldo;
 #pragma unroll 1
-        for (int c0 = 0; c0 < bt; c0 += 32) {
+        for (int c0 = group * 32; c0 < bt; c0 += 64) {
           const int valid = n < p.N ? p.M - t0 - c0 : 0;
           float r[32], v[32];
 #pragma unroll
@@ -797,7 +814,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         if (lane == 0) mbar_arrive_cluster(leader_acc_empty);
       } else if (whole && p.gated) {
 #pragma unroll 1
-        for (int c0 = 0; c0 < bt && t0 + c0 < p.M; c0 += 32) {
+        for (int c0 = piece0; c0 < bt && t0 + c0 < p.M; c0 += piece_step) {
           float v[32];
           tmem_ld16(acc_addr + c0, &v[0]);
           tmem_ld16(acc_addr + c0 + 16, &v[16]);
@@ -808,7 +825,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         if (lane == 0) mbar_arrive_cluster(leader_acc_empty);
       } else if (whole) {
 #pragma unroll 1
-        for (int c0 = 0; c0 < bt && t0 + c0 < p.M; c0 += 32) {
+        for (int c0 = piece0; c0 < bt && t0 + c0 < p.M; c0 += piece_step) {
           float v[32];
           tmem_ld16(acc_addr + c0, &v[0]);
           tmem_ld16(acc_addr + c0 + 16, &v[16]);
@@ -843,10 +860,10 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
               while (ld_acquire_gpu(counter) != others && ++polls < PAIR_FINISHER_POLLS && !*abort_p) __nanosleep(100);
               is_last = polls < PAIR_FINISHER_POLLS && !*abort_p;
             }
-            asm volatile("bar.sync 1, 128;" ::: "memory");
+            asm volatile("bar.sync 1, 256;" ::: "memory");
           }
           const bool fast = finisher && is_last;
-          asm volatile("bar.sync 1, 128;" ::: "memory");
+          asm volatile("bar.sync 1, 256;" ::: "memory");
           if (fast) {
             const float* fetched = (const float*)smem;  // [contributor][column][128 rows]
             bool fine = true;
@@ -866,14 +883,14 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
               fine = mbar_wait(fetch_bar, fetch_phase, abort_p, wait_limit);
               fetch_phase ^= 1;
               if (!fine) abort_flag = 1;
-              asm volatile("bar.sync 1, 128;" ::: "memory");
+              asm volatile("bar.sync 1, 256;" ::: "memory");
               if (abort_flag) {
                 if (ep_tid == 0) atomicExch(p.err, 14);
                 fine = false;
                 break;
               }
 #pragma unroll 1
-              for (int c0 = cb; c0 < cb + ncols && t0 + c0 < p.M; c0 += 32) {
+              for (int c0 = cb + piece0; c0 < cb + ncols && t0 + c0 < p.M; c0 += piece_step) {
                 float v[32];
                 tmem_ld16(acc_addr + c0, &v[0]);
                 tmem_ld16(acc_addr + c0 + 16, &v[16]);
@@ -885,7 +902,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                 if (p.gated) emit32_gated(t0, c0, n0, v);
                 else emit32(t0, c0, n0, v);
               }
-              asm volatile("bar.sync 1, 128;" ::: "memory");  // all have read the stages before the next copies land
+              asm volatile("bar.sync 1, 256;" ::: "memory");  // all have read the stages before the next copies land
             }
             tc_fence_before();
             __syncwarp();
@@ -898,19 +915,19 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
           // the partial leaves like the output: 32 columns at a time through shared memory, as bulk
           // stores into the workspace seen as rows of 128 floats
 #pragma unroll 1
-          for (int c0 = 0; c0 < bt; c0 += 32) {
+          for (int c0 = piece0; c0 < bt; c0 += piece_step) {
             float v[32];
             tmem_ld16(acc_addr + c0, &v[0]);
             tmem_ld16(acc_addr + c0 + 16, &v[16]);
-            float* st = (float*)stage_acquire();
+            float* st = (float*)stage_acquire(true);
 #pragma unroll
             for (int j = 0; j < 32; ++j) st[j * TILE_N + n_local] = v[j];
             stage_send((uint8_t*)st, &tmap_ws, false, 0, (int)(my_slot * ACC_COLS) + c0);
           }
-          if (ep_tid == 0) bulk_wait_all();  // the partial is written before it is announced
+          if (g_tid == 0) bulk_wait_all();  // the partial is written before it is announced
         } else {
 #pragma unroll 1
-          for (int c0 = 0; c0 < bt; c0 += 16) {
+          for (int c0 = group * 16; c0 < bt; c0 += 32) {
             float v[16];
             tmem_ld16(acc_addr + c0, v);
 #pragma unroll
@@ -921,23 +938,23 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster(leader_acc_empty);
         __threadfence();
-        asm volatile("bar.sync 1, 128;" ::: "memory");
+        asm volatile("bar.sync 1, 256;" ::: "memory");
         if (ep_tid == 0) {
           const int old = atomicAdd(counter, 1);
           is_last = old == n_contrib - 1;
           if (is_last) *counter = 0;
         }
-        asm volatile("bar.sync 1, 128;" ::: "memory");
+        asm volatile("bar.sync 1, 256;" ::: "memory");
         if (is_last && staged) {
           // The last arriver adds the partials in K order.  A thread takes four neighbouring
           // features of eight columns, two contributors at a time: 16-byte loads, 16 of them in
           // flight per thread (with one load of 4 bytes per feature and column this reduction,
           // not the products, set the time of a product of a few hundred tokens).
           __threadfence();
-          const int q4 = (ep_tid & 31) * 4, cg = (ep_tid >> 5) * 8;
+          const int q4 = (g_tid & 31) * 4, cg = (g_tid >> 5) * 8;
           auto slot_of = [&](int cc) { return ((size_t)cc * 2 + sched.slot_of(cc, tile)) * 2 + rank; };
 #pragma unroll 1
-          for (int c0 = 0; c0 < bt && t0 + c0 < p.M; c0 += 32) {
+          for (int c0 = piece0; c0 < bt && t0 + c0 < p.M; c0 += piece_step) {
             float4 acc[8];
 #pragma unroll
             for (int k = 0; k < 8; ++k) acc[k] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -958,7 +975,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                 acc[k].x += vb[k].x; acc[k].y += vb[k].y; acc[k].z += vb[k].z; acc[k].w += vb[k].w;
               }
             }
-            uint8_t* stage = stage_acquire();
+            uint8_t* stage = stage_acquire(floats);
             if (p.gated) {  // four neighbouring rows are two (gate, up) pairs
 #pragma unroll
               for (int k = 0; k < 8; ++k) {
@@ -982,10 +999,10 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             }
             stage_send(stage, &tmap_out, p.epilogue == TC_RESIDUAL, n0, t0 + c0);
           }
-        } else if (is_last) {  // the same for the four warps: they go through emit32 together
+        } else if (is_last) {  // the same: a group's warps go through emit32 together
           __threadfence();
 #pragma unroll 1
-          for (int c0 = 0; c0 < bt && t0 + c0 < p.M; c0 += 32) {
+          for (int c0 = piece0; c0 < bt && t0 + c0 < p.M; c0 += piece_step) {
             float a0[32];
 #pragma unroll
             for (int j = 0; j < 32; ++j) a0[j] = 0.f;
@@ -1000,7 +1017,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         }
       }
     }
-    if (staged && ep_tid == 0) bulk_wait_all();  // shared memory and `out` are settled before the CTA leaves
+    if (staged && g_tid == 0) bulk_wait_all();  // shared memory and `out` are settled before the CTA leaves
     tc_fence_before();
   }
 
@@ -1147,7 +1164,7 @@ static int launch_tc_pair(const CUtensorMap& mw, const CUtensorMap& mx, const CU
   }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(n_ctas);
-  cfg.blockDim = dim3(192);
+  cfg.blockDim = dim3(PAIR_THREADS);
   cfg.dynamicSmemBytes = PAIR_SMEM_BYTES;
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
