@@ -330,6 +330,13 @@ FERRUM_API int ferrum_bias_glu_reduce(const float* bias_gate, const float* bias_
 // product still in partials (deferred mode), summed while it is read.  The block of a
 // portion's last token also copies the staged row of its request into the state.
 __device__ __forceinline__ float gb_sigmoid(float z) { return 1.0f / (1.0f + expf(-z)); }
+// One element of it.  Which products are fused into sums is written out: left to the compiler, the two kernels below
+// rounded differently, and a token's bits depended on how many others were in the step.
+__device__ __forceinline__ float gb_residual(float x, float v1, float z1, bool second, float v2, float z2) {
+  float add = __fmul_rn(v1, gb_sigmoid(z1));
+  if (second) add = __fmaf_rn(v2, gb_sigmoid(z2), add);
+  return __fadd_rn(x, add);
+}
 
 __global__ void __launch_bounds__(GB_THREADS)
 gated_residual_kernel(float* __restrict__ x, int E, const float* __restrict__ y1, int ld_y1, const float* __restrict__ g1, int ld_g1,
@@ -350,12 +357,12 @@ gated_residual_kernel(float* __restrict__ x, int E, const float* __restrict__ y1
   const int lo = blockIdx.y * per, hi = min(E, lo + per);
   for (int i = lo + threadIdx.x; i < hi; i += blockDim.x) {
     const float v1 = L1.ws != nullptr ? partial_sum(L1, tab1, t, i) : y1[(size_t)t * ld_y1 + i];
-    float add = v1 * gb_sigmoid(g1[(size_t)t * ld_g1 + i] + (c1 ? c1[i] : 0.f));
+    float v2 = 0.f, z2 = 0.f;
     if (second) {
-      const float v2 = L2.ws != nullptr ? partial_sum(L2, tab2, t, i) : y2[(size_t)t * ld_y2 + i];
-      add += (v2 + (c2 ? c2[i] : 0.f)) * gb_sigmoid(g2[(size_t)t * ld_g2 + i] + (c3 ? c3[i] : 0.f));
+      v2 = (L2.ws != nullptr ? partial_sum(L2, tab2, t, i) : y2[(size_t)t * ld_y2 + i]) + (c2 ? c2[i] : 0.f);
+      z2 = g2[(size_t)t * ld_g2 + i] + (c3 ? c3[i] : 0.f);
     }
-    xr[i] += add;
+    xr[i] = gb_residual(xr[i], v1, g1[(size_t)t * ld_g1 + i] + (c1 ? c1[i] : 0.f), second, v2, z2);
   }
   if (state != nullptr) {
     const int r = req_of_token[t];
@@ -389,11 +396,7 @@ gated_residual_vec_kernel(float* __restrict__ x, int E, const float* __restrict_
     const float b2s[4] = {b2.x, b2.y, b2.z, b2.w}, b3s[4] = {b3.x, b3.y, b3.z, b3.w};
     float o[4];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      float add = v1s[k] * gb_sigmoid(z1s[k] + b1s[k]);
-      if (y2r != nullptr) add += (v2s[k] + b2s[k]) * gb_sigmoid(z2s[k] + b3s[k]);
-      o[k] = xs[k] + add;
-    }
+    for (int k = 0; k < 4; ++k) o[k] = gb_residual(xs[k], v1s[k], z1s[k] + b1s[k], y2r != nullptr, v2s[k] + b2s[k], z2s[k] + b3s[k]);
     gb_store4<float>(xr + i, o[0], o[1], o[2], o[3]);
   }
   if (state != nullptr) {

@@ -58,6 +58,36 @@ def test_gated_residual_widths(cuda, T, E, pad, second):
     assert not state[[0, 2, 4]].any()
 
 
+@pytest.mark.parametrize("E", [20, 1028, 2048])
+@pytest.mark.parametrize("second", [True, False])
+@pytest.mark.parametrize("biased", [True, False])
+def test_gated_residual_of_64_and_65_tokens(cuda, E, second, biased):
+    """A token's bits do not depend on how many others are in the step, and are those of sums whose only fused product is
+    the second one."""
+    from ferrum_b200.ops import lib as ops
+    g = torch.Generator(device="cuda").manual_seed(E)
+    x, y1, y2, g1, g2 = (rand(g, 65, E) for _ in range(5))
+    c1, c2, c3 = (rand(g, E) if biased else None for _ in range(3))
+
+    def run(n, rows, v1=y1, v2=y2):
+        out = rows[:n].clone()
+        ops.gated_residual(out, n, v1, g1, c1, *((v2, c2, g2, c3) if second else ()))
+        return out
+
+    few, many = run(64, x), run(65, x)
+    assert torch.equal(few, many[:64])
+    zero, one = torch.zeros_like(x), torch.ones_like(x)
+    s1 = zero.clone()
+    ops.gated_residual(s1, 65, one, g1, c1)         # 0 + 1 * sigmoid: the sigmoid's own bits
+    add = y1 * s1
+    if second:
+        s2 = zero.clone()
+        ops.gated_residual(s2, 65, one, g2, c3)
+        # the exact product of two float32, rounded once with the sum (in float64: a second rounding shows in one of 2^28)
+        add = ((y2 + c2 if biased else y2).double() * s2.double() + add.double()).float()
+    assert (many != x + add).float().mean() < 1e-5
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("E,groups", [(24, 8), (32, 8), (36, 9), (1020, 1), (1024, 2), (1032, 2), (2048, 8), (4112, 1)])
 def test_norm_pair_shift_widths(cuda, dtype, E, groups):
