@@ -278,7 +278,7 @@ FERRUM_API int ferrum_rmsnorm(const float* x, const float* w, void* out, int out
   if (E % 4 == 0 && E >= 512 && E <= 4 * NORM_VEC_MAX * 512 && ((uintptr_t)x & 15) == 0 && ((uintptr_t)w & 15) == 0 &&
       ((uintptr_t)out & 15) == 0) {
     const int n4 = E / 4;
-    const int vthreads = n4 >= 2048 ? 512 : (n4 >= 512 ? 256 : 128);
+    const int vthreads = n4 > 256 * NORM_VEC_MAX ? 512 : (n4 >= 512 ? 256 : 128);      // (a row fits its block's registers)
     FERRUM_DISPATCH_DTYPE(out_dtype, T, launch_kernel(rmsnorm_vec_kernel<T>, n_rows, vthreads, 0, stream, x, w, (T*)out, rows, E, eps));
     FERRUM_CHECK_LAUNCH("rmsnorm");
     return 0;

@@ -43,3 +43,19 @@ def test_float32_rotary_rows_do_not_depend_on_the_grid(cuda, T, Hq, Hkv, D, R, p
 
     (a, b), (c, d) = run(T), run(64)
     assert torch.equal(a, c) and torch.equal(b, d) and err.item() == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("E", [512, 2044, 2048, 4096, 4100, 5120, 6144, 8188, 8192, 8196])
+def test_norm_of_many_rows_covers_the_width(cuda, dtype, E):
+    """Widths on both sides of every change of the block's size: all of a row is normed, nothing beside it."""
+    from ferrum_b200.ops import lib as ops
+    g = torch.Generator(device="cuda").manual_seed(E)
+    x, w = torch.randn(70, E, device="cuda", generator=g), torch.randn(E, device="cuda", generator=g)
+    out = torch.full((71, E), 7.0, device="cuda", dtype=dtype)
+    ops.rmsnorm(x, w, out, 1e-5, n_rows=70)
+    v = x.double()
+    want = v / torch.sqrt((v * v).mean(-1, keepdim=True) + 1e-5) * w.double()
+    # a sum of squares in a tree of some 20 levels, a root, a division and two products; one rounding of the output type
+    bound = want.abs() * (24 * 2.0 ** -24 + (2.0 ** -8 if dtype == torch.bfloat16 else 0.0))
+    assert ((out[:70].double() - want).abs() <= bound).all() and (out[70] == 7).all()
