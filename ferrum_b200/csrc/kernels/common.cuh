@@ -38,8 +38,12 @@ void ferrum_set_error(const char* fmt, ...);
 // are visible; nothing that an earlier kernel of the stream writes may be read, and nothing it
 // reads may be written, before it.  pdl_launch() lets the next kernel of the stream begin its
 // own prologue.  In a kernel launched the ordinary way both are no-ops.
+// Weights before pdl_wait(): a kernel may ask the L2 for them (prefetch_l2: no value reaches the kernel).  The tensor-core products
+// and dyn_tanh go further and read them, so their weights must be settled when they are launched: written by a copy, or by a kernel
+// that was launched the ordinary way and has another such kernel, a copy or a synchronisation behind it.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
 bool ferrum_dependent_launch_enabled();
 

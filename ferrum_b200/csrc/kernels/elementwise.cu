@@ -107,18 +107,19 @@ rmsnorm_vec_kernel(const float* __restrict__ x, const float* __restrict__ w, TOu
   __shared__ float red[32];
   const int n4 = E >> 2;
   const float4* w4 = reinterpret_cast<const float4*>(w);
-  float4 g4[NORM_VEC_MAX];      // (the weights never change: they come while the kernel ahead of this one ends)
+  if (blockIdx.x == 0)          // (the weights start for the L2 while the kernel ahead of this one ends)
+    for (int i = threadIdx.x * 8; i < n4; i += blockDim.x * 8) prefetch_l2(w4 + i);
+  pdl_launch();
+  pdl_wait();
+  const int r = blockIdx.x;
+  const float4* xr = reinterpret_cast<const float4*>(x + (size_t)(rows ? rows[r] : r) * E);
+  float4 v[NORM_VEC_MAX], g4[NORM_VEC_MAX];
+  float ss = 0.f;
 #pragma unroll
   for (int k = 0; k < NORM_VEC_MAX; ++k) {
     const int i = threadIdx.x + k * blockDim.x;
     g4[k] = i < n4 ? __ldg(w4 + i) : make_float4(0.f, 0.f, 0.f, 0.f);
   }
-  pdl_launch();
-  pdl_wait();
-  const int r = blockIdx.x;
-  const float4* xr = reinterpret_cast<const float4*>(x + (size_t)(rows ? rows[r] : r) * E);
-  float4 v[NORM_VEC_MAX];
-  float ss = 0.f;
 #pragma unroll
   for (int k = 0; k < NORM_VEC_MAX; ++k) {
     const int i = threadIdx.x + k * blockDim.x;
@@ -185,21 +186,22 @@ rmsnorm_cluster_kernel(float* __restrict__ h, const float* __restrict__ w, TOut*
   const unsigned rank = norm_cluster_rank();
   const int per = (E + NORM_CLUSTER - 1) / NORM_CLUSTER;
   const int lo = rank * per, hi = min(E, lo + per);
-  // The norm's weights never change: they come while the kernel ahead of this one ends, not behind the cluster's sum.
-  // (B200, decode step of Llama-3.1-8B with 65 such norms: 3,289 -> 3,257 us with one token, 4,597 -> 4,589 with 8.)
-  float wk[NORM_KEEP];
-#pragma unroll
-  for (int k = 0; k < NORM_KEEP; ++k) {
-    const int i = lo + threadIdx.x + k * 256;
-    wk[k] = i < hi ? __ldg(w + i) : 0.f;
-  }
+  // The norm's weights start for the L2 while the kernel ahead of this one ends, and are read first thing after it, not behind the
+  // cluster's sum.  (B200, decode step of Llama-3.1-8B with 65 such norms, read behind the sum -> so: 3,283 -> 3,252 us with one token,
+  // 4,609 -> 4,604 with 8, 5,402 -> 5,386 with 64; read between the row's own loads 3,261.)
+  for (int i = lo + threadIdx.x * 32; i < hi; i += 256 * 32) prefetch_l2(w + i);
   pdl_launch();
   pdl_wait();
   TRACE_MARK(TRACE_WAITED);
   const int src = rows ? rows[r] : r;
   float* hr = h + (size_t)src * E;
-  float keep[NORM_KEEP];
+  float keep[NORM_KEEP], wk[NORM_KEEP];
   float ss = 0.f;
+#pragma unroll
+  for (int k = 0; k < NORM_KEEP; ++k) {
+    const int i = lo + threadIdx.x + k * 256;
+    wk[k] = i < hi ? __ldg(w + i) : 0.f;
+  }
 #pragma unroll
   for (int k = 0; k < NORM_KEEP; ++k) {
     const int i = lo + threadIdx.x + k * 256;

@@ -410,7 +410,7 @@ gemm_stream4_kernel(const float* __restrict__ x, const float* __restrict__ w, vo
     for (int i = 0; i < S4_STAGES && q.g < n_groups; ++i) {
       const int k = q.s * ST_KT + tid * 4;
       if ((tid & 7) == 0 && k < K)
-        for (int f = 0; f < q.nf; ++f) asm volatile("prefetch.global.L2 [%0];" ::"l"(w + (size_t)(q.n0 + f) * ldw + k));
+        for (int f = 0; f < q.nf; ++f) prefetch_l2(w + (size_t)(q.n0 + f) * ldw + k);
       advance(q);
     }
   }

@@ -239,13 +239,15 @@ mamba_gate_norm_kernel(const float* __restrict__ y, int inner, const float* __re
   const float* yr = y + (size_t)t * inner + (size_t)grp * width;
   const float* zr = proj + (size_t)t * ldp + off_z + (size_t)grp * width;
   const float* wr = w + (size_t)grp * width;
+  if (t == 0)          // (the weights start for the L2 while the kernel ahead of this one ends)
+    for (int i = threadIdx.x * 32; i < width; i += 256 * 32) prefetch_l2(wr + i);
+  pdl_wait();
   float keep[GN_KEEP], wk[GN_KEEP];
 #pragma unroll
-  for (int k = 0; k < GN_KEEP; ++k) {      // (the weights never change: they come while the kernel ahead of this one ends)
+  for (int k = 0; k < GN_KEEP; ++k) {
     const int i = threadIdx.x + k * 256;
     wk[k] = i < width ? wr[i] : 0.f;
   }
-  pdl_wait();
   float ss = 0.f;
   {
     float yv[GN_KEEP], zv[GN_KEEP];

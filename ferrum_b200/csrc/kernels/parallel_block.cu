@@ -105,7 +105,7 @@ norm_scaled_add_kernel(float* __restrict__ x, const float* __restrict__ y, const
 
 // Rows of E = 4 * (pieces) elements, at most PB_PIECES pieces a thread, kept in registers from the read to the last store.
 // A step of a few tokens is a chain of such kernels: each is launched behind the one before it in dependent mode, and both norms'
-// weights are on their way before it waits.  (B200, 8 tokens of the hybrid model with 4 layers, this and the kernels of
+// weights are on their way to the L2 before it waits.  (B200, 8 tokens of the hybrid model with 4 layers, this and the kernels of
 // mamba2.cu, attention_prep.cu, attention_generic.cu and thin_linear.cu: a step 372 -> 350 us.)
 constexpr int PB_PIECES = 4;
 template <typename T>
@@ -117,17 +117,13 @@ norm_scaled_add_vec_kernel(float* __restrict__ x, const float* __restrict__ y, c
   __shared__ PartialTable tab;
   if (L.ws != nullptr) build_partial_table(L, tab);
   const int t = blockIdx.x, n4 = E >> 2;
-  float4 v[PB_PIECES], xo[PB_PIECES], wg[PB_PIECES], wg2[PB_PIECES];
-#pragma unroll
-  for (int k = 0; k < PB_PIECES; ++k) {      // (the weights never change: they come while the kernel ahead of this one ends)
-    const int i = threadIdx.x + k * blockDim.x;
-    wg[k] = wg2[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (i < n4) {
-      wg[k] = *reinterpret_cast<const float4*>(w + 4 * i);
-      if (out != nullptr) wg2[k] = *reinterpret_cast<const float4*>(w2 + 4 * i);
+  if (blockIdx.x == 0)          // (the weights start for the L2 while the kernel ahead of this one ends)
+    for (int i = threadIdx.x * 8; i < n4; i += blockDim.x * 8) {
+      prefetch_l2(w + 4 * i);
+      if (out != nullptr) prefetch_l2(w2 + 4 * i);
     }
-  }
   pdl_wait();
+  float4 v[PB_PIECES], xo[PB_PIECES];
   float ss = 0.f;
 #pragma unroll
   for (int k = 0; k < PB_PIECES; ++k) {
@@ -153,7 +149,7 @@ norm_scaled_add_vec_kernel(float* __restrict__ x, const float* __restrict__ y, c
   for (int k = 0; k < PB_PIECES; ++k) {
     const int i = threadIdx.x + k * blockDim.x;
     if (i >= n4) continue;
-    const float4 g = wg[k];
+    const float4 g = *reinterpret_cast<const float4*>(w + 4 * i);
     xo[k].x = fmaf(mult, v[k].x * r * g.x, xo[k].x);
     xo[k].y = fmaf(mult, v[k].y * r * g.y, xo[k].y);
     xo[k].z = fmaf(mult, v[k].z * r * g.z, xo[k].z);
@@ -171,7 +167,7 @@ norm_scaled_add_vec_kernel(float* __restrict__ x, const float* __restrict__ y, c
   for (int k = 0; k < PB_PIECES; ++k) {
     const int i = threadIdx.x + k * blockDim.x;
     if (i >= n4) continue;
-    const float4 g = wg2[k];
+    const float4 g = *reinterpret_cast<const float4*>(w2 + 4 * i);
     const float a = xo[k].x * r2 * g.x, b = xo[k].y * r2 * g.y, c = xo[k].z * r2 * g.z, d = xo[k].w * r2 * g.w;
     if constexpr (sizeof(T) == 4) {
       *reinterpret_cast<float4*>(out + (size_t)t * E + 4 * i) = make_float4(a, b, c, d);

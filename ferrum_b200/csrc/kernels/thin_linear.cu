@@ -48,7 +48,7 @@ thin_linear_kernel(const T* __restrict__ x, int ldx, const T* __restrict__ w, in
   // The weights never change: they start for the L2 while the kernel ahead of this one ends.
   for (int k = tid * 8; k < K; k += TL_THREADS * 8)
 #pragma unroll
-    for (int j = 0; j < NF; ++j) asm volatile("prefetch.global.L2 [%0];" ::"l"(wr[j] + k));
+    for (int j = 0; j < NF; ++j) prefetch_l2(wr[j] + k);
   pdl_wait();
   for (int k = tid * 8; k < K; k += TL_THREADS * 8) {
     uint4 xraw[TL_TOKENS];

@@ -565,7 +565,8 @@ def gemm_tc(x, w, out, epilogue, err, workspace, counters, M=None, N=None, dual_
     output features (rows of w used per product); with dual_offset > 0 rows dual_offset + n
     feed the second product of the SwiGLU epilogue.  `workspace` (float32) and `counters`
     (int32, all zero) are scratch for tiles that several CTAs share; n_ctas = 0 means one CTA
-    per SM."""
+    per SM.  The weights must be settled before the call: they are read while the kernel ahead of this
+    one still runs (as are those of the other tensor-core products and of `dyn_tanh`; other kernels wait)."""
     _need16(x, "x", 2); _need16(w, "w", 2, like=x); _need(out, None, "out", 2)
     M = x.shape[0] if M is None else M
     K = w.shape[1]

@@ -1,0 +1,82 @@
+"""Kernels in dependent launches read nothing that the kernel ahead of them may write before they have waited for it: the sources, on
+the CPU, and weights that the kernel directly ahead writes, on the GPU."""
+import glob
+import os
+import re
+
+import pytest
+import torch
+
+KERNELS = os.path.join(os.path.dirname(os.path.abspath(__file__)), "..", "ferrum_b200", "csrc", "kernels")
+# These read settled weights, or the plan that copies have brought, early; common.cuh says so.
+EARLY = {"dyn_tanh_kernel", "dyn_tanh_vec_kernel", "combine_kernel"}
+
+
+def kernels():
+    """(file, kernel, pointer parameters, text before the first wait) of every kernel that waits."""
+    for path in sorted(glob.glob(os.path.join(KERNELS, "*.cu"))):
+        text = re.sub(r"//[^\n]*", "", open(path).read())
+        for m in re.finditer(r"(\w+_kernel)\s*\(([^{};]*?)\)\s*\{", text):
+            body = text[m.end():closing(text, m.end())]
+            if "pdl_wait()" in body:
+                pointers = re.findall(r"\*\s*(?:__restrict__\s+)?(\w+)\s*(?:,|$)", m.group(2))
+                yield os.path.basename(path), m.group(1), pointers, body[:body.index("pdl_wait()")]
+
+
+def closing(text, begin):
+    """The place behind the brace that closes the one before `begin`."""
+    depth = 1
+    while depth:
+        depth += {"{": 1, "}": -1}.get(text[begin], 0)
+        begin += 1
+    return begin
+
+
+def reads(pointers, text):
+    """The statements that load through a pointer parameter, or through a variable that was made of one."""
+    names, found = set(pointers), []
+    while m := re.search(r"\[&\]\s*\([^()]*(?:\([^()]*\)[^()]*)*\)\s*\{", text):       # a lambda: what it does is done where it is called
+        text = text[:m.start()] + text[closing(text, m.end()):]
+    for statement in re.split(r"[;{}]", text):
+        named = [n for n in names if re.search(rf"\b{n}\b", statement)]
+        if any(re.search(rf"(?<![&\w]){n}\s*\[", statement) or re.search(rf"(?<![\w)\]])\*\s*{n}\b(?!\s*=)", statement) or
+               re.search(rf"(__ldg|__ldcg)\s*\([^;]*\b{n}\b", statement) or
+               re.search(rf"\*\s*reinterpret_cast<[^>]*>\s*\(\s*{n}\b", statement) for n in named) and "prefetch_l2" not in statement:
+            found.append(statement.strip())
+        made = re.search(r"\*\s*(?:const\s+|__restrict__\s+)?(\w+)(?:\[\w+\])?\s*=", statement)
+        if made and named:
+            names.add(made.group(1))
+    return found
+
+
+def test_nothing_is_read_before_the_wait():
+    seen, wrong = set(), []
+    for file, kernel, pointers, before in kernels():
+        seen.add(kernel)
+        if kernel not in EARLY:
+            wrong += [f"{file}: {kernel}: {s}" for s in reads(pointers, before)]
+    assert {"rmsnorm_vec_kernel", "rmsnorm_cluster_kernel", "norm_scaled_add_vec_kernel", "mamba_gate_norm_kernel", "thin_linear_kernel"} <= seen
+    assert not wrong, wrong
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows", [1, 8, 64, 65, 300])
+def test_norm_weights_that_the_kernel_ahead_writes(cuda, rows):
+    from ferrum_b200.ops import lib as ops
+    E = 4096
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    x, y = torch.randn(rows, E, device="cuda", generator=g), torch.randn(rows, E, device="cuda", generator=g)
+    w, out = torch.empty(E, device="cuda"), torch.empty(rows, E, device="cuda")
+
+    def norm(v):
+        v = v.double()
+        return v / torch.sqrt((v * v).mean(-1, keepdim=True) + 1e-5)
+
+    for i in range(1, 9):
+        w.fill_(float(i))
+        ops.rmsnorm(x, w, out, 1e-5)
+        assert ((out.double() - i * norm(x)).abs() <= i * norm(x).abs() * 24 * 2.0 ** -24).all()
+        s = x.clone()
+        w.fill_(float(-i))
+        ops.norm_scaled_add(s, y, w, 1.0, 1e-5, rows)
+        assert ((s.double() - (x.double() - i * norm(y))).abs() <= (x.abs() + i * norm(y).abs()) * 24 * 2.0 ** -24).all()
