@@ -17,7 +17,8 @@
 //                    root mean square and multiplied by the weight; out in the compute type.
 #include "common.cuh"
 
-constexpr int MS_TC = 32;        // tokens per chunk that the walk stages in shared memory (4 when no request brings more)
+constexpr int MS_TC = 32;        // tokens per chunk that the walk stages in shared memory ...
+constexpr int MS_STEP_TOKENS = 4;   // ... and when no request brings more than these
 constexpr int MS_WARPS = 8;      // warps of the walk's block: each owns an eighth of a head's state elements
 constexpr int MS_MAX_TAPS = 16;
 
@@ -50,8 +51,8 @@ mamba_conv_kernel(const float* __restrict__ proj, int ldp, int off_xbc, int C, i
 __global__ void __launch_bounds__(256)
 mamba_conv_state_kernel(const float* __restrict__ proj, int ldp, int off_xbc, int C, int taps, float* __restrict__ state,
                         long long state_stride, long long conv_off, const int* __restrict__ q_start,
-                        const int* __restrict__ slots, int n_reqs) {
-  pdl_launch();
+                        const int* __restrict__ slots, int n_reqs, int early) {
+  if (early) pdl_launch();
   pdl_wait();
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (long long)n_reqs * C) return;
@@ -306,8 +307,12 @@ FERRUM_API int ferrum_mamba2_mix(const float* proj, int ldp, int n_tokens, int n
   }
   if (taps > 1) {
     const long long n = (long long)n_reqs * C;
+    // The walk's blocks may come early only in a step of a few tokens.  Over a portion a block of it holds half of an SM's shared memory
+    // for all of the walk, and those that come while the convolution's blocks still fill most SMs share the few that are free, two by
+    // two.  (B200, 64 heads of 64 x 128, the whole mixer, us, early -> not: 128 tokens 43.9 -> 33.6, 300 92 -> 69, 1,000 292 -> 220,
+    // 2,048 592 -> 449; 8 requests of one token 15.8 -> 15.9.)
     launch_kernel(mamba_conv_state_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, stream, proj, ldp, off_xbc, C, taps, state, state_stride,
-                                                                            conv_off, q_start, slots, n_reqs);
+                                                                            conv_off, q_start, slots, n_reqs, (int)(max_q_len <= MS_STEP_TOKENS));
     FERRUM_CHECK_LAUNCH("mamba_conv_state");
   }
   {
@@ -329,7 +334,7 @@ FERRUM_API int ferrum_mamba2_mix(const float* proj, int ldp, int n_tokens, int n
   } while (0)
 #define MS_SCAN(NQ_)                  \
   do {                                \
-    if (max_q_len <= 4) MS_SCAN2(NQ_, 4); \
+    if (max_q_len <= MS_STEP_TOKENS) MS_SCAN2(NQ_, MS_STEP_TOKENS); \
     else MS_SCAN2(NQ_, MS_TC);        \
   } while (0)
     if (N <= 32) MS_SCAN(4);
