@@ -508,8 +508,12 @@ static int launch_generic(const void* x, const void* w, void* out, int M, int N,
   const T* wp = (const T*)w;
   if constexpr (sizeof(T) == 4) {
     if (vec && M <= S4_TOK) {
-      static const cudaError_t e4 = cudaFuncSetAttribute(gemm_stream4_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S4_SMEM_BYTES);
-      FERRUM_CHECK_ARG(e4 == cudaSuccess, "gemm: cannot reserve %d bytes of shared memory: %s", S4_SMEM_BYTES, cudaGetErrorString(e4));
+      static bool configured = false;
+      if (!configured) {
+        cudaError_t e = cudaFuncSetAttribute(gemm_stream4_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S4_SMEM_BYTES);
+        FERRUM_CHECK_ARG(e == cudaSuccess, "gemm: cannot reserve %d bytes of shared memory: %s", S4_SMEM_BYTES, cudaGetErrorString(e));
+        configured = true;
+      }
       const int ctas = std::min((N + 3) / 4, S4_CTAS_PER_SM * stream_sm_count());      // (every CTA has a feature)
       launch_kernel(gemm_stream4_kernel, dim3(ctas), dim3(S4_THREADS), S4_SMEM_BYTES, stream, (const float*)x, (const float*)w, out, M, N, K,
                     ldx, ldw, ldo, epilogue);
