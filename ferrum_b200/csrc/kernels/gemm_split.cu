@@ -685,8 +685,12 @@ FERRUM_API int ferrum_gemm_split(const float* x, const float* w, float* out, int
   FERRUM_CHECK_ARG(need[1] == 0 || (partials && partial_floats >= need[1]), "gemm_split: needs %lld floats for partial sums, got %lld", need[1], partial_floats);
   FERRUM_CHECK_ARG(((uintptr_t)partials & 15) == 0, "gemm_split: the partial sums must be 16-byte aligned");
   FERRUM_CHECK_ARG((long long)s.tiles_n * s.tiles_t * s.splits < (1LL << 30) && 3LL * M < (1LL << 31), "gemm_split: too many tiles");
-  static const cudaError_t configured = cudaFuncSetAttribute(gemm_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GS_SMEM_BYTES);
-  FERRUM_CHECK_ARG(configured == cudaSuccess, "gemm_split: cannot reserve %d bytes of shared memory: %s", GS_SMEM_BYTES, cudaGetErrorString(configured));
+  static bool configured = false;
+  if (!configured) {
+    const cudaError_t e = cudaFuncSetAttribute(gemm_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GS_SMEM_BYTES);
+    FERRUM_CHECK_ARG(e == cudaSuccess, "gemm_split: cannot reserve %d bytes of shared memory: %s", GS_SMEM_BYTES, cudaGetErrorString(e));
+    configured = true;
+  }
   CUtensorMap mw, mx;
   if (int r = gs_tensor_map(&mw, true, w, N, K, ldw, GS_TILE_N)) return r;
   if (int r = gs_tensor_map(&mx, false, parts, 3LL * M, K, K, s.bt)) return r;
