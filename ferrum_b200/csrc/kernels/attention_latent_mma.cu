@@ -470,13 +470,7 @@ FERRUM_API int ferrum_attention_latent_mma(const void* q, int ldq, void* out, in
   // smaller grid runs stages of 64 keys (fewer barriers per key).  (Measured at 16 heads, rows of
   // 576: prompt of 2,048 tokens 559 us against 684 us with four row tiles on stages of 32 keys; 8
   // single tokens over 8,192 keys 71 against 88 us, over 2,048 keys 32 against 26 us.)
-  static int sms = 0;
-  if (sms == 0) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
-      sms = 148;
-  }
-  bool big_grid = (long long)n_tokens * hchunks * (part ? split_slots : 1) > 2LL * sms;
+  bool big_grid = (long long)n_tokens * hchunks * (part ? split_slots : 1) > 2LL * ferrum_sm_count();
   int fit64 = lm_smem(Dk, 3, 64, wide).bytes <= LM_SMEM_LIMIT ? 3 : (lm_smem(Dk, 2, 64, wide).bytes <= LM_SMEM_LIMIT ? 2 : 0);
   if (g_force_stage == 32) big_grid = true, fit64 = 0;
   if (g_force_stage == 64) big_grid = false;

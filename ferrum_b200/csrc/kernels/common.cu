@@ -24,3 +24,12 @@ FERRUM_API int ferrum_kernels_abi() { return 24; }
 static bool g_dependent_launch = true;
 bool ferrum_dependent_launch_enabled() { return g_dependent_launch; }
 FERRUM_API void ferrum_set_dependent_launch(int on) { g_dependent_launch = on != 0; }
+
+int ferrum_sm_count() {
+  static const int n = [] {
+    int dev = 0, v = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v <= 0) v = 148;
+    return v;
+  }();
+  return n;
+}

@@ -47,6 +47,9 @@ __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefe
 
 bool ferrum_dependent_launch_enabled();
 
+// Multiprocessors of the device that was current at the first call (148 where that cannot be asked).
+int ferrum_sm_count();
+
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                                  Args&&... args) {

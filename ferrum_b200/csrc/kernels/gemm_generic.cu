@@ -490,15 +490,6 @@ gemm_stream4_kernel(const float* __restrict__ x, const float* __restrict__ w, vo
   }
 }
 
-static int stream_sm_count() {
-  static const int n = [] {
-    int dev = 0, v = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v <= 0) v = 148;
-    return v;
-  }();
-  return n;
-}
-
 template <typename T>
 static int launch_generic(const void* x, const void* w, void* out, int M, int N, int K, int ldx, int ldw, int ldo,
                           int epilogue, cudaStream_t stream) {
@@ -514,7 +505,7 @@ static int launch_generic(const void* x, const void* w, void* out, int M, int N,
         FERRUM_CHECK_ARG(e == cudaSuccess, "gemm: cannot reserve %d bytes of shared memory: %s", S4_SMEM_BYTES, cudaGetErrorString(e));
         configured = true;
       }
-      const int ctas = std::min((N + 3) / 4, S4_CTAS_PER_SM * stream_sm_count());      // (every CTA has a feature)
+      const int ctas = std::min((N + 3) / 4, S4_CTAS_PER_SM * ferrum_sm_count());      // (every CTA has a feature)
       launch_kernel(gemm_stream4_kernel, dim3(ctas), dim3(S4_THREADS), S4_SMEM_BYTES, stream, (const float*)x, (const float*)w, out, M, N, K,
                     ldx, ldw, ldo, epilogue);
       FERRUM_CHECK_LAUNCH("gemm_generic");

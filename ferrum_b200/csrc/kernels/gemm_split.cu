@@ -635,15 +635,6 @@ int gs_tensor_map(CUtensorMap* out, bool f32, const void* ptr, long long rows, l
   return 0;
 }
 
-int gs_sm_count() {
-  static const int n = [] {
-    int dev = 0, v = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v <= 0) v = 148;
-    return v;
-  }();
-  return n;
-}
-
 // Ranges of K: as many as let one token tile's items fill the GPU, of 512 elements or more.  A function of N and K alone.
 int gs_splits(int N, int K) {
   const int tiles_n = (N + GS_TILE_N - 1) / GS_TILE_N;
@@ -695,16 +686,16 @@ FERRUM_API int ferrum_gemm_split(const float* x, const float* w, float* out, int
   if (int r = gs_tensor_map(&mw, true, w, N, K, ldw, GS_TILE_N)) return r;
   if (int r = gs_tensor_map(&mx, false, parts, 3LL * M, K, K, s.bt)) return r;
   const long long pieces = (long long)M * (K / 8);
-  const int blocks = (int)std::min<long long>((pieces + 255) / 256, 8LL * gs_sm_count());
+  const int blocks = (int)std::min<long long>((pieces + 255) / 256, 8LL * ferrum_sm_count());
   launch_kernel(split_rows_kernel, dim3(blocks), dim3(256), 0, stream, x, M, K, ldx, (uint16_t*)parts);
   FERRUM_CHECK_LAUNCH("split_rows");
   SplitParams p{x, w, out, partials, err_flag, M, N, K, ldx, ldw, ldo, s.bt, s.tiles_n, s.tiles_t, s.splits, add};
-  const int grid = std::min(gs_sm_count(), s.tiles_n * s.tiles_t * s.splits);
+  const int grid = std::min(ferrum_sm_count(), s.tiles_n * s.tiles_t * s.splits);
   launch_kernel(gemm_split_kernel, dim3(grid), dim3(320), GS_SMEM_BYTES, stream, mw, mx, p);
   FERRUM_CHECK_LAUNCH("gemm_split");
   if (s.splits > 1) {
     const long long quads = (long long)M * ((N + 3) / 4);
-    launch_kernel(split_sum_kernel, dim3((int)std::min<long long>((quads + 255) / 256, 8LL * gs_sm_count())), dim3(256), 0, stream, p);
+    launch_kernel(split_sum_kernel, dim3((int)std::min<long long>((quads + 255) / 256, 8LL * ferrum_sm_count())), dim3(256), 0, stream, p);
     FERRUM_CHECK_LAUNCH("split_sum");
   }
   return 0;

@@ -1182,17 +1182,6 @@ static int launch_tc_pair(const CUtensorMap& mw, const CUtensorMap& mx, const CU
   return 0;
 }
 
-static int sm_count() {
-  static int n = 0;
-  if (n == 0) {
-    int dev = 0;
-    cudaDeviceProp prop;
-    if (cudaGetDevice(&dev) == cudaSuccess && cudaGetDeviceProperties(&prop, dev) == cudaSuccess) n = prop.multiProcessorCount;
-    if (n <= 0) n = 148;
-  }
-  return n;
-}
-
 // How the pair kernel cuts M tokens x `rows` weight rows over K among `pairs` pairs: the width of its token tiles, and
 // whether left-over tiles are cut along K.  256 tokens a tile is the cheapest per token, but a step of a few hundred
 // tokens has too few such tiles for the pairs (12 tiles of [3072, K] on 74 pairs), or a last wave that is nearly empty.
@@ -1258,7 +1247,7 @@ FERRUM_API int ferrum_gemm_tc_token_tile(int M, int dual) {
 }
 
 // The grid the kernel runs with when the caller passes n_ctas = 0: one CTA per SM.
-FERRUM_API int ferrum_gemm_tc_default_ctas() { return sm_count(); }
+FERRUM_API int ferrum_gemm_tc_default_ctas() { return ferrum_sm_count(); }
 
 // The single-CTA kernel's counters: one per 128-row tile (rounded up to pairs of them).
 static long long single_cta_tiles(int M, int N, int bt) { return 2LL * ((N + 2 * TILE_N - 1) / (2 * TILE_N)) * ((M + bt - 1) / bt); }
@@ -1268,7 +1257,7 @@ static long long single_cta_floats(int bt, int dual, int n_ctas) { return 2LL * 
 // range of units begins or ends inside a tile, so every CTA has two partial slots.
 FERRUM_API long long ferrum_gemm_tc_workspace(int M, int N, int K, int dual, int n_ctas, int* n_tiles) {
   const int bt = ferrum_gemm_tc_token_tile(M, dual);
-  if (n_ctas <= 0) n_ctas = sm_count();
+  if (n_ctas <= 0) n_ctas = ferrum_sm_count();
   long long tiles = single_cta_tiles(M, N, bt);
   const bool pair = M >= PAIR_MIN_TOKENS && n_ctas >= 2;
   if (pair) {
@@ -1305,7 +1294,7 @@ FERRUM_API int ferrum_gemm_tc(const void* x, const void* w, void* out, int dtype
   FERRUM_CHECK_ARG(dual == (epilogue == TC_SWIGLU), "gemm_tc: the SwiGLU epilogue needs dual_offset, and only it does");
   FERRUM_CHECK_ARG(epilogue >= 0 && epilogue <= 3, "gemm_tc: unknown epilogue %d", epilogue);
   FERRUM_CHECK_ARG(w_rows >= N + dual_offset, "gemm_tc: w has %d rows, needs %d", w_rows, N + dual_offset);
-  if (n_ctas <= 0) n_ctas = sm_count();
+  if (n_ctas <= 0) n_ctas = ferrum_sm_count();
   const int bt = ferrum_gemm_tc_token_tile(M, dual);
   int tiles = 0;
   const long long need = ferrum_gemm_tc_workspace(M, N, K, dual, n_ctas, &tiles);
@@ -1445,7 +1434,7 @@ FERRUM_API int ferrum_gemm_pair_launch_schedule(int M, long long rows, int K, in
 // partial_sum() of partials.cuh.  Requirements: one token tile (M <= 256, or 128 for two
 // products) and at most one output tile per CTA, so that a CTA writes at most two partials.
 FERRUM_API int ferrum_gemm_tc_can_defer(int M, int N, int K, int dual, int n_ctas) {
-  if (n_ctas <= 0) n_ctas = sm_count();
+  if (n_ctas <= 0) n_ctas = ferrum_sm_count();
   const int bt = ferrum_gemm_tc_token_tile(M, dual);
   const long long tiles = (N + TILE_N - 1) / TILE_N;
   const long long units = tiles * ((K + TILE_K - 1) / TILE_K);
@@ -1476,7 +1465,7 @@ FERRUM_API int ferrum_gemm_tc_deferred(const void* x, const void* w, int dtype, 
   FERRUM_CHECK_ARG(w_rows >= N + dual_offset, "gemm_tc_deferred: w has %d rows, needs %d", w_rows, N + dual_offset);
   FERRUM_CHECK_ARG(ferrum_gemm_tc_can_defer(M, N, K, dual, n_ctas), "gemm_tc_deferred: shape M=%d N=%d K=%d cannot defer its "
                    "reduction (more than one token tile, or more output tiles than CTAs)", M, N, K);
-  if (n_ctas <= 0) n_ctas = sm_count();
+  if (n_ctas <= 0) n_ctas = ferrum_sm_count();
   const int bt = ferrum_gemm_tc_token_tile(M, dual);
   const int nkb = (K + TILE_K - 1) / TILE_K, tiles = (N + TILE_N - 1) / TILE_N;
   if (n_ctas > (long long)tiles * nkb) n_ctas = tiles * nkb;
@@ -1564,7 +1553,7 @@ FERRUM_API int ferrum_gemm_tc_noalloc(const void* x, const void* w, void* out, i
   FERRUM_CHECK_ARG(epilogue >= 0 && epilogue <= 3, "gemm_tc_noalloc: unknown epilogue %d", epilogue);
   FERRUM_CHECK_ARG(dual == (epilogue == TC_SWIGLU), "gemm_tc_noalloc: the SwiGLU epilogue needs dual_offset, and only it does");
   FERRUM_CHECK_ARG(w_rows >= N + dual_offset, "gemm_tc_noalloc: w has %d rows, needs %d", w_rows, N + dual_offset);
-  int n_ctas = sm_count();
+  int n_ctas = ferrum_sm_count();
   const int bt = ferrum_gemm_tc_token_tile(M, dual);
   int tiles = 0;
   const long long need_floats = single_cta_floats(bt, dual, n_ctas);      // (this entry never takes the pair kernel)
@@ -1855,7 +1844,7 @@ FERRUM_API int ferrum_gemm_tc_grouped(const void* x, const void* w, void* out, i
   if (int r = get_tensor_map(w, (long long)n_exp * w_rows, K, K, TILE_N, &mw)) return r;
   if (int r = get_tensor_map(x, x_rows, K, ldx, GR_BT, &mx)) return r;
   const long long tiles_bound = (long long)((n_rows + GR_BT - 1) / GR_BT + n_exp) * ((N + TILE_N - 1) / TILE_N);
-  int n_ctas = sm_count();
+  int n_ctas = ferrum_sm_count();
   if (n_ctas > tiles_bound) n_ctas = (int)tiles_bound;
   return dual ? launch_tc_grouped<true>(mw, mx, p, g, n_ctas, stream) : launch_tc_grouped<false>(mw, mx, p, g, n_ctas, stream);
 }
