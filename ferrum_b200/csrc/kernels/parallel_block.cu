@@ -107,15 +107,22 @@ norm_scaled_add_kernel(float* __restrict__ x, const float* __restrict__ y, const
 // A step of a few tokens is a chain of such kernels: each is launched behind the one before it in dependent mode, and both norms'
 // weights are on their way to the L2 before it waits.  (B200, 8 tokens of the hybrid model with 4 layers, this and the kernels of
 // mamba2.cu, attention_prep.cu, attention_generic.cu and thin_linear.cu: a step 372 -> 350 us.)
+// PIECES, PARTIALS: kept apart because a block of up to 1024 threads has 64 registers a thread: four pieces beside the loads of a sum of
+// partials leave none for weights, and one kernel for all spilled.  WITH_ROW: the weights are read with the row, not where they are
+// used; with many rows other blocks hide that latency and the registers count.
+// (B200, us, x += norm(y) and its norm, one kernel with early weights -> so: 2,048 elements, 8 tokens 2.19 -> 1.98, 65 2.94 -> 2.12, 300 4.47 -> 3.94,
+// 2,048 14.4 -> 12.8; 4,096 elements, 8 2.83 -> 2.50, 300 6.37 -> 5.69, 600 10.2 -> 10.4, 2,048 26.3 -> 22.2; from partials, 4,096 elements, 8 3.87 -> 3.27, 100
+// 12.2 -> 6.7.  Weights with the row beyond the line drawn here: 1,000 x 2,048 7.73 -> 8.01, 2,048 x 4,096 22.9 -> 25.3.)
 constexpr int PB_PIECES = 4;
-template <typename T>
-__global__ void __launch_bounds__(1024)
+constexpr int PB_ROW_THREADS = 512;     // threads an SM up to which the weights come with the row
+template <typename T, int PIECES, bool PARTIALS, bool WITH_ROW, int THREADS>
+__global__ void __launch_bounds__(THREADS, 1)
 norm_scaled_add_vec_kernel(float* __restrict__ x, const float* __restrict__ y, const float* __restrict__ w, float mult, float eps,
                            int E, const PartialLayout L, const float* __restrict__ w2, float eps2, T* __restrict__ out) {
   pdl_launch();      // the kernel that follows may fetch its weights meanwhile
   __shared__ float red[32];
   __shared__ PartialTable tab;
-  if (L.ws != nullptr) build_partial_table(L, tab);
+  if constexpr (PARTIALS) build_partial_table(L, tab);
   const int t = blockIdx.x, n4 = E >> 2;
   if (blockIdx.x == 0)          // (the weights start for the L2 while the kernel ahead of this one ends)
     for (int i = threadIdx.x * 8; i < n4; i += blockDim.x * 8) {
@@ -123,15 +130,26 @@ norm_scaled_add_vec_kernel(float* __restrict__ x, const float* __restrict__ y, c
       if (out != nullptr) prefetch_l2(w2 + 4 * i);
     }
   pdl_wait();
-  float4 v[PB_PIECES], xo[PB_PIECES];
+  float4 v[PIECES], xo[PIECES], wg[PIECES], wg2[PIECES];
+  if constexpr (WITH_ROW) {
+#pragma unroll
+    for (int k = 0; k < PIECES; ++k) {
+      const int i = threadIdx.x + k * blockDim.x;
+      wg[k] = wg2[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (i < n4) {
+        wg[k] = *reinterpret_cast<const float4*>(w + 4 * i);
+        if (out != nullptr) wg2[k] = *reinterpret_cast<const float4*>(w2 + 4 * i);
+      }
+    }
+  }
   float ss = 0.f;
 #pragma unroll
-  for (int k = 0; k < PB_PIECES; ++k) {
+  for (int k = 0; k < PIECES; ++k) {
     const int i = threadIdx.x + k * blockDim.x;
     v[k] = xo[k] = make_float4(0.f, 0.f, 0.f, 0.f);
     if (i < n4) {
       xo[k] = *reinterpret_cast<const float4*>(x + (size_t)t * E + 4 * i);
-      if (L.ws != nullptr) {
+      if (PARTIALS) {
         v[k] = partial_sum4(L, tab, t, 4 * i);
       } else {
         v[k] = *reinterpret_cast<const float4*>(y + (size_t)t * E + 4 * i);
@@ -146,10 +164,10 @@ norm_scaled_add_vec_kernel(float* __restrict__ x, const float* __restrict__ y, c
   const float r = 1.f / sqrtf(ss / (float)E + eps);
   float s2 = 0.f;
 #pragma unroll
-  for (int k = 0; k < PB_PIECES; ++k) {
+  for (int k = 0; k < PIECES; ++k) {
     const int i = threadIdx.x + k * blockDim.x;
     if (i >= n4) continue;
-    const float4 g = *reinterpret_cast<const float4*>(w + 4 * i);
+    const float4 g = WITH_ROW ? wg[k] : *reinterpret_cast<const float4*>(w + 4 * i);
     xo[k].x = fmaf(mult, v[k].x * r * g.x, xo[k].x);
     xo[k].y = fmaf(mult, v[k].y * r * g.y, xo[k].y);
     xo[k].z = fmaf(mult, v[k].z * r * g.z, xo[k].z);
@@ -164,10 +182,10 @@ norm_scaled_add_vec_kernel(float* __restrict__ x, const float* __restrict__ y, c
   s2 = block_sum(s2, red);
   const float r2 = 1.f / sqrtf(s2 / (float)E + eps2);
 #pragma unroll
-  for (int k = 0; k < PB_PIECES; ++k) {
+  for (int k = 0; k < PIECES; ++k) {
     const int i = threadIdx.x + k * blockDim.x;
     if (i >= n4) continue;
-    const float4 g = *reinterpret_cast<const float4*>(w2 + 4 * i);
+    const float4 g = WITH_ROW ? wg2[k] : *reinterpret_cast<const float4*>(w2 + 4 * i);
     const float a = xo[k].x * r2 * g.x, b = xo[k].y * r2 * g.y, c = xo[k].z * r2 * g.z, d = xo[k].w * r2 * g.w;
     if constexpr (sizeof(T) == 4) {
       *reinterpret_cast<float4*>(out + (size_t)t * E + 4 * i) = make_float4(a, b, c, d);
@@ -253,7 +271,18 @@ FERRUM_API int ferrum_norm_scaled_add(float* x, const float* y, const float* w, 
     // a few rows: a piece a thread; many: four, so that several rows share an SM
     const int n4 = E / 4, most = n_tokens <= 64 ? n4 : (n4 + PB_PIECES - 1) / PB_PIECES;
     const int threads = min(1024, max((most + 31) / 32 * 32, (n4 + 32 * PB_PIECES - 1) / (32 * PB_PIECES) * 32));
-    FERRUM_DISPATCH_DTYPE(dtype, T, (launch_kernel(norm_scaled_add_vec_kernel<T>, dim3(n_tokens), dim3(threads), 0, stream, x, y, w, mult, eps, E, L, w2, eps2, (T*)out)));
+    const bool one = threads >= n4, part = L.ws != nullptr;
+    const bool with_row = threads <= 512 && (long long)n_tokens * threads <= (long long)PB_ROW_THREADS * ferrum_sm_count();
+#define PB_LAUNCH(...)                                                                                                                     \
+  launch_kernel(norm_scaled_add_vec_kernel<T, __VA_ARGS__>, dim3(n_tokens), dim3(threads), 0, stream, x, y, w, mult, eps, E, L, w2, eps2, (T*)out)
+    FERRUM_DISPATCH_DTYPE(dtype, T, {
+      if (part && one) PB_LAUNCH(1, true, true, 1024);
+      else if (part) PB_LAUNCH(PB_PIECES, true, false, 1024);
+      else if (one) PB_LAUNCH(1, false, true, 1024);
+      else if (with_row) PB_LAUNCH(PB_PIECES, false, true, 512);
+      else PB_LAUNCH(PB_PIECES, false, false, 1024);
+    });
+#undef PB_LAUNCH
     FERRUM_CHECK_LAUNCH("norm_scaled_add");
     return 0;
   }

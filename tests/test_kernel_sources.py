@@ -2,6 +2,9 @@
 import glob
 import os
 import re
+import subprocess
+
+import pytest
 
 KERNELS = os.path.join(os.path.dirname(os.path.abspath(__file__)), "..", "ferrum_b200", "csrc", "kernels")
 
@@ -17,3 +20,15 @@ def test_a_failed_call_is_made_again():
 def test_the_number_of_multiprocessors_is_asked_in_one_place():
     asked = [os.path.basename(f) for f in glob.glob(os.path.join(KERNELS, "*.cu*")) if re.search(r"MultiProcessorCount|multiProcessorCount", open(f).read())]
     assert asked == ["common.cu"], asked
+
+
+@pytest.mark.parametrize("file,kernel,instances", [("parallel_block.cu", "norm_scaled_add_vec_kernel", 15)])
+def test_rows_kept_in_registers_stay_there(file, kernel, instances, tmp_path):
+    """Kernels whose comment says that a row stays in registers have no stack."""
+    from ferrum_b200.ops import build
+    nvcc = build._find("nvcc", ["/usr/local/cuda/bin"])
+    r = subprocess.run([nvcc, *build.NVCC_ARCH, "-O3", "-std=c++17", "-Xptxas", "-v", "-c", os.path.join(KERNELS, file), "-o", str(tmp_path / "o.o")],
+                       capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    stacks = [int(n) for n in re.findall(rf"Compiling entry function '\w*{kernel}\w*'[^\n]*\n(?:[^\n]*Function properties[^\n]*\n)?\s*(\d+) bytes stack frame", r.stderr)]
+    assert len(stacks) == instances and not any(stacks), stacks

@@ -59,3 +59,49 @@ def test_norm_of_many_rows_covers_the_width(cuda, dtype, E):
     # a sum of squares in a tree of some 20 levels, a root, a division and two products; one rounding of the output type
     bound = want.abs() * (24 * 2.0 ** -24 + (2.0 ** -8 if dtype == torch.bfloat16 else 0.0))
     assert ((out[:70].double() - want).abs() <= bound).all() and (out[70] == 7).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("T,E", [(1, 4), (3, 1028), (64, 2048), (65, 2048), (592, 2048), (593, 2048), (64, 4096), (296, 4096), (297, 4096), (8, 4100), (64, 8192),
+                                 (65, 8200), (2, 16384), (70, 16384), (1200, 2052)])
+def test_norm_scaled_add_on_both_sides_of_its_lines(cuda, dtype, T, E):
+    """Token counts and widths where the kernel changes pieces a thread, threads a block and the place its weights are read."""
+    from ferrum_b200.ops import lib as ops
+    g = torch.Generator(device="cuda").manual_seed(T + E)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    x, y, w, w2, out = r(T + 1, E), r(T, E), r(E), r(E), torch.full((T + 1, E), 7.0, device="cuda", dtype=dtype)
+    norm = lambda v, eps: v / torch.sqrt((v * v).mean(-1, keepdim=True) + eps)
+    add = 0.7 * norm(y.double(), 1e-5) * w.double()
+    want = x[:T].double() + add
+    alone, both = x.clone(), x.clone()
+    ops.norm_scaled_add(alone, y, w, 0.7, 1e-5, T)
+    ops.norm_scaled_add(both, y, w, 0.7, 1e-5, T, norm=(w2, 1e-6, out))
+    assert torch.equal(alone, both) and torch.equal(alone[T], x[T]) and (out[T] == 7).all()
+    # a sum of squares in some 20 levels, a root, a division and three products; then the same of the new rows
+    assert ((alone[:T].double() - want).abs() <= (x[:T].abs().double() + add.abs()) * 24 * 2.0 ** -24).all()
+    want = norm(alone[:T].double(), 1e-6) * w2.double()
+    rounding = {torch.float32: 0.0, torch.float16: 2.0 ** -11, torch.bfloat16: 2.0 ** -8}[dtype]
+    assert ((out[:T].double() - want).abs() <= want.abs() * (24 * 2.0 ** -24 + rounding) + 1e-7).all()
+
+
+@pytest.mark.parametrize("T,E,K,ctas", [(1, 1028, 256, 0), (8, 4096, 4096, 0), (40, 2048, 2048, 32), (64, 4096, 2048, 0), (100, 2048, 1024, 40), (100, 3588, 2048, 0), (8, 8192, 4096, 0),
+                                        (128, 8192, 1024, 0)])
+def test_norm_scaled_add_of_partials(cuda, T, E, K, ctas):
+    """A product left in several partials a tile (widths that end inside a tile too) gives the bits of the same sums stored."""
+    from ferrum_b200.ops import lib as ops
+    g = torch.Generator(device="cuda").manual_seed(E + K)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    a, b = r(T, K).bfloat16(), (r(E, K) * 0.05).bfloat16()
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    floats, _ = ops.gemm_tc_workspace(T, E, K, False)
+    part = ops.gemm_tc_deferred(a, b, err, torch.empty(floats, device="cuda"), n_ctas=ctas)
+    y = torch.zeros(T, E, device="cuda")
+    ops.residual_reduce(y, T, part)
+    assert ((y - a.float() @ b.float().T).abs() <= 1e-2 * y.std()).all() and err.item() == 0
+    x, w, w2 = r(T, E), r(E), r(E)
+    one, two, three = x.clone(), x.clone(), x.clone()
+    out, out2 = (torch.empty(T, E, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    ops.norm_scaled_add(one, y, w, 0.7, 1e-5, T, norm=(w2, 1e-6, out))
+    ops.norm_scaled_add(two, None, w, 0.7, 1e-5, T, partials=part)
+    ops.norm_scaled_add(three, None, w, 0.7, 1e-5, T, partials=part, norm=(w2, 1e-6, out2))
+    assert torch.equal(one, two) and torch.equal(one, three) and torch.equal(out, out2)
