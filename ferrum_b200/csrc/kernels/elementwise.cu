@@ -597,10 +597,11 @@ FERRUM_API int ferrum_rope_cache_write(void* qkv, int dtype, int n_tokens, int l
   const int threads = 256;
   // few tokens, or a product still in partials (several loads per element): several blocks per
   // token, four head slots each, so that a row is read by many SMs at once
-  // more: eight head slots each while a block a token would leave an SM fewer than eight (float32, 300 tokens of 40 slots of
-  // 128: 9.7 us with a block a token, 7.7 so)
+  // more: as many as keep eight blocks an SM in all, with eight head slots each at least.  (B200, float32, a block a token / this / eight
+  // slots each, us: 40 slots of 128, 300 tokens 10.3 / 8.7 / 8.5, 600 11.9 / 11.9 / 13.4, 1,183 20.4 / 20.4 / 23.3; 48 slots, 300 tokens 11.0 / 9.2 / 9.2, 800
+  // 14.1 / 14.1 / 19.1; twelve blocks an SM: 8.5, 12.3, 20.4; 8.6, 15.4.)
   const int slots = Hq + 2 * Hkv;
-  const dim3 grid(n_tokens, (n_tokens <= 64 || partials != nullptr) ? (slots + 3) / 4 : (n_tokens < 8 * 148 ? (slots + 7) / 8 : 1));
+  const dim3 grid(n_tokens, (n_tokens <= 64 || partials != nullptr) ? (slots + 3) / 4 : max(1, min((slots + 7) / 8, 8 * ferrum_sm_count() / n_tokens)));
   FERRUM_DISPATCH_DTYPE(dtype, T, launch_kernel(rope_cache_kernel<T>, grid, threads, 0, stream, (T*)qkv, ld, positions, req_of_token,
                                                 block_table, table_width, cos_sin, n_pos, (T*)kv_plane, page_stride, page_size, Hq,
                                                 Hkv, D, R, pairing, write_kv, err_flag, L));

@@ -19,7 +19,7 @@ def test_float32_swiglu_widths(cuda, T, F, pad):
     assert not act[T].any() and not act[:, F:].any()
 
 
-@pytest.mark.parametrize("T", [65, 300, 1183, 1184])
+@pytest.mark.parametrize("T", [65, 300, 591, 592, 593, 800, 1183, 1184, 1185])
 @pytest.mark.parametrize("Hq,Hkv,D,R,pairing", [(24, 8, 128, 128, 1), (3, 1, 20, 12, 0), (5, 5, 64, 64, 0)])
 def test_float32_rotary_rows_do_not_depend_on_the_grid(cuda, T, Hq, Hkv, D, R, pairing):
     from ferrum_b200.ops import lib as ops
@@ -43,6 +43,30 @@ def test_float32_rotary_rows_do_not_depend_on_the_grid(cuda, T, Hq, Hkv, D, R, p
 
     (a, b), (c, d) = run(T), run(64)
     assert torch.equal(a, c) and torch.equal(b, d) and err.item() == 0
+
+
+def test_float32_rotary_rows_take_no_longer_for_a_token_less(cuda):
+    """The grid shrinks as the tokens grow, not all at once (with six blocks a token up to a line 800 tokens took longer than 1,184)."""
+    from ferrum_b200.ops import lib as ops
+    Hq, Hkv, D, page, T = 32, 8, 128, 16, 1184
+    qkv, plane = torch.zeros(T, (Hq + 2 * Hkv) * D, device="cuda"), torch.zeros(T // page, 2, Hkv, page, D, device="cuda")
+    cos_sin, positions = torch.ones(T, D // 2, 2, device="cuda"), torch.arange(T, dtype=torch.int32, device="cuda")
+    req, table = torch.zeros(T, dtype=torch.int32, device="cuda"), torch.arange(T // page, dtype=torch.int32, device="cuda")[None]
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+
+    def time(n):
+        begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        torch.cuda._sleep(4_000_000)           # some 2 ms: all launches are queued before the first runs
+        begin.record()
+        for _ in range(40):
+            ops.rope_cache_write(qkv, n, positions, req, table, cos_sin, plane, plane.stride(0), page, Hq, Hkv, D, D, 1, True, err)
+        end.record()
+        torch.cuda.synchronize()
+        return begin.elapsed_time(end)
+
+    time(T)
+    few, many = (min(time(n) for _ in range(7)) for n in (800, T))
+    assert few < 0.87 * many           # (1.04 with the line, 0.72 without)
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
