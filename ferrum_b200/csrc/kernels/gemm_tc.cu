@@ -563,6 +563,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
   const PairSchedule sched(tiles_n, tiles_t, nkb, P, cluster, p.cut != 0);
   const int stage_bytes = A_BYTES + bt / 2 * TILE_K * 2;   // each CTA stages half of the tile's tokens
   const int STAGES = PAIR_RING_BYTES / stage_bytes;
+  const bool floats = p.epilogue == TC_RESIDUAL || p.epilogue == TC_STORE_F32;
+  const int groups = floats ? 1 : 2;      // of four epilogue warps; see there
 
   const uint32_t smem_base = smem_u32(smem);
   const uint32_t bar_base = smem_u32(bars);
@@ -587,7 +589,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(acc_full_bar(b), 1);
-      mbar_init(acc_empty_bar(b), 16);  // the leader's: eight epilogue warps of each CTA
+      mbar_init(acc_empty_bar(b), 8 * groups);  // the leader's: the epilogue warps of each CTA
     }
     mbar_init(fetch_bar, 1);
     fence_barrier_init();
@@ -684,26 +686,29 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         if (ok) umma_commit_pair(acc_full_bar(buf), 3);
       }
     }
-  } else {
-    // ------------------------------------------------------------ epilogue (warps 2..9, both CTAs)
+  } else if (warp < 2 + 4 * groups) {
+    // ------------------------------------------------------------ epilogue (warps 2..9, or 2..5, both CTAs)
     const int quarter = warp & 3;
     const int n_local = quarter * 32 + lane;
     const int ep_tid = threadIdx.x - 64;
     const uint32_t lane_addr = tmem_base + ((uint32_t)(quarter * 32) << 16);
     const size_t tile_floats = (size_t)ACC_COLS * TILE_N;
-    const bool staged = p.out_tma != 0, floats = p.epilogue == TC_RESIDUAL || p.epilogue == TC_STORE_F32;
+    const bool staged = p.out_tma != 0;
     // Two groups of four warps take the 32-column pieces of a tile of 16-bit results in turn, each with half of the staging (two
     // buffers of 32 tokens x 128 features) and a barrier of its own: what follows a tile's last product is a chain of read,
     // stage and send for every piece, up to eight of them, and with short K it is a good part of the kernel.  float32 results need
-    // twice the staging and keep one group with both buffers (two groups with one each: 512 x [4096, 4096] 20.0 -> 21.2 us).
+    // twice the staging and keep one group with both buffers (two groups with one each: 512 x [4096, 4096] 20.0 -> 21.2 us); the other
+    // four warps then stay out of all of it.
     // B200, us, one group -> two: 391 x 2 x [8192, 3072] 42.5 -> 38.3, 200 x the same 34.3 -> 30.3, 391 x [5120, 3072] 17.7 -> 16.9,
-    // 512 x 2 x [8192, 3072] 47.1 -> 42.4, 1,024 x the same 83 -> 76; 391 tokens of Llama-3.2-3B 3,984 -> 3,878..3,949 (2 to 3 %).
-    // (float32 results of tiles that are cut along K pay for the wider barriers: 200 x [3072, 8192] 24.1 -> 24.9, 391 x [4096, 14336]
-    // 55.8 -> 56.8, the others the same.)
+    // 512 x 2 x [8192, 3072] 47.1 -> 42.4, 1,024 x the same 83 -> 76; 391 tokens of Llama-3.2-3B 3,984 -> 3,878..3,949 (1 to 3 %).
+    // float32 results with all eight warps at every barrier -> four: 200 x [3072, 8192] 25.1 -> 24.5 us, 391 x [4096, 14336] 56.6 -> 55.8, 150 x the same 43.0 ->
+    // 42.2, 200 tokens of Llama-3.2-3B 3,287 -> 3,260, 391 3,811 -> 3,793.  (An instance of 192 threads and 255 registers for them is as fast alone, but
+    // steps that go back and forth between two such kernels lose: 3,335 and 3,893.)
     const int group = ep_tid >> 7, g_tid = ep_tid & 127;
-    const int piece0 = floats ? (group ? PAIR_BT : 0) : group * 32, piece_step = floats ? 32 : 64;
+    const int piece0 = group * 32, piece_step = groups * 32;
     uint8_t* out_stage = smem + PAIR_RING_BYTES + 256 + (floats ? 0 : group * PAIR_OUT_BYTES);
     bool whole_stage = false;     // 16-bit results: the last store (of a partial) reads the group's whole staging, not a half of it
+    auto all_sync = [&]() { asm volatile("bar.sync 1, %0;" ::"r"(groups * 128) : "memory"); };
     auto group_sync = [&]() { asm volatile("bar.sync %0, 128;" ::"r"(2 + group) : "memory"); };
     int emitted = 0;  // staged stores issued so far; buffer = emitted & 1
     pdl_wait();
@@ -780,7 +785,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
       const int buf = seg & 1, use = seg >> 1;
       bool ok = mbar_wait(acc_full_bar(buf), use & 1, abort_p, wait_limit);
       if (!ok) abort_flag = 1;
-      asm volatile("bar.sync 1, 256;" ::: "memory");
+      all_sync();
       if (abort_flag) {
         if (ep_tid == 0) atomicExch(p.err, 12);
         break;
@@ -798,7 +803,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         float* out = (float*)p.out + (size_t)t0 * p.ldo + n;
         const size_t ld = (size_t)p.ldo;
 #pragma unroll 1
-        for (int c0 = group * 32; c0 < bt; c0 += 64) {
+        for (int c0 = piece0; c0 < bt; c0 += piece_step) {
           const int valid = n < p.N ? p.M - t0 - c0 : 0;
           float r[32], v[32];
 #pragma unroll
@@ -860,10 +865,10 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
               while (ld_acquire_gpu(counter) != others && ++polls < PAIR_FINISHER_POLLS && !*abort_p) __nanosleep(100);
               is_last = polls < PAIR_FINISHER_POLLS && !*abort_p;
             }
-            asm volatile("bar.sync 1, 256;" ::: "memory");
+            all_sync();
           }
           const bool fast = finisher && is_last;
-          asm volatile("bar.sync 1, 256;" ::: "memory");
+          all_sync();
           if (fast) {
             const float* fetched = (const float*)smem;  // [contributor][column][128 rows]
             bool fine = true;
@@ -883,7 +888,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
               fine = mbar_wait(fetch_bar, fetch_phase, abort_p, wait_limit);
               fetch_phase ^= 1;
               if (!fine) abort_flag = 1;
-              asm volatile("bar.sync 1, 256;" ::: "memory");
+              all_sync();
               if (abort_flag) {
                 if (ep_tid == 0) atomicExch(p.err, 14);
                 fine = false;
@@ -902,7 +907,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                 if (p.gated) emit32_gated(t0, c0, n0, v);
                 else emit32(t0, c0, n0, v);
               }
-              asm volatile("bar.sync 1, 256;" ::: "memory");  // all have read the stages before the next copies land
+              all_sync();  // all have read the stages before the next copies land
             }
             tc_fence_before();
             __syncwarp();
@@ -927,7 +932,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
           if (g_tid == 0) bulk_wait_all();  // the partial is written before it is announced
         } else {
 #pragma unroll 1
-          for (int c0 = group * 16; c0 < bt; c0 += 32) {
+          for (int c0 = group * 16; c0 < bt; c0 += groups * 16) {
             float v[16];
             tmem_ld16(acc_addr + c0, v);
 #pragma unroll
@@ -938,13 +943,13 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster(leader_acc_empty);
         __threadfence();
-        asm volatile("bar.sync 1, 256;" ::: "memory");
+        all_sync();
         if (ep_tid == 0) {
           const int old = atomicAdd(counter, 1);
           is_last = old == n_contrib - 1;
           if (is_last) *counter = 0;
         }
-        asm volatile("bar.sync 1, 256;" ::: "memory");
+        all_sync();
         if (is_last && staged) {
           // The last arriver adds the partials in K order.  A thread takes four neighbouring
           // features of eight columns, two contributors at a time: 16-byte loads, 16 of them in
