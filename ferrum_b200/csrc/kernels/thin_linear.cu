@@ -45,10 +45,16 @@ thin_linear_kernel(const T* __restrict__ x, int ldx, const T* __restrict__ w, in
   for (int i = 0; i < TL_TOKENS; ++i) xr[i] = x + (size_t)(t0 + min(i, nt - 1)) * ldx;     // (rows past the last repeat it and are dropped)
 #pragma unroll
   for (int j = 0; j < NF; ++j) wr[j] = w + (size_t)min(n0 + j, N - 1) * K;
-  // The weights never change: they start for the L2 while the kernel ahead of this one ends.
-  for (int k = tid * 8; k < K; k += TL_THREADS * 8)
+  // The weights start for the L2 while the kernel ahead of this one ends: a line a lane, or a piece a thread where that measured better
+  // (B200, us, 16-byte pieces -> lines, two features a block: 8 tokens x 8 features of 2,048 2.41 -> 1.81, x 16 of 4,096 3.78 -> 2.66, 1 x 256 of 2,048 2.57 ->
+  // 2.49, 64 x 64 3.17 -> 2.98; eight features a block, nothing / lines / pieces: 65 x 8 of 2,048 2.74 / 3.10 / 2.51, 1,000 3.9 / 3.9 / 3.3, 2,048 7.2 / 7.6 / 6.4).
+  if constexpr (NF > 2) {
+    for (int k = tid * 8; k < K; k += TL_THREADS * 8)
 #pragma unroll
-    for (int j = 0; j < NF; ++j) prefetch_l2(wr[j] + k);
+      for (int j = 0; j < NF; ++j) prefetch_l2(wr[j] + k);
+  } else if (warp < NF) {
+    for (int k = lane * 64; k < K; k += 32 * 64) prefetch_l2(w + (size_t)min(n0 + warp, N - 1) * K + k);
+  }
   pdl_wait();
   for (int k = tid * 8; k < K; k += TL_THREADS * 8) {
     uint4 xraw[TL_TOKENS];
