@@ -351,7 +351,8 @@ gemm_stream_kernel(const float* __restrict__ x, const float* __restrict__ w, voi
 // holds) come through registers one slice ahead.  Same sums in the same order as the kernel above: over slices in a thread, over a
 // warp's lanes in a butterfly, over the four warps in order.
 // B200, weights from memory, us, the kernel above -> this one, 4 tokens: 3072 x 3072 12.2 -> 10.5, 5120 x 3072 18.2 -> 14.8,
-// 16384 x 3072 45.4 -> 34.6, 3072 x 8192 25.9 -> 21.8, 128256 x 3072 333 -> 244 (6.5 TB/s); one token the same, 64 x 64 2.6 -> 2.0.
+// 16384 x 3072 45.4 -> 34.6, 3072 x 8192 25.9 -> 21.8, 128256 x 3072 333 -> 244 (6.5 TB/s), 64 x 64 2.6 -> 2.0; one token gains as
+// much (3072 x 3072 11.9 -> 10.1, 16384 x 3072 44.9 -> 33.6).
 // From five tokens on it loses (8 tokens, two sets of threads or eight sums a feature: 12.4 -> 14.6..15.8, 26.2 -> 30.8..33.6): every group
 // reads the tokens again, and a group of five or six features has then as many of their bytes as of the weights'.
 constexpr int S4_FEAT = 8;       // features of a group at most

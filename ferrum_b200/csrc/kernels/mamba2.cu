@@ -227,7 +227,8 @@ mamba_scan_kernel(const float* __restrict__ xbc, int C, const float* __restrict_
 
 // A step of a few tokens has as many blocks: nothing hides a load behind another block's work, so a thread has the loads of
 // GN_KEEP elements on their way together and keeps their values for the second pass.  (One dependent pair of loads after
-// the other: 8 tokens x 4,096 took 15.4 us on a B200, now 3.8.)
+// the other: 8 tokens x 4,096 took 15.4 us on a B200, now 3.8.  With many tokens it is the better form too, for all its 72 registers:
+// the whole mixer of 64, 300 and 2,048 tokens 28 -> 21, 75 -> 69, 466 -> 449 us.)
 constexpr int GN_KEEP = 16;
 template <typename T>
 __global__ void __launch_bounds__(256)
