@@ -251,8 +251,9 @@ bias_glu_kernel(const float* __restrict__ gu, int ld, const float* __restrict__ 
   }
 }
 
-// The same, four features a thread (F and both strides multiples of 4, 16-byte boundaries).
-constexpr int GLU_VEC_THREADS = 128;
+// The same, four features a thread (F and both strides multiples of 4, 16-byte boundaries), from nine tokens on: with fewer the blocks are too
+// few to gain from wide loads.  (B200, F = 5,632, us, one feature a thread / four: 1 token 1.09 / 1.22, 8 1.13 / 1.22, 16 1.31 / 1.30, 64 2.47 / 2.01, 1,500 35 / 17.)
+constexpr int GLU_VEC_THREADS = 128, GLU_VEC_MIN_TOKENS = 9;
 template <typename TOut>
 __global__ void __launch_bounds__(GLU_VEC_THREADS)
 bias_glu_vec_kernel(const float* __restrict__ gu, int ld, const float* __restrict__ bg, const float* __restrict__ bu, TOut* __restrict__ act,
@@ -273,7 +274,7 @@ FERRUM_API int ferrum_bias_glu(const float* gu, int ld, const float* bias_gate, 
   FERRUM_CHECK_ARG(kind >= 0 && kind <= GLU_SWISH_CLAMP, "bias glu: unknown activation %d", kind);
   if (n_tokens == 0) return 0;
   FERRUM_CHECK_ARG(n_tokens <= 65535, "bias glu: too many tokens");
-  if (F % 4 == 0 && ld % 4 == 0 && ld_out % 4 == 0 && gb_aligned({gu, bias_gate, bias_up, act})) {
+  if (n_tokens >= GLU_VEC_MIN_TOKENS && F % 4 == 0 && ld % 4 == 0 && ld_out % 4 == 0 && gb_aligned({gu, bias_gate, bias_up, act})) {
     const dim3 vgrid((F / 4 + GLU_VEC_THREADS - 1) / GLU_VEC_THREADS, n_tokens);
     FERRUM_DISPATCH_DTYPE(act_dtype, T, launch_kernel(bias_glu_vec_kernel<T>, vgrid, dim3(GLU_VEC_THREADS), 0, stream, gu, ld, bias_gate, bias_up, (T*)act, ld_out, F, kind, limit));
     FERRUM_CHECK_LAUNCH("bias_glu");

@@ -22,7 +22,8 @@ def rand(g, *shape):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
-@pytest.mark.parametrize("T,F,pad", [(1, 4, 0), (3, 508, 4), (3, 512, 0), (3, 516, 8), (3, 516, 1), (2, 513, 0), (70, 5632, 2048)])
+@pytest.mark.parametrize("T,F,pad", [(1, 4, 0), (3, 508, 4), (3, 512, 0), (3, 516, 8), (3, 516, 1), (2, 513, 0), (70, 5632, 2048), (8, 512, 0), (9, 4, 0), (9, 508, 4),
+                                     (9, 512, 0), (9, 516, 8), (9, 516, 1), (9, 513, 0)])
 def test_bias_glu_widths(cuda, dtype, T, F, pad):
     from ferrum_b200.ops import lib as ops
     g = torch.Generator(device="cuda").manual_seed(F + pad)
@@ -30,6 +31,10 @@ def test_bias_glu_widths(cuda, dtype, T, F, pad):
     act = torch.zeros(T + 1, F, device="cuda", dtype=dtype)
     for gate, up in ((bg, bu), (None, bu), (None, None)):
         ops.bias_glu(gu, gate, up, act[:T], T, F, "silu")
+        if T > 8:          # fewer tokens run one feature a thread: the same bits
+            first = torch.empty(8, F, device="cuda", dtype=dtype)
+            ops.bias_glu(gu, gate, up, first, 8, F, "silu")
+            assert torch.equal(first, act[:8])
         z = gu[:, :F].double() + (gate.double() if gate is not None else 0)
         u = gu[:, F:2 * F].double() + (up.double() if up is not None else 0)
         close(act[:T], torch.nn.functional.silu(z) * u, dtype)
