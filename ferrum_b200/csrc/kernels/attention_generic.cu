@@ -422,8 +422,8 @@ attention_generic_tokens_kernel(const T* __restrict__ q, int ldq, T* __restrict_
   const int G = Hq / Hkv;
   const int hchunks = (G + AG_HEADS - 1) / AG_HEADS;
   // The last chunks first: a portion's later tokens see more keys, and what does not fit the first wave should be short.  (Of several
-  // portions the last comes first, whatever their lengths.  B200, float32, 300 tokens, 24 heads, 8 KV heads, 312 CTAs on 296 places:
-  // 79 us in ascending order, 64 in this one.)
+  // portions the last comes first, whatever their lengths.  B200, float32, 24 heads, 8 KV heads, 28 layers, ascending -> this, us: steps of 100
+  // tokens 5,613 -> 5,608, 300 14,030 -> 13,800, 500 21,780 -> 20,590; three portions of 20, 140 and 260 tokens 17,820 -> 17,710.)
   const int c = (int)(gridDim.x / (Hkv * hchunks)) - 1 - (int)(blockIdx.x / (Hkv * hchunks));
   const int kvh = (blockIdx.x / hchunks) % Hkv;
   const int hchunk = blockIdx.x % hchunks;
