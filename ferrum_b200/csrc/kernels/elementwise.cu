@@ -188,7 +188,8 @@ rmsnorm_cluster_kernel(float* __restrict__ h, const float* __restrict__ w, TOut*
   const int lo = rank * per, hi = min(E, lo + per);
   // The norm's weights start for the L2 while the kernel ahead of this one ends, and are read first thing after it, not behind the
   // cluster's sum.  (B200, decode step of Llama-3.1-8B with 65 such norms, read behind the sum -> so: 3,283 -> 3,252 us with one token,
-  // 4,609 -> 4,604 with 8, 5,402 -> 5,386 with 64; read between the row's own loads 3,261.)
+  // 4,609 -> 4,604 with 8, 5,402 -> 5,386 with 64; read between the row's own loads 3,261.  Read before the wait, which the kernel ahead
+  // might still write, 3,252; one token of Llama-3.2-3B 1,898 behind the sum, 1,887 so, 1,875 before the wait.)
   for (int i = lo + threadIdx.x * 32; i < hi; i += 256 * 32) prefetch_l2(w + i);
   pdl_launch();
   pdl_wait();
